@@ -124,8 +124,9 @@ void graph_release_on(bbtc_graph* g, cudaStream_t s) {
   if (g->d_indptr) cudaFreeAsync(g->d_indptr, s);
   if (g->d_indices) cudaFreeAsync(g->d_indices, s);
   if (g->d_words) cudaFreeAsync(g->d_words, s);
-  if (g->d_wptr) cudaFreeAsync(g->d_wptr, s);
-  if (g->d_desc) cudaFreeAsync(g->d_desc, s);
+  if (g->d_rec) cudaFreeAsync(g->d_rec, s);
+  if (g->d_piv) cudaFreeAsync(g->d_piv, s);
+  if (g->d_crow) cudaFreeAsync(g->d_crow, s);
   if (g->d_count) cudaFreeAsync(g->d_count, s);
   delete g;
 }
@@ -190,15 +191,8 @@ int bbtc_ctx_create(int device, bbtc_ctx** out) {
     }
     cudaGetLastError();
   }
-  e = dev_malloc_sync(&c->d_unit_counter, 64 * sizeof(uint32_t));
-  if (e != cudaSuccess) {
-    cudaStreamDestroy(c->stream);
-    delete c;
-    return cuda_fail(e, "cudaMalloc");
-  }
   e = cudaMallocHost(&c->h_stage, kStageBytes);
   if (e != cudaSuccess) {
-    cudaFree(c->d_unit_counter);
     cudaStreamDestroy(c->stream);
     delete c;
     return cuda_fail(e, "cudaMallocHost");
@@ -212,9 +206,10 @@ int bbtc_ctx_destroy(bbtc_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->d_scratch) cudaFreeAsync(ctx->d_scratch, ctx->stream);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  if (ctx->d_unit_counter) cudaFree(ctx->d_unit_counter);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->h_plan_done) cudaEventDestroy(ctx->h_plan_done);
+  for (cudaEvent_t ev : ctx->ev_layout)
+    if (ev) cudaEventDestroy(ev);
   if (ctx->h_plan) cudaFreeHost(ctx->h_plan);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -265,19 +260,10 @@ int bbtc_graph_upload_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_indptr
 int bbtc_graph_free(bbtc_graph* g) {
   if (!g) return BBTC_OK;
   cudaSetDevice(g->ctx->device);
-  cudaStreamSynchronize(g->ctx->stream);
-  for (auto& kv : g->plans) kv.second->release();
   cudaStream_t s = g->ctx->stream;
-  g->fwd.release(s);
-  g->rev.release(s);
-  if (g->d_indptr) cudaFreeAsync(g->d_indptr, s);
-  if (g->d_indices) cudaFreeAsync(g->d_indices, s);
-  if (g->d_words) cudaFreeAsync(g->d_words, s);
-  if (g->d_wptr) cudaFreeAsync(g->d_wptr, s);
-  if (g->d_desc) cudaFreeAsync(g->d_desc, s);
-  if (g->d_count) cudaFreeAsync(g->d_count, s);
   cudaStreamSynchronize(s);
-  delete g;
+  graph_release_on(g, s);
+  cudaStreamSynchronize(s);
   return BBTC_OK;
 }
 
@@ -390,24 +376,25 @@ static int count_async_impl(bbtc_ctx* ctx, bbtc_graph* g, const bbtc_task* tasks
   if (opts) o = *opts; else bbtc_opts_default(&o);
   if (o.mode != BBTC_MODE_PLAIN && o.mode != BBTC_MODE_PERSISTENT) return fail(BBTC_ERR_ARG, "unknown mode");
   if (o.kernel < BBTC_KERNEL_AUTO || o.kernel > BBTC_KERNEL_FUSED) return fail(BBTC_ERR_ARG, "unknown kernel");
-  // The fused task rows count the whole task list at once.  A caller that
+  // The fused count takes the whole task list at once.  A caller that
   // passes the whole list (the reference's driver does, in its cost order)
   // gets them too: the sum does not depend on the order, and with one device
   // queue the border only orders the queue.
   const bool whole = !tasks || is_full_task_list(g->P, tasks, ntasks);
   if (o.kernel == BBTC_KERNEL_FUSED && !whole)
-    return fail(BBTC_ERR_ARG, "fused task rows run the whole task list: pass tasks = NULL or every task once");
+    return fail(BBTC_ERR_ARG, "a fused count runs the whole task list: pass tasks = NULL or every task once");
   const bool fused = whole && (o.kernel == BBTC_KERNEL_FUSED ||
                                (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT));
   BBTC_CUDA(cudaSetDevice(ctx->device));
-  if (!fused) BBTC_TRY(ensure_fwd(g));  // task-list counting reads the forward block CSR
   std::vector<std::vector<bbtc_task>> tl(1);
-  // fused task rows run every task whatever the order: no sort (it would need the forward tiles)
-  if (tasks) tl[0].assign(tasks, tasks + ntasks); else tl[0] = default_tasks(g, !fused && o.sort_tasks != 0);
+  if (!fused) {  // task-list counting reads the block CSRs; a fused count runs every task and needs no list
+    BBTC_TRY(o.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(g) : ensure_tiles(g));
+    if (tasks) tl[0].assign(tasks, tasks + ntasks); else tl[0] = default_tasks(g, o.sort_tasks != 0);
+  }
   // border b >= 0: tasks [0, b) are queued ahead of the rest; with one device queue in list
   // order that is the list order itself, so the value only has to be in range.
   std::vector<bbtc_graph*> gs{g};
-  const std::string key = plan_key(gs, tl, o);
+  const std::string key = fused ? plan_key(gs, {}, o) : plan_key(gs, tl, o);
   auto it = g->plans.find(key);
   const bool reuse = it != g->plans.end();
   if (!reuse) {
@@ -437,9 +424,10 @@ int bbtc_count_wait(bbtc_ctx* ctx, bbtc_graph* g, uint64_t* out) {
   if (!ctx || !g || !out) return fail(BBTC_ERR_ARG, "NULL argument");
   BBTC_CUDA(cudaSetDevice(ctx->device));
   uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut);
-  BBTC_CUDA(cudaMemcpyAsync(h, g->d_count, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  BBTC_TRY(staging_status(ctx));  // synchronises the stream
-  *out = *h;
+  BBTC_CUDA(cudaMemcpyAsync(h, g->d_count, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  BBTC_CUDA(cudaStreamSynchronize(ctx->stream));
+  BBTC_TRY(control_status(h[1]));
+  *out = h[0];
   return BBTC_OK;
 }
 
@@ -535,14 +523,16 @@ int bbtc_count_batch(bbtc_ctx* ctx, bbtc_graph* const* graphs, uint32_t ng, cons
   BBTC_CUDA(cudaSetDevice(ctx->device));
   std::vector<bbtc_graph*> gs(graphs, graphs + ng);
   std::vector<std::vector<bbtc_task>> tl(ng);
-  const bool fused_all = o.kernel == BBTC_KERNEL_FUSED || (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
+  const bool fused = o.kernel == BBTC_KERNEL_FUSED || (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
   for (uint32_t i = 0; i < ng; i++) {
     if (!gs[i] || gs[i]->ctx != ctx) return fail(BBTC_ERR_ARG, "graph is NULL or belongs to another context");
-    if (!fused_all) BBTC_TRY(ensure_fwd(gs[i]));
-    tl[i] = default_tasks(gs[i], !fused_all && o.sort_tasks != 0);
+    if (fused) continue;
+    BBTC_TRY(o.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(gs[i]) : ensure_tiles(gs[i]));
+    tl[i] = default_tasks(gs[i], o.sort_tasks != 0);
   }
   uint64_t* d_outs = nullptr;
-  BBTC_CUDA(dev_malloc(&d_outs, ng * sizeof(uint64_t), ctx->stream));
+  const size_t bytes = ((size_t)ng + 1) * sizeof(uint64_t);  // the counts and the control word
+  BBTC_CUDA(dev_malloc(&d_outs, bytes, ctx->stream));
   struct F {
     uint64_t* p;
     cudaStream_t s;
@@ -550,17 +540,20 @@ int bbtc_count_batch(bbtc_ctx* ctx, bbtc_graph* const* graphs, uint32_t ng, cons
   } guard{d_outs, ctx->stream};
   Plan plan;
   o.use_cuda_graph = 0;
-  // one queue for all graphs: tasks of every graph merged by cost, heaviest first
-  const bool fused = o.kernel == BBTC_KERNEL_FUSED || (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
+  // one queue for all graphs, heaviest first
   int rc = count_enqueue(ctx, gs, tl, o, fused, d_outs, &plan, false);
   if (rc == BBTC_OK) {
-    const bool staged = (size_t)ng * sizeof(uint64_t) <= kStageBytes - kStageOut;
-    uint64_t* h = staged ? reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut) : outs;
-    cudaError_t e = cudaMemcpyAsync(h, d_outs, ng * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream);
+    std::vector<uint64_t> big;
+    uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut);
+    if (bytes > kStageBytes - kStageOut) {
+      big.resize(ng + 1);
+      h = big.data();
+    }
+    cudaError_t e = cudaMemcpyAsync(h, d_outs, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "batch readback");
-    else rc = staging_status(ctx);
-    if (rc == BBTC_OK && staged) std::memcpy(outs, h, ng * sizeof(uint64_t));
+    else rc = control_status(h[ng]);
+    if (rc == BBTC_OK) std::memcpy(outs, h, ng * sizeof(uint64_t));
   }
   for (uint32_t i = 0; i < ng; i++) gs[i]->last_launches = plan.launches;
   plan.release();

@@ -16,18 +16,11 @@
 //   u-centric (the reference's row order, BBTC_KERNEL_MERGE): pivot = ac[r],
 //     the rows bc[b] for b in ab[r] are streamed against it.
 //
-// Fused task rows (persistent form over the whole task list): the tasks
-// (i, j, k) for all k >= j share their ab tile, and their sum over k is
-// sum_{(u, v) in ab} |N+(u) ∩ N+(v) ∩ [cuts[j], ∞)|.  One pass over the
-// reversed tile (j, i) takes it: per pivot v the row N+(v) from cuts[j] on
-// (for a CSR oriented from lower to higher ids, the whole row) is the
-// structure, and per in-edge (u, v) the ids of N+(u) that can meet it are
-// streamed -- their range is stored with the in-edge, so no row pointer is
-// chased.  This visits each edge once instead of once per k.
+// The whole task list at once runs as pivot lists instead (fused.cu).
 //
-// Membership structures: a bitmap (of the column part, or of the pivot row's
-// id span), a sorted copy searched by bisection, or -- for pivot rows longer
-// than the shared buffer -- bisection in global memory.
+// Membership structures: a bitmap of the column part, a sorted copy searched
+// by bisection, or -- for pivot rows longer than the shared buffer -- bisection
+// in global memory.
 //
 // Work units are runs of `unit_edges` consecutive entries of the rows tile.
 // In the persistent form every warp of a grid sized to the SM count claims
@@ -36,6 +29,7 @@
 // Inside a unit the rows met by 32 entries are concatenated and walked 32
 // consecutive ids at a time (see probe_entries).
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstring>
 #include <mutex>
@@ -48,10 +42,8 @@ namespace bbtc {
 namespace {
 
 constexpr uint32_t FULL = 0xffffffffu;
-// per warp after its bitmap: 33 segment starts, 32 bases, a pad word and the
-// 8-byte aligned FusedFrame (28 words), rounded up to an even count
+// per warp after its bitmap: 33 segment starts, 32 bases and the staging state
 constexpr uint32_t kSegWords = 96;
-constexpr uint32_t kFrameOffset = 66;  // words after the bitmap
 // per-warp bulk-staging state of the per-task kernels, after the bitmap:
 // an mbarrier (8 bytes) at kBarOffset, its phase bit and a "staging off" flag
 constexpr uint32_t kBarOffset = 92;
@@ -61,7 +53,6 @@ constexpr uint32_t kStageMin = 64;         // pivot rows this long or longer are
 constexpr uint32_t kWaitLimit = 1u << 20;  // try_wait polls before a staging copy is given up
 // values of the warp's staging flag (state[kStageOffFlag])
 constexpr uint32_t kStageOn = 0, kStageOff = 1, kStageDead = 2;
-constexpr uint32_t kSplitList = 128; // split pivots: room for the ids below the bitmap window
 
 // ---- bulk copies into shared memory (cp.async.bulk + mbarrier) ------------
 
@@ -124,8 +115,6 @@ struct PivotView {
   uint32_t base;  // bitmap bit 0 <-> id `base`
   uint32_t cap;   // a bit of the warp's last buffer word, which stays zero
   uint32_t first, last;
-  const uint32_t* res;  // split kind: the pivot ids below `base`, sorted
-  uint32_t rlen;
 };
 
 // First p in [from, n) with a[p] >= x (n if none) for a sorted a, given
@@ -161,14 +150,6 @@ __device__ __forceinline__ uint32_t member(const uint32_t* bm, const PivotView& 
     // always-zero last word: no branch
     const uint32_t y = min(x - pv.base, pv.cap);
     return (bm[y >> 5] >> (y & 31)) & 1u;
-  } else if constexpr (KIND == kPivotSplit) {
-    if (x >= pv.base) {
-      const uint32_t y = min(x - pv.base, pv.cap);
-      return (bm[y >> 5] >> (y & 31)) & 1u;
-    }
-    if (x < pv.first) return 0;
-    const uint32_t p = lower_bound_u32(pv.res, pv.rlen, x);
-    return (p < pv.rlen && pv.res[p] == x) ? 1u : 0u;
   } else if constexpr (KIND == kPivotList) {
     if (x < pv.first || x > pv.last) return 0;
     const uint32_t p = lower_bound_u32(bm, pv.len, x);
@@ -177,40 +158,6 @@ __device__ __forceinline__ uint32_t member(const uint32_t* bm, const PivotView& 
     if (x < pv.first || x > pv.last) return 0;
     const uint32_t p = lower_bound_u32(pv.row, pv.len, x);
     return (p < pv.len && pv.row[p] == x) ? 1u : 0u;
-  }
-}
-
-// Hits of one word-compressed pair (32-id word w.x, bit mask w.y).  The
-// bitmap kinds use a word-aligned base, so a pair meets one bitmap word; ids
-// below a split pivot's window, and the list kinds, test the set bits one by one.
-template <uint32_t KIND>
-__device__ __forceinline__ uint32_t member_word(const uint32_t* bm, const PivotView& pv, uint2 w) {
-  if constexpr (KIND == kPivotBitmap) {
-    const uint32_t yw = min(w.x - (pv.base >> 5), pv.cap >> 5);
-    return __popc(w.y & bm[yw]);
-  } else if constexpr (KIND == kPivotRank) {
-    // pv.base: the pivot's first word; pv.cap: its span in words; bm: one
-    // (presence bits, index of the block's first pair) entry per 32 words;
-    // pv.res: the pivot's masks in pair order.  A word the pivot lacks costs
-    // one 8-byte load.
-    const uint32_t rel = w.x - pv.base;  // words below the first wrap high
-    if (rel >= pv.cap) return 0;
-    const uint2 e = reinterpret_cast<const uint2*>(bm)[rel >> 5];
-    const uint32_t bit = 1u << (rel & 31);
-    if (!(e.x & bit)) return 0;
-    return __popc(w.y & pv.res[e.y + __popc(e.x & (bit - 1u))]);
-  } else {
-    if constexpr (KIND == kPivotSplit) {
-      if (w.x >= (pv.base >> 5)) return __popc(w.y & bm[min(w.x - (pv.base >> 5), pv.cap >> 5)]);
-    }
-    uint32_t hits = 0;
-    uint32_t mask = w.y;
-    while (mask) {
-      const uint32_t x = (w.x << 5) | (uint32_t)(__ffs(mask) - 1);
-      mask &= mask - 1;
-      hits += member<KIND>(bm, pv, x);
-    }
-    return hits;
   }
 }
 
@@ -224,15 +171,6 @@ struct TileSegs {  // per task: the probe tile's row r = rows.col[q]
     len = rp[r + 1] - start;
   }
 };
-struct RecSegs {  // fused: the stored (start, end) of N+(u) after v
-  const uint2* __restrict__ rec;
-  __device__ __forceinline__ void get(uint32_t q, uint32_t& start, uint32_t& len) const {
-    const uint2 r = rec[q];
-    start = r.x;
-    len = r.y - r.x;
-  }
-};
-
 // Probe the rows met by entries [e, ee) against the pivot structure; returns
 // this lane's hit count.
 //
@@ -243,7 +181,7 @@ struct RecSegs {  // fused: the stored (start, end) of N+(u) after v
 // shared memory) and moves it forward when its id passes the row's end --
 // less than once per window on average -- so the owner costs one compare per
 // id.  Four windows are loaded before any is tested.
-template <uint32_t KIND, bool WORDS, class Segs>
+template <uint32_t KIND, class Segs>
 __device__ __forceinline__ uint32_t probe_entries(const Segs& segs, uint32_t e, uint32_t ee,
                                                   const uint32_t* __restrict__ prb_col, const uint32_t* bm,
                                                   uint32_t* sstart, uint32_t* sbase, const PivotView& pv,
@@ -275,63 +213,41 @@ __device__ __forceinline__ uint32_t probe_entries(const Segs& segs, uint32_t e, 
     uint32_t bs = sbase[owner];
     uint32_t gown = 0xffffffffu, gpos = 0;  // global kind: probe row and position of the last search
     for (uint32_t c = 0; c < total; c += 128) {
-      if constexpr (WORDS) {
-        const uint2* __restrict__ words = reinterpret_cast<const uint2*>(prb_col);
-        uint2 x[4];
-        bool ok[4];
+      uint32_t x[4];
+      bool ok[4];
+      uint32_t own[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t id = c + 32u * k + lane;
+        ok[k] = id < total;
+        x[k] = 0;
+        if (ok[k]) {
+          while (id >= nb) {
+            owner++;
+            nb = sstart[owner + 1];
+            bs = sbase[owner];
+          }
+          x[k] = __ldg(prb_col + bs + id);
+        }
+        own[k] = owner;
+      }
+      if constexpr (KIND == kPivotGlobal) {
+        // galloping search in the pivot row from this lane's last position
+        // in the same probe row (ids of one row come in increasing order)
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          const uint32_t id = c + 32u * k + lane;
-          ok[k] = id < total;
-          x[k] = make_uint2(0, 0);
-          if (ok[k]) {
-            while (id >= nb) {
-              owner++;
-              nb = sstart[owner + 1];
-              bs = sbase[owner];
-            }
-            x[k] = __ldg(words + bs + id);
+          if (!ok[k]) continue;
+          if (own[k] != gown) {
+            gown = own[k];
+            gpos = 0;
           }
+          if (x[k] < pv.first || x[k] > pv.last) continue;
+          gpos = gallop_lb(pv.row, pv.len, gpos, x[k]);
+          hits += (gpos < pv.len && pv.row[gpos] == x[k]) ? 1u : 0u;
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++) hits += ok[k] ? member_word<KIND>(bm, pv, x[k]) : 0u;
       } else {
-        uint32_t x[4];
-        bool ok[4];
-        uint32_t own[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const uint32_t id = c + 32u * k + lane;
-          ok[k] = id < total;
-          x[k] = 0;
-          if (ok[k]) {
-            while (id >= nb) {
-              owner++;
-              nb = sstart[owner + 1];
-              bs = sbase[owner];
-            }
-            x[k] = __ldg(prb_col + bs + id);
-          }
-          own[k] = owner;
-        }
-        if constexpr (KIND == kPivotGlobal) {
-          // galloping search in the pivot row from this lane's last position
-          // in the same probe row (ids of one row come in increasing order)
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            if (!ok[k]) continue;
-            if (own[k] != gown) {
-              gown = own[k];
-              gpos = 0;
-            }
-            if (x[k] < pv.first || x[k] > pv.last) continue;
-            gpos = gallop_lb(pv.row, pv.len, gpos, x[k]);
-            hits += (gpos < pv.len && pv.row[gpos] == x[k]) ? 1u : 0u;
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; k++) hits += ok[k] ? member<KIND>(bm, pv, x[k]) : 0u;
-        }
+        for (int k = 0; k < 4; k++) hits += ok[k] ? member<KIND>(bm, pv, x[k]) : 0u;
       }
     }
     __syncwarp();
@@ -340,28 +256,15 @@ __device__ __forceinline__ uint32_t probe_entries(const Segs& segs, uint32_t e, 
 }
 
 // Build the pivot structure, probe entries [e, ee), restore the buffer to zero.
-// Split kind: ids >= base go to a bitmap of `words` words, the first `rlen`
-// ids of the row (those below base) to a sorted list after the zero word.
-template <uint32_t KIND, bool WORDS, class Segs>
+template <uint32_t KIND, class Segs>
 __device__ __forceinline__ uint32_t pivot_pass(const uint32_t* __restrict__ prow, uint32_t pd, uint32_t base,
-                                               uint32_t words, uint32_t rlen, const Segs& segs, uint32_t e,
+                                               uint32_t words, const Segs& segs, uint32_t e,
                                                uint32_t ee, const uint32_t* __restrict__ prb_col, uint32_t* bm,
                                                uint32_t* sstart, uint32_t* sbase, uint32_t lane) {
-  uint32_t* res = bm + words + 1;
   if constexpr (KIND == kPivotBitmap) {
     for (uint32_t i = lane; i < pd; i += 32) {
       const uint32_t y = prow[i] - base;
       atomicOr(&bm[y >> 5], 1u << (y & 31));
-    }
-  } else if constexpr (KIND == kPivotSplit) {
-    for (uint32_t i = lane; i < pd; i += 32) {
-      const uint32_t x = prow[i];
-      if (i < rlen) {
-        res[i] = x;
-      } else {
-        const uint32_t y = x - base;
-        atomicOr(&bm[y >> 5], 1u << (y & 31));
-      }
     }
   } else if constexpr (KIND == kPivotList) {
     for (uint32_t i = lane; i < pd; i += 32) bm[i] = prow[i];
@@ -374,9 +277,7 @@ __device__ __forceinline__ uint32_t pivot_pass(const uint32_t* __restrict__ prow
   pv.cap = words * 32;  // callers keep words < the buffer size, so word `words` is never set
   pv.first = prow[0];
   pv.last = prow[pd - 1];
-  pv.res = res;
-  pv.rlen = rlen;
-  const uint32_t hits = probe_entries<KIND, WORDS>(segs, e, ee, prb_col, bm, sstart, sbase, pv, lane);
+  const uint32_t hits = probe_entries<KIND>(segs, e, ee, prb_col, bm, sstart, sbase, pv, lane);
   // the buffer is all-zero between pivots whatever kind used it last: the
   // persistent queue hands one warp bitmap and list work in any order
   __syncwarp();
@@ -386,13 +287,6 @@ __device__ __forceinline__ uint32_t pivot_pass(const uint32_t* __restrict__ prow
     } else {
       for (uint32_t i = lane; i < words; i += 32) bm[i] = 0;
     }
-  } else if constexpr (KIND == kPivotSplit) {
-    if (pd - rlen < words) {
-      for (uint32_t i = lane + rlen; i < pd; i += 32) bm[(prow[i] - base) >> 5] = 0;
-    } else {
-      for (uint32_t i = lane; i < words; i += 32) bm[i] = 0;
-    }
-    for (uint32_t i = lane; i < rlen; i += 32) res[i] = 0;
   } else if constexpr (KIND == kPivotList) {
     for (uint32_t i = lane; i < pd; i += 32) bm[i] = 0;
   }
@@ -493,10 +387,8 @@ __device__ __forceinline__ bool staged_pass(const uint32_t* __restrict__ tile_co
   pv.cap = words * 32;
   pv.first = ids[0];
   pv.last = ids[pd - 1];
-  pv.res = nullptr;
-  pv.rlen = 0;
   const uint32_t hits =
-      probe_entries<KIND, false>(segs, e, ee, prb_col, KIND == kPivotList ? ids : bm, sstart, sbase, pv, lane);
+      probe_entries<KIND>(segs, e, ee, prb_col, KIND == kPivotList ? ids : bm, sstart, sbase, pv, lane);
   __syncwarp();
   // back to an all-zero buffer: the bitmap words the ids set, then the staged span
   if constexpr (KIND == kPivotBitmap) {
@@ -554,109 +446,18 @@ __device__ __noinline__ unsigned long long task_unit(const DevTask& tk, uint32_t
         case kPivotBitmap:
           if (!staged_pass<kPivotBitmap>(p_col, ps, pd, tk.words, segs, e, ee, tk.probe.col, bm, bm_words, sstart,
                                          sbase, lane, err, dbg, acc))
-            acc += pivot_pass<kPivotBitmap, false>(prow, pd, 0, tk.words, 0, segs, e, ee, tk.probe.col, bm, sstart,
+            acc += pivot_pass<kPivotBitmap>(prow, pd, 0, tk.words, segs, e, ee, tk.probe.col, bm, sstart,
                                                    sbase, lane);
           break;
         case kPivotList:
           if (!staged_pass<kPivotList>(p_col, ps, pd, 0, segs, e, ee, tk.probe.col, bm, bm_words, sstart, sbase, lane,
                                        err, dbg, acc))
-            acc += pivot_pass<kPivotList, false>(prow, pd, 0, 0, 0, segs, e, ee, tk.probe.col, bm, sstart, sbase, lane);
+            acc += pivot_pass<kPivotList>(prow, pd, 0, 0, segs, e, ee, tk.probe.col, bm, sstart, sbase, lane);
           break;
         default:
-          acc += pivot_pass<kPivotGlobal, false>(prow, pd, 0, 0, 0, segs, e, ee, tk.probe.col, bm, sstart, sbase, lane);
+          acc += pivot_pass<kPivotGlobal>(prow, pd, 0, 0, segs, e, ee, tk.probe.col, bm, sstart, sbase, lane);
       }
       if (staging_dead(bm, bm_words)) return acc;
-    }
-    e = ee;
-    if (e < e1) b = next_row(r_rp, H, b, e, lane);
-  }
-  return acc;
-}
-
-// The pivot of a fused task row (i, j): the tasks (i, j, k >= j) count the
-// common neighbours w of an in-edge (u, v) with w in column parts k >= j,
-// i.e. w >= lo = cuts[j] (the reference's tiles ac = (i, k), bc = (j, k),
-// src/triangle_counting/gpu_sparse_kernel.cu:25-46).  Drops the ids of
-// N+(v) below lo from the pivot row [ps, ps + pd) and from its word pairs
-// [ws, ws + wn); mask0 clears the dropped ids that share the first kept
-// pair's word.  Called only when N+(v) starts below lo, which a CSR oriented
-// from lower to higher ids never does (every id of N+(v) exceeds v >= lo).
-__device__ __noinline__ void pivot_suffix(const uint32_t* __restrict__ gi, const uint2* __restrict__ gw, uint32_t lo,
-                                          uint32_t& ps, uint32_t& pd, uint32_t& ws, uint32_t& wn, uint32_t& mask0) {
-  const uint32_t k = lower_bound_u32(gi + ps, pd, lo);
-  ps += k;
-  pd -= k;
-  if (pd == 0) {
-    wn = 0;
-    return;
-  }
-  const uint32_t first = gi[ps];
-  // first pair whose word holds `first` (a row's pair words strictly increase)
-  uint32_t lo_p = 0, n = wn;
-  while (n > 0) {
-    const uint32_t half = n >> 1;
-    if (gw[ws + lo_p + half].x < (first >> 5)) {
-      lo_p += half + 1;
-      n -= half + 1;
-    } else {
-      n = half;
-    }
-  }
-  ws += lo_p;
-  wn -= lo_p;
-  mask0 = FULL << (first & 31);
-}
-
-// One fused task-row unit: in-edges [unit*K, ...) of the reversed tile (j, i).
-__device__ __noinline__ unsigned long long fused_unit(const DevTask& tk, uint32_t unit, uint32_t* bm,
-                                                      uint32_t* sstart, uint32_t* sbase, uint32_t lane,
-                                                      uint32_t bm_words) {
-  const uint32_t* __restrict__ r_rp = tk.rows.rp;
-  const uint32_t* __restrict__ gp = tk.g_indptr;
-  const uint32_t* __restrict__ gi = tk.g_indices;
-  const RecSegs segs{tk.rows.rec};
-  const uint32_t H = tk.rows.H;
-  const uint64_t e0 = (uint64_t)unit * tk.unit_edges;
-  const uint64_t e1w = e0 + tk.unit_edges;
-  uint32_t e = (uint32_t)e0;
-  const uint32_t e1 = e1w < tk.rows.nnz ? (uint32_t)e1w : tk.rows.nnz;
-  uint32_t b = tk.rows.erow[e >> 5];  // units start at multiples of 32 entries
-  unsigned long long acc = 0;
-  while (e < e1) {
-    const uint32_t ee = min(r_rp[b + 1], e1);
-    const uint32_t v = tk.pivot_base + b;
-    uint32_t ps = gp[v];
-    uint32_t pd = gp[v + 1] - ps;
-    if (pd > 0 && gi[ps] < tk.pivot_base) {
-      // keep the ids in the task columns only (this pivot is built from ids)
-      const uint32_t k = lower_bound_u32(gi + ps, pd, tk.pivot_base);
-      ps += k;
-      pd -= k;
-    }
-    if (pd > 0) {
-      const uint32_t* prow = gi + ps;
-      const uint32_t first = prow[0];
-      const uint32_t last = prow[pd - 1];
-      // word-aligned bitmap: a streamed pair meets exactly one bitmap word
-      const uint32_t base = first & ~31u;
-      const uint32_t span_words = (last >> 5) - (first >> 5) + 1;
-      const uint32_t* gw = reinterpret_cast<const uint32_t*>(tk.g_words);
-      if (span_words < bm_words) {
-        acc += pivot_pass<kPivotBitmap, true>(prow, pd, base, span_words, 0, segs, e, ee, gw, bm, sstart, sbase,
-                                              lane);
-      } else {
-        // bitmap over the top words of the row, the few ids below them in a short list
-        const uint32_t wwords = bm_words - 1 - kSplitList;
-        const uint32_t wbase = ((last >> 5) - (wwords - 1)) << 5;
-        const uint32_t rlen = lower_bound_u32(prow, pd, wbase);
-        if (rlen <= kSplitList)
-          acc += pivot_pass<kPivotSplit, true>(prow, pd, wbase, wwords, rlen, segs, e, ee, gw, bm, sstart, sbase,
-                                               lane);
-        else if (pd <= bm_words)
-          acc += pivot_pass<kPivotList, true>(prow, pd, 0, 0, 0, segs, e, ee, gw, bm, sstart, sbase, lane);
-        else
-          acc += pivot_pass<kPivotGlobal, true>(prow, pd, 0, 0, 0, segs, e, ee, gw, bm, sstart, sbase, lane);
-      }
     }
     e = ee;
     if (e < e1) b = next_row(r_rp, H, b, e, lane);
@@ -668,13 +469,6 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
   return v;
-}
-
-__device__ __forceinline__ unsigned long long dispatch_unit(const DevTask& tk, uint32_t unit, uint32_t* bm,
-                                                            uint32_t* sstart, uint32_t* sbase, uint32_t lane,
-                                                            uint32_t bm_words, uint32_t* err, uint32_t dbg) {
-  if (tk.kind == kFusedRow) return fused_unit(tk, unit, bm, sstart, sbase, lane, bm_words);
-  return task_unit(tk, unit, bm, sstart, sbase, lane, bm_words, err, dbg);
 }
 
 // Persistent form: every warp claims units from one head until the queue is
@@ -705,7 +499,7 @@ __global__ void __launch_bounds__(256, MINB) k_count_queue(const DevTask* __rest
     }
     const DevTask& tk = tasks[lo];
     const unsigned long long c =
-        warp_sum(dispatch_unit(tk, g - prefix[lo], bm, sstart, sbase, lane, bm_words, err, dbg));
+        warp_sum(task_unit(tk, g - prefix[lo], bm, sstart, sbase, lane, bm_words, err, dbg));
     if (lane == 0 && c) atomicAdd(&outs[tk.slot], c);
     if (staging_dead(bm, bm_words)) break;
   }
@@ -726,370 +520,16 @@ __global__ void __launch_bounds__(256, 4) k_count_task(const DevTask* __restrict
   const uint32_t wpb = blockDim.x >> 5;
   unsigned long long acc = 0;
   for (uint32_t u = blockIdx.x * wpb + warp; u < units; u += gridDim.x * wpb) {
-    acc += dispatch_unit(tk, u, bm, sstart, sbase, lane, bm_words, err, dbg);
+    acc += task_unit(tk, u, bm, sstart, sbase, lane, bm_words, err, dbg);
     if (staging_dead(bm, bm_words)) break;
   }
   acc = warp_sum(acc);
   if (lane == 0 && acc) atomicAdd(&outs[tk.slot], acc);
 }
 
-// Fused persistent form.  A unit's loop state lives in a per-warp frame in
-// shared memory while the probe loop runs, so the loop keeps the whole
-// register budget (the persistent kernel runs at 40 registers per thread to
-// keep 48 warps per SM resident; state held in registers across the probe
-// loop would spill to local memory, which misses the small L1 left beside
-// the bitmaps).  Lane 0 writes the frame; every lane reads it back after a
-// __syncwarp.
-struct FusedFrame {
-  const uint32_t* rp;    // reversed tile (j, i): row pointers
-  const uint2* rec;      // its forward-edge records
-  const uint4* desc;     // per vertex: row start, pair start, first id, last id
-  const uint32_t* gi;    // oriented CSR ids
-  const uint2* gw;       // word-compressed rows
-  uint32_t H, e1, b, ee; // rows, unit end, current row, end of the current row's entries
-  uint32_t pivot_base, ps, pd, base, words, rlen, kind, slot;
-  uint32_t ws, wn;       // the pivot row's word pairs
-  uint32_t mask0;        // bits kept of the first pair (pivot_suffix)
-};
-static_assert(sizeof(FusedFrame) <= (kSegWords - kFrameOffset) * sizeof(uint32_t), "frame does not fit");
-
-enum : uint32_t { kNoPivot = 0xffffffffu };
-
-// Choose the pivot structure of row v (ids prow[0..pd)) and record it in the frame.
-// first / last: the row's first and last id.
-__device__ __forceinline__ void fused_choose(volatile FusedFrame* fr, const uint32_t* __restrict__ prow, uint32_t pd,
-                                             uint32_t wn, uint32_t first, uint32_t last, uint32_t bm_words,
-                                             uint32_t lane) {
-  uint32_t kind = kNoPivot, base = 0, words = 0, rlen = 0;
-  if (pd > 0) {
-    const uint32_t span_words = (last >> 5) - (first >> 5) + 1;
-    if (span_words < bm_words) {
-      kind = kPivotBitmap;
-      base = first & ~31u;  // word-aligned: a streamed pair meets exactly one bitmap word
-      words = span_words;
-    } else {
-      // a wide row: a rank bitmap when its block entries (2 words per 32
-      // words of span) and masks (1 per pair) fit the buffer
-      const uint32_t blocks = (span_words + 31) >> 5;
-      if (2 * blocks + wn <= bm_words) {
-        kind = kPivotRank;
-        base = first >> 5;  // first word
-        words = blocks;
-        rlen = span_words;
-      }
-    }
-    if (kind == kNoPivot && span_words >= bm_words) {
-      // bitmap over the top words of the row, the few ids below them in a short list
-      const uint32_t wwords = bm_words - 1 - kSplitList;
-      const uint32_t wbase = ((last >> 5) - (wwords - 1)) << 5;
-      rlen = lower_bound_u32(prow, pd, wbase);
-      if (rlen <= kSplitList) {
-        kind = kPivotSplit;
-        base = wbase;
-        words = wwords;
-      } else {
-        kind = pd <= bm_words ? kPivotList : kPivotGlobal;
-        rlen = 0;
-      }
-    }
-  }
-  if (lane == 0) {
-    fr->pd = pd;
-    fr->kind = kind;
-    fr->base = base;
-    fr->words = words;
-    fr->rlen = rlen;
-  }
-}
-
-template <uint32_t KIND>
-__device__ __forceinline__ void fused_build(const uint32_t* __restrict__ prow, uint32_t pd, uint32_t base,
-                                            uint32_t rlen, uint32_t* bm, uint32_t* res, uint32_t lane) {
-  if constexpr (KIND == kPivotBitmap) {
-    for (uint32_t i = lane; i < pd; i += 32) {
-      const uint32_t y = prow[i] - base;
-      atomicOr(&bm[y >> 5], 1u << (y & 31));
-    }
-  } else if constexpr (KIND == kPivotSplit) {
-    for (uint32_t i = lane; i < pd; i += 32) {
-      const uint32_t x = prow[i];
-      if (i < rlen) {
-        res[i] = x;
-      } else {
-        const uint32_t y = x - base;
-        atomicOr(&bm[y >> 5], 1u << (y & 31));
-      }
-    }
-  } else if constexpr (KIND == kPivotList) {
-    for (uint32_t i = lane; i < pd; i += 32) bm[i] = prow[i];
-  }
-}
-
-// Bitmap of a pivot row from its word pairs: one plain store per 32-id word
-// (a row holds each word once), where setting the bits id by id took one
-// shared-memory atomic per id, serialised on the words that several ids
-// share.  Split kind: only the words of its window (w >= base_w).
-template <uint32_t KIND>
-__device__ __forceinline__ void fused_build_words(const uint2* __restrict__ pw, uint32_t wn, uint32_t base_w,
-                                                  uint32_t mask0, uint32_t* bm, uint32_t lane) {
-  for (uint32_t i = lane; i < wn; i += 32) {
-    const uint2 w = pw[i];
-    if (KIND == kPivotBitmap || w.x >= base_w) bm[w.x - base_w] = i == 0 ? (w.y & mask0) : w.y;
-  }
-}
-
-// Rank pivot from its word pairs (first word fw, `blocks` entries of 32
-// words): pair i sets its presence bit, and the first pair of each block
-// writes its own index as the block's base; masks land in pair order (a
-// row's words strictly increase, so a word's rank is its pair index).
-__device__ __forceinline__ void fused_build_rank(const uint2* __restrict__ pw, uint32_t wn, uint32_t mask0,
-                                                 uint32_t fw, uint32_t blocks, uint32_t* bm, uint32_t lane) {
-  uint32_t* masks = bm + 2 * blocks;
-  for (uint32_t c = 0; c < wn; c += 32) {  // every lane runs every round: the shuffle needs them all
-    const uint32_t i = c + lane;
-    const uint2 w = i < wn ? pw[i] : make_uint2(fw, 0u);
-    uint32_t prev = __shfl_up_sync(FULL, w.x, 1);  // the previous pair's word, from the lane before
-    if (lane == 0 && c > 0) prev = pw[c - 1].x;
-    if (i < wn) {
-      const uint32_t rel = w.x - fw;
-      const uint32_t blk = rel >> 5;
-      atomicOr(&bm[2 * blk], 1u << (rel & 31));
-      if (i == 0 || ((prev - fw) >> 5) != blk) bm[2 * blk + 1] = i;
-      masks[i] = i == 0 ? (w.y & mask0) : w.y;
-    }
-  }
-}
-
-// Back to zero: the entries of the blocks that hold a pair, and the masks.
-__device__ __forceinline__ void fused_clear_rank(const uint2* __restrict__ pw, uint32_t wn, uint32_t fw,
-                                                 uint32_t blocks, uint32_t* bm, uint32_t lane) {
-  uint32_t* masks = bm + 2 * blocks;
-  for (uint32_t i = lane; i < wn; i += 32) {
-    const uint32_t blk = (pw[i].x - fw) >> 5;
-    bm[2 * blk] = 0;
-    bm[2 * blk + 1] = 0;
-    masks[i] = 0;
-  }
-}
-
-template <uint32_t KIND>
-__device__ __forceinline__ void fused_clear_words(const uint2* __restrict__ pw, uint32_t wn, uint32_t base_w,
-                                                  uint32_t words, uint32_t* bm, uint32_t lane) {
-  // a bitmap with at least a third of its words set (or a split window as
-  // many words as the row has pairs) is cleared as a range, stores only;
-  // otherwise the row's words are read again and cleared one by one
-  if ((KIND == kPivotBitmap && 3 * wn >= words) || wn >= words) {
-    for (uint32_t i = lane; i < words; i += 32) bm[i] = 0;
-  } else {
-    for (uint32_t i = lane; i < wn; i += 32) {
-      const uint32_t x = pw[i].x;
-      if (KIND == kPivotBitmap || x >= base_w) bm[x - base_w] = 0;
-    }
-  }
-}
-
-template <uint32_t KIND>
-__device__ __forceinline__ void fused_clear(const uint32_t* __restrict__ prow, uint32_t pd, uint32_t base,
-                                            uint32_t words, uint32_t rlen, uint32_t* bm, uint32_t* res,
-                                            uint32_t lane) {
-  // up to 512 words are cleared as a range (16 stores a lane, no loads);
-  // beyond that, the words of the row's ids, read again
-  if constexpr (KIND == kPivotBitmap) {
-    if (words <= 512 || pd >= words) {
-      for (uint32_t i = lane; i < words; i += 32) bm[i] = 0;
-    } else {
-      for (uint32_t i = lane; i < pd; i += 32) bm[(prow[i] - base) >> 5] = 0;
-    }
-  } else if constexpr (KIND == kPivotSplit) {
-    if (pd - rlen >= words) {
-      for (uint32_t i = lane; i < words; i += 32) bm[i] = 0;
-    } else {
-      for (uint32_t i = lane + rlen; i < pd; i += 32) bm[(prow[i] - base) >> 5] = 0;
-    }
-    for (uint32_t i = lane; i < rlen; i += 32) res[i] = 0;
-  } else if constexpr (KIND == kPivotList) {
-    for (uint32_t i = lane; i < pd; i += 32) bm[i] = 0;
-  }
-}
-
-// Probe entries [e, ee) of the frame's rows tile against the built pivot of kind KIND.
-template <uint32_t KIND>
-__device__ __forceinline__ uint32_t fused_probe(volatile FusedFrame* fr, const uint32_t* __restrict__ prow,
-                                                uint32_t e, uint32_t ee, uint32_t* bm, uint32_t* sstart,
-                                                uint32_t* sbase, uint32_t bm_words, uint32_t lane) {
-  PivotView pv;
-  pv.row = prow;
-  pv.len = fr->pd;
-  pv.base = fr->base;
-  pv.cap = KIND == kPivotRank ? fr->rlen : fr->words * 32;
-  pv.first = KIND == kPivotBitmap || KIND == kPivotRank ? 0u : prow[0];
-  pv.last = KIND == kPivotBitmap || KIND == kPivotRank ? 0u : prow[pv.len - 1];
-  pv.res = KIND == kPivotRank ? bm + 2 * fr->words : bm + fr->words + 1;
-  pv.rlen = fr->rlen;
-  const RecSegs segs{(const uint2*)fr->rec};
-  return probe_entries<KIND, true>(segs, e, ee, reinterpret_cast<const uint32_t*>(fr->gw), bm, sstart, sbase, pv,
-                                   lane);
-}
-
-// Pivots too wide for a span bitmap (split, list, global kinds): a separate
-// function, so their register needs do not weigh on the common bitmap path.
-__device__ __noinline__ uint32_t fused_wide(volatile FusedFrame* fr, uint32_t kind, const uint32_t* prow, uint32_t e,
-                                            uint32_t ee, uint32_t* bm, uint32_t* sstart, uint32_t* sbase,
-                                            uint32_t bm_words, uint32_t lane) {
-  uint32_t* res = bm + fr->words + 1;
-  if (kind == kPivotSplit) {
-    const uint32_t rlen = fr->rlen;
-    for (uint32_t i = lane; i < rlen; i += 32) res[i] = prow[i];
-    fused_build_words<kPivotSplit>((const uint2*)fr->gw + fr->ws, fr->wn, fr->base >> 5, fr->mask0, bm, lane);
-    __syncwarp();
-    return fused_probe<kPivotSplit>(fr, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-  }
-  if (kind == kPivotList) {
-    fused_build<kPivotList>(prow, fr->pd, 0, 0, bm, res, lane);
-    __syncwarp();
-    return fused_probe<kPivotList>(fr, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-  }
-  __syncwarp();
-  return fused_probe<kPivotGlobal>(fr, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-}
-
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_fused_queue(const DevTask* __restrict__ tasks,
-                                                        const uint32_t* __restrict__ prefix, uint32_t ntasks,
-                                                        uint32_t total_units, uint32_t* __restrict__ head,
-                                                        unsigned long long* __restrict__ outs, uint32_t bm_words) {
-  extern __shared__ __align__(16) uint32_t sh[];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* bm = sh + warp * (bm_words + kSegWords);
-  uint32_t* sstart = bm + bm_words;
-  uint32_t* sbase = sstart + 33;
-  volatile FusedFrame* fr = reinterpret_cast<volatile FusedFrame*>(bm + bm_words + kFrameOffset);
-  for (uint32_t i = lane; i < bm_words; i += 32) bm[i] = 0;
-  __syncwarp();
-  while (true) {
-    uint32_t g = 0;
-    if (lane == 0) g = atomicAdd(head, 1u);
-    g = __shfl_sync(FULL, g, 0);
-    if (g >= total_units) break;
-    uint32_t lo = 0, hi = ntasks;  // last t with prefix[t] <= g
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (prefix[mid] <= g) lo = mid; else hi = mid;
-    }
-    const uint32_t first_unit = prefix[lo];
-    if (lane == 0) {
-      const DevTask* tk = tasks + lo;
-      const uint32_t e0 = (g - first_unit) * tk->unit_edges;  // < nnz < 2^32
-      const uint32_t nnz = tk->rows.nnz;
-      fr->rp = tk->rows.rp;
-      fr->rec = tk->rows.rec;
-      fr->desc = tk->g_desc;
-      fr->gi = tk->g_indices;
-      fr->gw = tk->g_words;
-      fr->H = tk->rows.H;
-      fr->e1 = nnz - e0 > tk->unit_edges ? e0 + tk->unit_edges : nnz;
-      fr->b = tk->rows.erow[e0 >> 5];  // units start at multiples of 32 entries
-      fr->ee = e0;
-      fr->pivot_base = tk->pivot_base;
-      fr->slot = tk->slot;
-    }
-    __syncwarp();
-    unsigned long long acc = 0;
-    while (true) {
-      const uint32_t e = fr->ee;
-      if (e >= fr->e1) break;
-      // row b's entries in this unit and its pivot row N+(v), v = pivot_base + b
-      {
-        const uint32_t b = fr->b;
-        const uint32_t ee = min(fr->rp[b + 1], fr->e1);
-        const uint32_t lo = fr->pivot_base;
-        const uint32_t v = lo + b;
-        const uint32_t* gi = fr->gi;
-        // the pivot row's extent in one pair of 16-byte loads
-        const uint4 d0 = fr->desc[v], d1 = fr->desc[v + 1];
-        uint32_t ps = d0.x, pd = d1.x - d0.x, ws = d0.y, wn = d1.y - d0.y;
-        uint32_t first = d0.z;
-        uint32_t mask0 = FULL;
-        // ids of N+(v) below the task columns (never, for a CSR oriented from
-        // lower to higher ids) are left out of the pivot
-        if (pd > 0 && first < lo) {
-          pivot_suffix(gi, (const uint2*)fr->gw, lo, ps, pd, ws, wn, mask0);
-          if (pd > 0) first = gi[ps];
-        }
-        fused_choose(fr, gi + ps, pd, wn, first, d0.w, bm_words, lane);
-        if (lane == 0) {
-          fr->ee = ee;
-          fr->ps = ps;
-          fr->ws = ws;
-          fr->wn = wn;
-          fr->mask0 = mask0;
-        }
-        __syncwarp();
-      }
-      const uint32_t kind = fr->kind;
-      if (kind != kNoPivot) {
-        const uint32_t* prow = fr->gi + fr->ps;
-        const uint32_t ee = fr->ee;
-        uint32_t* res = bm + fr->words + 1;
-        switch (kind) {
-          case kPivotBitmap:
-            fused_build_words<kPivotBitmap>((const uint2*)fr->gw + fr->ws, fr->wn, fr->base >> 5, fr->mask0, bm,
-                                            lane);
-            __syncwarp();
-            acc += fused_probe<kPivotBitmap>(fr, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-            break;
-          case kPivotRank:
-            fused_build_rank((const uint2*)fr->gw + fr->ws, fr->wn, fr->mask0, fr->base, fr->words, bm, lane);
-            __syncwarp();
-            acc += fused_probe<kPivotRank>(fr, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-            break;
-          default:
-            acc += fused_wide(fr, kind, prow, e, ee, bm, sstart, sbase, bm_words, lane);
-        }
-        __syncwarp();
-        // the buffer returns to all-zero for the next pivot, whatever its kind
-        {
-          const uint32_t* prow2 = fr->gi + fr->ps;
-          uint32_t* res2 = bm + fr->words + 1;
-          const uint2* pw = (const uint2*)fr->gw + fr->ws;
-          switch (fr->kind) {
-            case kPivotBitmap: fused_clear_words<kPivotBitmap>(pw, fr->wn, fr->base >> 5, fr->words, bm, lane); break;
-            case kPivotRank: fused_clear_rank(pw, fr->wn, fr->base, fr->words, bm, lane); break;
-            case kPivotSplit: {
-              fused_clear_words<kPivotSplit>(pw, fr->wn, fr->base >> 5, fr->words, bm, lane);
-              const uint32_t rlen = fr->rlen;
-              for (uint32_t i = lane; i < rlen; i += 32) res2[i] = 0;
-              break;
-            }
-            case kPivotList: fused_clear<kPivotList>(prow2, fr->pd, 0, 0, 0, bm, res2, lane); break;
-            default: break;
-          }
-        }
-        __syncwarp();
-      }
-      const uint32_t e2 = fr->ee;
-      if (e2 < fr->e1) {
-        const uint32_t nb = next_row(fr->rp, fr->H, fr->b, e2, lane);
-        if (lane == 0) fr->b = nb;
-      }
-      __syncwarp();
-    }
-    const unsigned long long c = warp_sum(acc);
-    if (lane == 0 && c) atomicAdd(&outs[fr->slot], c);
-  }
-}
-
 size_t smem_bytes(uint32_t bm_words, uint32_t warps) {
   return (size_t)warps * (bm_words + kSegWords) * sizeof(uint32_t);
 }
-
-uint32_t norm_bm_words(uint32_t w) {
-  if (w == 0) w = 1024;
-  w = (w + 3) & ~3u;
-  return std::max<uint32_t>(w, 2 * kSplitList);
-}
-
-uint32_t norm_warps(uint32_t w) { return w == 0 ? 8 : std::min<uint32_t>(std::max<uint32_t>(w, 1), 8); }
 
 }  // namespace
 
@@ -1106,37 +546,86 @@ int kernel_smem_optin(bbtc_ctx* ctx, const bbtc_opts& o) {
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_fused_queue<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_fused_queue<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_fused_queue<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_fused_queue<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_task, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  BBTC_TRY(pivots_smem_optin(sm));
   ctx->smem_set = sm;
   return BBTC_OK;
 }
 
-// Average out-row length of row part i over its tiles (for unit sizing).
-static double part_row_len(const bbtc_graph* g, uint32_t i) {
-  uint64_t z = 0;
-  uint32_t rows = 1;
-  for (uint32_t k = 0; k < g->P; k++) {
-    z += g->rev.nnz[k * g->P + i];  // reversed tile (k, i) holds the edges of forward tile (i, k)
-    if (g->fwd_built) rows = std::max(rows, g->fwd.nerows[i * g->P + k]);
+// Queue of a fused request: its graphs, the largest first.  A graph's units
+// are first single batches of 32 entries, where the layout found short in-lists
+// (a batch there holds many pivots and takes longest), then 8, 4, 2 and 1
+// batches: a larger unit builds its pivot less often (R-MAT s20 1.03 ms with
+// single batches throughout, 0.89 with fours), a smaller one evens out the
+// queue's end, so each size is kept until about two units of it per warp are
+// left.  o.unit_work asks for one size throughout.
+static int make_pivot_plan(const bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs, const bbtc_opts& o, Plan* plan) {
+  uint64_t left = 0;  // batches from the current graph on
+  for (const bbtc_graph* g : graphs) left += (g->m + 31) / 32;
+  const uint64_t warps = (uint64_t)ctx->sms * 40;  // about as many as run at once
+  std::vector<uint32_t> order(graphs.size());
+  for (uint32_t q = 0; q < order.size(); q++) order[q] = q;
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return graphs[a]->m > graphs[b]->m; });
+  plan->tasks.clear();
+  plan->pivots.clear();
+  plan->prefix.assign(1, 0);
+  uint64_t total = 0;
+  for (uint32_t q : order) {
+    const bbtc_graph* g = graphs[q];
+    if (!g->m || !g->npiv) {
+      left -= (g->m + 31) / 32;
+      continue;
+    }
+    PivotGraph d{};
+    d.words = reinterpret_cast<const uint2*>(g->d_words);
+    d.rec = reinterpret_cast<const uint2*>(g->d_rec);
+    d.piv = static_cast<const uint4*>(g->d_piv);
+    d.crow = g->d_crow;
+    d.entries = (uint32_t)g->m;
+    d.npiv = g->npiv;
+    d.plain = g->oriented ? 1 : 0;
+    d.slot = q;
+    const uint64_t batches = (g->m + 31) / 32;  // 64-bit: m may be near 2^32
+    if (o.unit_work) {  // about half a row is streamed per entry
+      const double avg = std::max(1.0, 0.5 * (double)g->m / std::max(1u, g->n));
+      d.level_size[0] = (uint32_t)std::min(512.0, std::max(1.0, std::ceil(o.unit_work / avg / 32)));
+      d.level_units[0] = (uint32_t)((batches + d.level_size[0] - 1) / d.level_size[0]);
+      total += d.level_units[0];
+    } else {
+      const uint64_t sparse = std::min<uint64_t>(g->sparse_end, batches);
+      d.level_size[0] = 1;
+      d.level_units[0] = (uint32_t)sparse;
+      total += sparse;
+      uint64_t rest = batches - sparse, after = left - batches;
+      for (int l = 1; l < kLevels; l++) {
+        const uint64_t size = 1ull << (kLevels - 1 - l);  // 8, 4, 2, 1
+        const uint64_t keep = 2 * warps * size;           // batches that smaller units are kept for
+        uint64_t units = rest + after > keep ? std::min(rest, rest + after - keep) / size : 0;
+        if (l == kLevels - 1) units = rest;
+        d.level_size[l] = (uint32_t)size;
+        d.level_units[l] = (uint32_t)units;
+        total += units;
+        rest -= units * size;
+      }
+    }
+    left -= batches;
+    // every warp claims one unit past the end: leave room in the 32-bit head
+    if (total >= 0xffff0000ull) return fail(BBTC_ERR_UNSUPPORTED, "about 2^32 work units or more in one request");
+    plan->pivots.push_back(d);
+    plan->prefix.push_back((uint32_t)total);
   }
-  if (!g->fwd_built) rows = std::max<uint32_t>(1, g->cuts[i + 1] - g->cuts[i]);
-  return (double)z / rows;
+  plan->total_units = (uint32_t)total;
+  plan->fused = true;
+  return BBTC_OK;
 }
 
-// Build the device task array for a request.  A single graph keeps the
-// caller's task order (its border split); several graphs are merged into one
-// queue ordered by estimated probe work, heaviest first.  With `fused`, every
-// graph's full task list runs as task rows (i, j).
+// Build the device task array for a per-task request.  A single graph keeps
+// the caller's task order (its border split); several graphs are merged into
+// one queue ordered by estimated probe work, heaviest first.
 static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<std::vector<bbtc_task>>& tasks,
-                     const bbtc_opts& o, bool fused, Plan* plan) {
+                     const bbtc_opts& o, Plan* plan) {
   const uint32_t bmw = norm_bm_words(o.bitmap_words);
-  // default unit size: task rows of the fused form run as 32-entry units
-  // (below); explicit task lists as units of ~8192 probes
-  const uint32_t unit_work = o.unit_work ? o.unit_work : (fused ? 256 : 8192);
+  const uint32_t unit_work = o.unit_work ? o.unit_work : 8192;  // units of about 8192 probes
   std::vector<DevTask> list;
   std::vector<double> cost;
   auto add = [&](DevTask d, double avg_probe) {
@@ -1149,25 +638,6 @@ static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<s
   for (size_t gi = 0; gi < graphs.size(); gi++) {
     const bbtc_graph* g = graphs[gi];
     const uint32_t P = g->P;
-    if (fused) {
-      for (uint32_t i = 0; i < P; i++)
-        for (uint32_t j = i; j < P; j++) {
-          if (!g->rev.nnz[j * P + i]) continue;  // forward tile (i, j) is empty
-          DevTask d{};
-          d.rows = dev_tile(g->rev, g->cuts, j, i);
-          d.kind = kFusedRow;
-          d.slot = (uint32_t)gi;
-          d.g_indptr = g->d_indptr;
-          d.g_indices = g->d_indices;
-          d.g_words = reinterpret_cast<const uint2*>(g->d_words);
-          d.g_wptr = g->d_wptr;
-          d.g_desc = static_cast<const uint4*>(g->d_desc);
-          d.pivot_base = g->cuts[j];
-          add(d, 0.5 * part_row_len(g, i));
-          if (!o.unit_work) list.back().unit_edges = 0;  // set below from the request's size
-        }
-      continue;
-    }
     for (const bbtc_task& t : tasks[gi]) {
       if (t.ab >= P * P || t.bc >= P * P || t.ac >= P * P)
         return fail(BBTC_ERR_ARG, "task names a tile outside the P x P grid");
@@ -1199,21 +669,12 @@ static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<s
       add(d, (double)d.probe.nnz / probe_rows);
     }
   }
-  if (fused && !o.unit_work) {
-    // default units of the fused task rows: 32 in-edges (one probe batch), or
-    // 64 when the request has 2^25 in-edges or more -- at R-MAT s22 (64 M)
-    // 64 was 5 % faster, at s20 (16 M) 13 % slower (too few units per warp
-    // to balance the tail)
-    uint64_t entries = 0;
-    for (const DevTask& d : list) entries += d.rows.nnz;
-    const uint32_t K = entries >= (1ull << 25) ? 64 : 32;
-    for (DevTask& d : list) d.unit_edges = K;
-  }
   std::vector<uint32_t> order(list.size());
   for (uint32_t q = 0; q < order.size(); q++) order[q] = q;
-  if (graphs.size() > 1 || fused)
+  if (graphs.size() > 1)
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
   plan->tasks.clear();
+  plan->pivots.clear();
   plan->prefix.assign(1, 0);
   uint64_t total = 0;
   for (uint32_t q : order) {
@@ -1224,17 +685,15 @@ static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<s
     plan->prefix.push_back((uint32_t)total);
   }
   plan->total_units = (uint32_t)total;
-  plan->fused = fused;
+  plan->fused = false;
   return BBTC_OK;
 }
 
 void Plan::release() {
   if (exec) cudaGraphExecDestroy(exec);
-  if (d_tasks) cudaFreeAsync(d_tasks, stream);
-  if (d_prefix) cudaFreeAsync(d_prefix, stream);
+  if (d_queue) cudaFreeAsync(d_queue, stream);
   exec = nullptr;
-  d_tasks = nullptr;
-  d_prefix = nullptr;
+  d_queue = nullptr;
   cap = 0;
 }
 
@@ -1244,71 +703,64 @@ static int enqueue_launches(bbtc_ctx* ctx, Plan* plan, const bbtc_opts& o, uint6
   const uint32_t wpb = norm_warps(o.warps_per_block);
   const size_t sm = smem_bytes(bmw, wpb);
   auto* outs = reinterpret_cast<unsigned long long*>(d_outs);
-  BBTC_CUDA(cudaMemsetAsync(d_outs, 0, nouts * sizeof(uint64_t), s));
-  BBTC_CUDA(cudaMemsetAsync(ctx->d_unit_counter, 0, 2 * sizeof(uint32_t), s));  // queue head, staging flag
+  // the counts and, after them, the control word: queue head, staging flag
+  BBTC_CUDA(cudaMemsetAsync(d_outs, 0, (nouts + 1) * sizeof(uint64_t), s));
+  uint32_t* ctrl = reinterpret_cast<uint32_t*>(d_outs + nouts);
   plan->launches = 0;
-  const uint32_t ntasks = (uint32_t)plan->tasks.size();
+  const uint32_t ntasks = (uint32_t)plan->prefix.size() - 1;
   if (ntasks == 0) return BBTC_OK;
+  const uint32_t* d_prefix = reinterpret_cast<const uint32_t*>(static_cast<const char*>(plan->d_queue) + plan->prefix_at);
+  if (plan->fused) {
+    BBTC_TRY(pivots_launch(ctx, plan->pivots[0], static_cast<const PivotGraph*>(plan->d_queue), d_prefix, ntasks,
+                           plan->total_units, o, d_outs, nouts));
+    plan->launches = 1;
+    return BBTC_OK;
+  }
+  const DevTask* d_tasks = static_cast<const DevTask*>(plan->d_queue);
   if (o.mode == BBTC_MODE_PLAIN) {
     for (uint32_t t = 0; t < ntasks; t++) {
       const uint32_t units = plan->prefix[t + 1] - plan->prefix[t];
       const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((units + wpb - 1) / wpb, ctx->sms * 8));
-      k_count_task<<<grid, wpb * 32, sm, s>>>(plan->d_tasks + t, units, outs, bmw, ctx->d_unit_counter + 1,
-                                              ctx->debug_stage_polls);
+      k_count_task<<<grid, wpb * 32, sm, s>>>(d_tasks + t, units, outs, bmw, ctrl + 1, ctx->debug_stage_polls);
       BBTC_CUDA(cudaGetLastError());
       plan->launches++;
     }
   } else {
-    // the register budget: 4, 5, 6 or 8 resident blocks per SM (the per-task
-    // queue kernel has no 5-block variant and runs 4 there)
-    const uint32_t occ = o.occupancy >= 8 ? 8 : (o.occupancy >= 6 ? 6 : (o.occupancy == 5 ? 5 : 4));
-    auto* fkern = occ == 8 ? k_fused_queue<8>
-                           : (occ == 6 ? k_fused_queue<6> : (occ == 5 ? k_fused_queue<5> : k_fused_queue<4>));
+    // the register budget: 4, 6 or 8 resident blocks per SM
+    const uint32_t occ = o.occupancy >= 8 ? 8 : (o.occupancy >= 6 ? 6 : 4);
     auto* qkern = occ == 8 ? k_count_queue<8> : (occ == 6 ? k_count_queue<6> : k_count_queue<4>);
     int per_sm = 0;
-    if (plan->fused)
-      BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fkern, wpb * 32, sm));
-    else
-      BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qkern, wpb * 32, sm));
+    BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qkern, wpb * 32, sm));
     per_sm = std::max(1, per_sm);
     if (o.blocks_per_sm) per_sm = std::min<int>(per_sm, (int)o.blocks_per_sm);
     // no more blocks than the queue has units for a warp each (a small batch
     // leaves the rest of the GPU to other streams)
     const uint64_t want = ((uint64_t)plan->total_units + wpb - 1) / wpb;
     const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * per_sm, want));
-    if (plan->fused)
-      fkern<<<grid, wpb * 32, sm, s>>>(plan->d_tasks, plan->d_prefix, ntasks, plan->total_units,
-                                       ctx->d_unit_counter, outs, bmw);
-    else
-      qkern<<<grid, wpb * 32, sm, s>>>(plan->d_tasks, plan->d_prefix, ntasks, plan->total_units,
-                                       ctx->d_unit_counter, outs, bmw, ctx->debug_stage_polls);
+    qkern<<<grid, wpb * 32, sm, s>>>(d_tasks, d_prefix, ntasks, plan->total_units, ctrl, outs, bmw,
+                                     ctx->debug_stage_polls);
     BBTC_CUDA(cudaGetLastError());
     plan->launches = 1;
   }
   return BBTC_OK;
 }
 
-int staging_status(bbtc_ctx* ctx) {
-  uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageBad);
-  BBTC_CUDA(cudaMemcpyAsync(h, ctx->d_unit_counter + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  BBTC_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (*h) return fail(BBTC_ERR_TIMEOUT, "a shared-memory staging copy did not complete; the count is void");
+int control_status(uint64_t ctrl) {
+  if (ctrl >> 32) return fail(BBTC_ERR_TIMEOUT, "a shared-memory staging copy did not complete; the count is void");
   return BBTC_OK;
 }
 
-// Options left at 0 ("auto") resolved for the request's graphs.  The
-// bitmap: 1024 words per warp.  Rows wider than that run as rank bitmaps,
-// so a larger buffer only costs occupancy (one B200, ms per count, 512 / 768
-// / 1024 / 1536 / 2048 words: R-MAT s22 7.92 / 7.63 / 7.49 / 8.16 / 9.56;
-// s24 - / - / 41.8 / 46.5 / 56.5).  Occupancy: fused task rows 6 blocks per
-// SM (40 registers) while the bitmap leaves shared memory for them, else 4
-// (64 registers); per-task kernels 4 (R-MAT s20: bitmap 10.4 ms at 4 against
-// 12.4 at 6, search 14.4 / 15.7, merge 27.5 / 31.5).
-static bbtc_opts resolve_opts(const std::vector<bbtc_graph*>& graphs, const bbtc_opts& in, bool fused) {
+// Options left at 0 ("auto") resolved.  The buffer: 1024 words per warp
+// (wider pivots run as rank bitmaps or hashes, so a larger buffer only costs
+// occupancy).  Occupancy: the fused count 5 blocks per SM while the buffer
+// leaves shared memory for them (R-MAT s22 / s20 / Chung-Lu 2^23, ms: 4 blocks
+// 6.19 / 0.95 / 4.99, 5 blocks 5.61 / 0.91 / 4.76, 6 blocks 5.88 / 0.88 /
+// 4.94), else 4 (64 registers); per-task kernels 4 (R-MAT s20: bitmap 10.4 ms
+// at 4 against 12.4 at 6, search 14.4 / 15.7, merge 27.5 / 31.5).
+static bbtc_opts resolve_opts(const bbtc_opts& in, bool fused) {
   bbtc_opts o = in;
-  (void)graphs;
   if (!o.bitmap_words) o.bitmap_words = 1024;
-  if (!o.occupancy) o.occupancy = fused && norm_bm_words(o.bitmap_words) <= 1024 ? 6 : 4;
+  if (!o.occupancy) o.occupancy = fused && norm_bm_words(o.bitmap_words) <= 1024 ? 5 : 4;
   return o;
 }
 
@@ -1317,31 +769,34 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
                   uint64_t* d_outs, Plan* plan, bool reuse) {
   Range range("bbtc count enqueue");
   cudaStream_t s = ctx->stream;
-  const bbtc_opts o = resolve_opts(graphs, in, fused);
+  const bbtc_opts o = resolve_opts(in, fused);
   BBTC_TRY(kernel_smem_optin(ctx, o));
   if (!reuse) {
     if (plan->exec) cudaGraphExecDestroy(plan->exec);
     plan->exec = nullptr;
-    BBTC_TRY(make_plan(graphs, tasks, o, fused, plan));
-    const size_t nt = plan->tasks.size();
+    if (fused) BBTC_TRY(make_pivot_plan(ctx, graphs, o, plan));
+    else BBTC_TRY(make_plan(graphs, tasks, o, plan));
+    // one graph's fused queue rides in the kernel's arguments; other queues are uploaded
+    const size_t nt = fused && plan->pivots.size() == 1 ? 0 : plan->prefix.size() - 1;
     if (nt) {
-      if (nt > plan->cap || plan->stream != s) {
+      const void* items = fused ? static_cast<const void*>(plan->pivots.data()) : plan->tasks.data();
+      const size_t tb = nt * (fused ? sizeof(PivotGraph) : sizeof(DevTask)), pb = (nt + 1) * sizeof(uint32_t);
+      if (tb + pb > plan->cap || plan->stream != s) {
         plan->release();
         plan->stream = s;
-        const size_t cap = std::max<size_t>(nt, 256);
-        if (dev_malloc(&plan->d_tasks, cap * sizeof(DevTask), s) != cudaSuccess ||
-            dev_malloc(&plan->d_prefix, (cap + 1) * sizeof(uint32_t), s) != cudaSuccess) {
+        const size_t cap = std::max<size_t>(tb + pb, 64 << 10);
+        if (dev_malloc(&plan->d_queue, cap, s) != cudaSuccess) {
           cudaGetLastError();
           plan->release();
           return fail(BBTC_ERR_NOMEM, "device allocation of the task queue failed");
         }
         plan->cap = cap;
       }
+      plan->prefix_at = tb;
       // upload from the context's pinned staging (a pageable copy would go
       // through the driver's shared staging buffers, which other threads'
       // copies hold); the context keeps it across plans, since pinning host
       // memory can take milliseconds
-      const size_t tb = nt * sizeof(DevTask), pb = (nt + 1) * sizeof(uint32_t);
       if (ctx->h_plan_done) BBTC_CUDA(cudaEventSynchronize(ctx->h_plan_done));  // the last upload has read it
       if (tb + pb > ctx->h_plan_cap) {
         if (ctx->h_plan) cudaFreeHost(ctx->h_plan);
@@ -1352,10 +807,9 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
         ctx->h_plan_cap = want;
       }
       if (!ctx->h_plan_done) BBTC_CUDA(cudaEventCreateWithFlags(&ctx->h_plan_done, cudaEventDisableTiming));
-      std::memcpy(ctx->h_plan, plan->tasks.data(), tb);
+      std::memcpy(ctx->h_plan, items, tb);
       std::memcpy(ctx->h_plan + tb, plan->prefix.data(), pb);
-      BBTC_CUDA(cudaMemcpyAsync(plan->d_tasks, ctx->h_plan, tb, cudaMemcpyHostToDevice, s));
-      BBTC_CUDA(cudaMemcpyAsync(plan->d_prefix, ctx->h_plan + tb, pb, cudaMemcpyHostToDevice, s));
+      BBTC_CUDA(cudaMemcpyAsync(plan->d_queue, ctx->h_plan, tb + pb, cudaMemcpyHostToDevice, s));
       BBTC_CUDA(cudaEventRecord(ctx->h_plan_done, s));
     }
     plan->captured = false;
@@ -1366,10 +820,11 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
     plan->captured = false;
   }
   plan->stage_polls = ctx->debug_stage_polls;
-  // A plan's first count launches directly: capturing and instantiating a
-  // graph costs more host time than one launch, and pays only on replays,
-  // so the capture waits for the plan's second count.
-  if (!o.use_cuda_graph || !reuse) return enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size());
+  // A plan of one launch is launched directly (a memset and a kernel cost
+  // less host time than a graph launch), and so is any plan's first count:
+  // capturing and instantiating a graph pays only on replays, so the capture
+  // waits for the plan's second count.
+  if (!o.use_cuda_graph || !reuse || plan->fused || o.mode != BBTC_MODE_PLAIN) return enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size());
   if (!plan->captured) {
     cudaGraph_t graph = nullptr;
     BBTC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1495,12 +950,12 @@ __global__ void __launch_bounds__(256, 4) k_count_csr_static(const uint32_t* __r
       const uint32_t first = prow[0], last = prow[pd - 1];
       const uint32_t span_words = last >= first ? ((last - first) >> 5) + 1 : 0xffffffffu;
       if (span_words < bm_words)
-        acc += pivot_pass<kPivotBitmap, false>(prow, pd, first, span_words, 0, segs, e, ee, indices, bm, sstart, sbase,
+        acc += pivot_pass<kPivotBitmap>(prow, pd, first, span_words, segs, e, ee, indices, bm, sstart, sbase,
                                         lane);
       else if (pd <= bm_words)
-        acc += pivot_pass<kPivotList, false>(prow, pd, 0, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
+        acc += pivot_pass<kPivotList>(prow, pd, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
       else
-        acc += pivot_pass<kPivotGlobal, false>(prow, pd, 0, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
+        acc += pivot_pass<kPivotGlobal>(prow, pd, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
       e = ee;
       if (e < e1) u = next_row(indptr, n, u, e, lane);
     }

@@ -77,7 +77,6 @@ constexpr uint64_t kNoSegment = ~0ull;
 struct DevTile {
   const uint32_t* rp;
   const uint32_t* col;
-  const uint2* rec;  // reversed tiles: pair range [word of v, end) in row u, per entry's forward edge (u, v)
   const uint32_t* erow;  // row of entry 32 q, for q < ceil(nnz / 32)
   uint32_t H, W, nnz, maxdeg;
 };
@@ -87,10 +86,6 @@ enum TaskKind : uint32_t {
   kPivotBitmap = 0,  // pivot row -> shared bitmap of the column part, probes test bits
   kPivotList = 1,    // pivot row -> sorted shared list, probes binary-search it
   kPivotGlobal = 2,  // pivot row too long for shared memory: binary search in global memory
-  kFusedRow = 3,     // task row (i, j): all tasks (i, j, k >= j) in one pass, structure chosen per pivot
-  kPivotSplit = 4,   // pivot row -> bitmap of its top id window + short sorted list of the ids below it
-  kPivotRank = 5,    // fused task rows: per 32-word block of the row's span a (presence bits, first pair)
-                     // entry, then the row's masks in pair order (a rank bitmap over the words)
 };
 
 // One queued task: `rows` is the tile whose rows are the pivot vertices and
@@ -103,16 +98,29 @@ struct DevTask {
   DevTile rows;
   DevTile pivot;
   DevTile probe;
-  const uint32_t* g_indptr;   // fused task rows: the resident oriented CSR
-  const uint32_t* g_indices;
-  const uint2* g_words;       // fused: word-compressed rows
-  const uint32_t* g_wptr;     // fused: their row pointers (n + 1)
-  const uint4* g_desc;        // fused: per vertex (row start, pair start, first id, last id), n + 1
-  uint32_t pivot_base;        // fused: first vertex id of part j
   uint32_t kind;
   uint32_t unit_edges;  // entries of `rows` per work unit
   uint32_t slot;        // output counter index
   uint32_t words;       // bitmap words the pivot part needs (ceil(W/32))
+};
+
+// One graph of a fused count: the pivot lists that the layout builds.  Entry
+// q is an in-edge (u, v): rec[q] = (first, end) of the pairs of N+(u) that
+// can meet N+(v).  Pivot k is 8 words: its entries [e0, e1), its row's first
+// pair and number of pairs, first word, span in words, the bits kept of the
+// first pair, the vertex; pivots are in entry order and end with one whose
+// e0 is ~0.  crow[x] = the first pivot with entries past 32 x.
+constexpr int kLevels = 5;
+struct PivotGraph {
+  const uint2* words;  // (32-id word, bit mask) pairs of the rows
+  const uint2* rec;
+  const uint4* piv;
+  const uint32_t* crow;
+  uint32_t entries;
+  uint32_t npiv;
+  uint32_t level_units[kLevels], level_size[kLevels];  // work units in queue order: counts, batches of 32 entries each
+  uint32_t slot;        // output counter index
+  uint32_t plain;       // 1: every pivot keeps its whole row (all bits of its first pair)
 };
 
 // A block CSR over one cut vector, for the forward or the reversed graph.
@@ -122,7 +130,6 @@ struct BlockTiles {
   std::vector<uint64_t> rp_off, col_off;      // element offsets, kNoSegment when empty
   uint32_t* d_rp = nullptr;                    // row-pointer pool
   uint32_t* d_col = nullptr;                   // column pool
-  void* d_rec = nullptr;                       // reversed tiles: forward-edge records (uint2), col-aligned
   uint32_t* d_erow = nullptr;                  // row index of every 32nd entry, per tile
   size_t rp_len = 0, col_len = 0, erow_len = 0;
   cudaStream_t stream = nullptr;
@@ -130,15 +137,16 @@ struct BlockTiles {
 };
 
 struct Plan {
-  std::vector<DevTask> tasks;      // host copy
-  std::vector<uint32_t> prefix;    // unit prefix, ntasks + 1
-  DevTask* d_tasks = nullptr;      // stream-ordered, reused while large enough
-  uint32_t* d_prefix = nullptr;
-  size_t cap = 0;                  // tasks the device buffers hold
+  std::vector<DevTask> tasks;      // host copy: the tasks, or
+  std::vector<PivotGraph> pivots;  // the graphs of a fused count
+  std::vector<uint32_t> prefix;    // unit prefix, one more than items
+  void* d_queue = nullptr;         // items and prefix; stream-ordered, reused while large enough
+  size_t cap = 0;                  // bytes the device buffer holds
+  size_t prefix_at = 0;            // byte offset of the prefix
   cudaStream_t stream = nullptr;   // stream the buffers were allocated on
   uint32_t total_units = 0;
   uint32_t launches = 0;
-  bool fused = false;              // every task is a fused task row
+  bool fused = false;              // pivot lists (fused.cu)
   cudaGraphExec_t exec = nullptr;
   bool captured = false;
   uint32_t stage_polls = 0;        // the context's staging test hook when the launch was captured
@@ -152,7 +160,6 @@ struct bbtc_ctx {
   cudaStream_t stream = nullptr;
   int sms = 0;
   size_t smem_optin = 0;
-  uint32_t* d_unit_counter = nullptr;  // persistent-queue head (one word per launch slot)
   size_t smem_set = 0;                 // dynamic shared memory the count kernels are opted in to
   bool open_carveout = false;          // layout kernels ask for the largest shared-memory carveout (launch_layout)
   uint32_t layout_blocks_per_sm = 8;   // grid cap of the layout kernels (256 threads a block)
@@ -171,6 +178,7 @@ struct bbtc_ctx {
   char* h_plan = nullptr;
   size_t h_plan_cap = 0;
   cudaEvent_t h_plan_done = nullptr;  // recorded after the last upload from h_plan
+  cudaEvent_t ev_layout[2] = {nullptr, nullptr};  // start and end of the last layout build
   // Layout scratch kept between builds (bbtc::Scratch), at most kScratchKeep bytes.
   char* d_scratch = nullptr;
   size_t scratch_cap = 0;
@@ -230,10 +238,10 @@ inline int dalloc(DevBuf& b, size_t bytes, cudaStream_t s) {
 
 // Regions of bbtc_ctx::h_stage (one graph build or count at a time per context).
 constexpr size_t kStageBytes = 1u << 20;
-constexpr size_t kStageCuts = 0;          // cut vector and a flags word, <= (64 + 2) x 4 bytes
-constexpr size_t kStageBad = 3072;        // validation flags
-constexpr size_t kStageOff[2] = {4096, 40960};  // per block CSR: tile + part row offsets (<= 33,288 bytes)
-constexpr size_t kStageStats = 81920;     // tile statistics of both block CSRs (<= 163,840 bytes)
+constexpr size_t kStageCuts = 0;          // cut vector, <= (64 + 2) x 4 bytes
+constexpr size_t kStageFlags = 3072;      // contract flags and totals of a layout build; small read-backs
+constexpr size_t kStageOff = 4096;        // tile + part row offsets of a block CSR (<= 33,288 bytes)
+constexpr size_t kStageStats = 81920;     // its tile statistics (<= 81,920 bytes)
 constexpr size_t kStageOut = 262144;      // counts read back (<= 98,304 of them)
 
 }  // namespace bbtc
@@ -246,13 +254,20 @@ struct bbtc_graph {
   uint32_t* d_indptr = nullptr;   // resident oriented CSR (global ids)
   uint32_t* d_indices = nullptr;
   void* d_words = nullptr;        // word-compressed rows: (word, mask) uint2 pairs
-  uint32_t* d_wptr = nullptr;     // n + 1 pair offsets
-  void* d_desc = nullptr;         // n + 1 pivot descriptors (uint4): row start, pair start, first id, last id
-  bbtc::BlockTiles fwd, rev;
-  uint64_t* d_count = nullptr;  // result slot
+  uint64_t nwords = 0;            // pairs
+  void* d_rec = nullptr;          // pivot lists (PivotGraph): one uint2 per in-edge
+  void* d_piv = nullptr;          // npiv + 1 pivots of 32 bytes
+  uint32_t* d_crow = nullptr;     // pivot of every 32nd entry
+  uint32_t npiv = 0;
+  uint64_t nentry_rows = 0;       // words of d_crow
+  uint32_t sparse_end = 0;        // 32-entry batches up to which pivots have few in-edges
+  bool oriented = false;          // every id exceeds its row's
+  bbtc::BlockTiles fwd, rev;      // tiles of the per-task kernels, built on first use
+  uint64_t* d_count = nullptr;  // the count and its control word
   uint64_t device_bytes = 0;
   double layout_ms = 0;
   bool fwd_built = false;         // the forward block CSR is built on first use (task-list counting, tile stats)
+  bool rev_built = false;         // the reversed one too (v-centric task-list counting)
   bool zero_copy = false;         // the upload read the host CSR with a kernel (no copy-engine transfer)
   uint32_t last_launches = 0;
   std::map<std::string, std::unique_ptr<bbtc::Plan>> plans;  // cached queues keyed by request
@@ -266,6 +281,8 @@ namespace bbtc {
 int build_layout(bbtc_graph* g, const uint32_t* indptr, const uint32_t* indices, bool host);
 // Build g's forward block CSR if it is not built yet (on g's context stream; synchronises it).
 int ensure_fwd(bbtc_graph* g);
+// The same for both block CSRs.
+int ensure_tiles(bbtc_graph* g);
 DevTile dev_tile(const BlockTiles& t, const std::vector<uint32_t>& cuts, uint32_t x, uint32_t y);
 
 // count.cu
@@ -273,9 +290,23 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
                   const std::vector<std::vector<bbtc_task>>& tasks, const bbtc_opts& o, bool fused,
                   uint64_t* d_outs, Plan* plan, bool reuse);
 int kernel_smem_optin(bbtc_ctx* ctx, const bbtc_opts& o);
-// After a count has finished on ctx's stream: BBTC_ERR_TIMEOUT if a
-// shared-memory staging copy of the launch gave up waiting (the count is void).
-int staging_status(bbtc_ctx* ctx);
+// Every launch of count_enqueue leaves a control word after its counts
+// (d_outs[graphs.size()]): BBTC_ERR_TIMEOUT if a shared-memory staging copy
+// gave up waiting (the counts are void).
+int control_status(uint64_t ctrl);
 size_t smem_bytes_for(const bbtc_opts& o);
+
+// Options shared by the count kernels.
+inline uint32_t norm_bm_words(uint32_t w) {
+  if (w == 0) w = 1024;
+  w = (w + 3) & ~3u;
+  return w < 256 ? 256 : w;
+}
+inline uint32_t norm_warps(uint32_t w) { return w == 0 || w > 8 ? 8 : w; }
+
+// fused.cu
+int pivots_smem_optin(size_t bytes);
+int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
+                  uint32_t total_units, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts);
 
 }  // namespace bbtc

@@ -8,27 +8,31 @@
 // (src/triangle_counting/bb_tc_helper.cpp:75-110).  Here the whole layout is
 // built on the device once and stays resident:
 //
-//   * the oriented CSR itself (global ids), which the fused task rows probe;
+//   * the oriented CSR itself (global ids);
+//   * its rows word-compressed: row u's ids grouped by 32-id word into (word
+//     index, bit mask) pairs, which the fused count streams;
+//   * the pivot lists of the fused count (internal.h: PivotGraph): the in-edges
+//     (u, v) of every vertex v that has a row of its own, each with the range
+//     of row u's pairs that can meet row v -- from the pair that holds v (or,
+//     when row v has kept ids below v, from the first pair that can hold one:
+//     see record_start) to the row's end.
+//
+// The P x P tiles of the per-task kernels are built on first use:
+//
 //   * forward tiles (x, y): rows of part x, tile-local columns of part y --
-//     the reference's tiles, used as ab / bc / ac by the per-task kernels;
+//     the reference's tiles, used as ab / bc / ac;
 //   * reversed tiles (y, x): the same edges grouped by their column vertex --
-//     the CSC of forward tile (x, y) -- with, beside each entry, the record
-//     of its forward edge (u, v): the range of row u's word-compressed pairs
-//     from the one that holds v (or, when the pivot row N+(v) has ids below
-//     v inside the task columns, from the first pair that can hold one: see
-//     record_start) to the row's end, which is what a fused task row streams
-//     per entry;
-//   * the word-compressed rows of the oriented CSR: row u's ids grouped by
-//     32-id word into (word index, bit mask) pairs.
+//     the CSC of forward tile (x, y).
 //
 // Every tile owns a row-pointer segment of H+1 tile-local offsets (first
 // entry 0) in one pool, laid out like the reference's rows_ array (P segments
 // per row part); column segments hold only the non-empty tiles.  Segments
-// start on 16-byte boundaries.  All passes are edge-parallel: each edge finds
-// its tile by bisection of the cut vector and the first edge of every (row,
-// tile) run writes the run length, so no thread walks a whole row.
+// start on 16-byte boundaries.  All passes are edge-parallel, so no thread
+// walks a whole row.
 #include <cub/cub.cuh>
 #include <cuda.h>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cstring>
@@ -88,40 +92,264 @@ __global__ void k_copy_mapped(uint32_t* __restrict__ dst0, const uint32_t* __res
   copy_words(dst1, src1, words1, t0, stride);
 }
 
-// Input contract check and per-edge expansion, one warp per row: row
-// pointers start at 0, never decrease and end at m; rows are strictly
-// increasing; ids are < n.  Rows whose pointers are out of order or past m
-// are flagged and skipped.  Writes the row id of every edge; with `flags`,
-// marks the edges that open a new 32-id word of their row (flags[e] = 1), the
-// input of the word-compressed rows; with `iota`, iota[e] = e (the edge ids
-// that the reversed graph's sort carries).  Nothing downstream reads `bad`
-// on the host before the layout is done: every later kernel that indexes by
-// these arrays returns at once when `*bad` is set.
-__global__ void k_expand_check(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
-                               uint32_t n, uint64_t m, uint32_t* __restrict__ rows, uint32_t* __restrict__ bad,
-                               uint32_t* __restrict__ flags, uint32_t* __restrict__ iota) {
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t u = warp; u < n; u += nwarps) {
+// Cut vector of a launch, by value.
+struct CutVec {
+  uint32_t c[kMaxParts + 1];
+  uint32_t P;
+};
+
+// Words of the flags block that the build leaves for the host.
+enum : uint32_t { kFlagBad = 0, kFlagUnoriented = 1, kFlagPivots = 2, kFlagPairs = 3, kFlagSparse = 4, kFlagWords = 8 };
+
+// Row part of the input contract, a thread per row: row pointers start at 0,
+// never decrease and end at m.  Sets the bit of every edge that starts a row
+// in `heads`, and the unoriented flag when some row's first id does not exceed
+// the row.
+__global__ void k_row_heads(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices, uint32_t n,
+                            uint64_t m, uint32_t* __restrict__ heads, uint32_t* __restrict__ flags) {
+  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t a = indptr[u], b = indptr[u + 1];
-    if (lane == 0) {
-      if (u == 0 && a != 0) atomicOr(bad, 1u);
-      if (u == n - 1 && (uint64_t)b != m) atomicOr(bad, 2u);
-    }
+    if (u == 0 && a != 0) atomicOr(&flags[kFlagBad], 1u);
+    if (u == n - 1 && (uint64_t)b != m) atomicOr(&flags[kFlagBad], 2u);
     if (b < a || (uint64_t)b > m) {
-      if (lane == 0) atomicOr(bad, 4u);
-      continue;
+      atomicOr(&flags[kFlagBad], 4u);
+    } else if (b > a) {
+      atomicOr(&heads[a >> 5], 1u << (a & 31));
+      if (indices[a] <= u) flags[kFlagUnoriented] = 1u;
     }
-    for (uint32_t e = a + lane; e < b; e += 32) {
-      rows[e] = u;
-      const uint32_t c = indices[e];
-      const uint32_t prev = e > a ? indices[e - 1] : 0u;
-      if (c >= n) atomicOr(bad, 8u);
-      if (e > a && prev >= c) atomicOr(bad, 16u);
-      if (flags) flags[e] = (e == a || (c >> 5) != (prev >> 5)) ? 1u : 0u;
-      if (iota) iota[e] = e;
+  }
+}
+
+__device__ __forceinline__ bool is_head(const uint32_t* __restrict__ heads, uint64_t e) {
+  return (heads[e >> 5] >> (e & 31)) & 1u;
+}
+
+// 1 for an edge that opens a new (word, mask) pair of its row: the input of the pair positions' scan.
+struct OpensPair {
+  const uint32_t* indices;
+  const uint32_t* heads;
+  __device__ __forceinline__ uint32_t operator()(uint64_t e) const {
+    return e == 0 || (indices[e] >> 5) != (indices[e - 1] >> 5) || is_head(heads, e) ? 1u : 0u;
+  }
+};
+
+// Edge part of the input contract (rows strictly increasing, ids < n), the
+// word-compressed rows and the records.  wpos = inclusive scan of OpensPair,
+// so edge e lands in pair wpos[e] - 1.  A warp takes 32 consecutive edges; a
+// pair's edges are consecutive, so a segmented suffix OR by shuffles (five
+// steps, no divergence) gives the first lane of each pair in the chunk the
+// bits of the pair's edges in the chunk.  The lane of the edge that opens a
+// pair stores it, after ORing in the bits of its edges past the chunk (at most
+// 31 more, only for the chunk's last pair); a pair that opened in an earlier
+// chunk is that chunk's to store.  So each pair has one writer and no atomics.
+// Record of edge e: its own pair and the end of its row's pairs, which is the
+// pair of the next row's first edge -- in the chunk, or (one search a chunk)
+// after it.  Needs m > 0.
+__global__ void k_pairs(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ heads,
+                        const uint32_t* __restrict__ wpos, uint32_t n, uint64_t m, uint2* __restrict__ words,
+                        uint2* __restrict__ rec, uint32_t* __restrict__ flags) {
+  const uint32_t W = wpos[m - 1];
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nheads = (m + 31) / 32;
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;  // a multiple of 32: warps keep their chunks aligned
+  if (t0 == 0) flags[kFlagPairs] = W;
+  for (uint64_t e = t0; e - lane < m; e += stride) {
+    const bool valid = e < m;
+    const uint32_t hw = heads[e >> 5];
+    const uint32_t x = valid ? indices[e] : 0u;
+    const uint32_t p = valid ? wpos[e] - 1u : 0xffffffffu;
+    uint32_t prev = __shfl_up_sync(FULLMASK, x, 1);
+    if (lane == 0) prev = e > 0 ? indices[e - 1] : 0u;
+    const bool head = e == 0 || ((hw >> lane) & 1u);
+    uint32_t v = valid ? 1u << (x & 31) : 0u;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_down_sync(FULLMASK, v, d);
+      const uint32_t po = __shfl_down_sync(FULLMASK, p, d);
+      if (lane + d < 32 && po == p) v |= o;
     }
+    const uint32_t p_last = __shfl_sync(FULLMASK, p, 31);
+    // the end of this edge's row: the next head's pair
+    const uint32_t later = lane < 31 ? hw & (FULLMASK << (lane + 1)) : 0u;
+    const uint32_t end = __shfl_sync(FULLMASK, p, later ? __ffs(later) - 1 : 0);
+    uint32_t far = W;  // the first head after the chunk
+    for (uint64_t c = (e >> 5) + 1; c < nheads; c += 32) {
+      const uint32_t o = c + lane < nheads ? heads[c + lane] : 0u;
+      const uint32_t some = __ballot_sync(FULLMASK, o != 0);
+      if (!some) continue;
+      const uint32_t src = __ffs(some) - 1;
+      const uint32_t word = __shfl_sync(FULLMASK, o, src);
+      const uint64_t at = (c + src) * 32 + (__ffs(word) - 1);
+      if (at < m) far = wpos[at] - 1u;
+      break;
+    }
+    if (!valid) continue;
+    if (x >= n) atomicOr(&flags[kFlagBad], 8u);
+    if (!head && prev >= x) atomicOr(&flags[kFlagBad], 16u);
+    rec[e] = make_uint2(p, later ? end : far);
+    if (!head && (prev >> 5) == (x >> 5)) continue;  // not the opening edge of its pair
+    if (p_last == p) {  // the pair reaches the chunk's last edge: it may go on past the chunk
+      const uint64_t far_k = min(e - lane + 63, m);
+      for (uint64_t k = e - lane + 32; k < far_k && wpos[k] - 1u == p; k++) v |= 1u << (indices[k] & 31);
+    }
+    words[p] = make_uint2(x >> 5, v);
+  }
+}
+
+// First and end position of every key in the sorted keys (both arrays start at zero).
+__global__ void k_key_bounds(const uint32_t* __restrict__ keys, uint64_t m, uint32_t n, uint32_t* __restrict__ first,
+                             uint32_t* __restrict__ end) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride) {
+    const uint32_t k = keys[q];
+    if (k >= n) continue;  // a refused input
+    if (q == 0 || keys[q - 1] != k) first[k] = (uint32_t)q;
+    if (q == m - 1 || keys[q + 1] != k) end[k] = (uint32_t)(q + 1);
+  }
+}
+
+// A vertex is a pivot when it has in-edges and a row.
+struct IsPivot {
+  const uint32_t* first;
+  const uint32_t* end;
+  const uint32_t* indptr;
+  __device__ __forceinline__ uint32_t operator()(uint32_t v) const {
+    return end[v] > first[v] && indptr[v + 1] > indptr[v] ? 1u : 0u;
+  }
+};
+
+// What the passes after the sort read.
+struct PivotInput {
+  const uint32_t* indptr;
+  const uint32_t* indices;
+  const uint32_t* wpos;
+  const uint32_t* keys;   // entries' vertices, sorted
+  const uint32_t* first;  // per vertex, its entries [first, end)
+  const uint32_t* end;
+  const uint32_t* pos;    // exclusive scan of IsPivot
+  const uint2* words;
+  uint32_t n;
+  uint64_t m;
+};
+
+// First pair of row u (u <= n).
+__device__ __forceinline__ uint32_t row_pair(const PivotInput& in, uint32_t u) {
+  const uint32_t e = in.indptr[u];
+  return (uint64_t)e < in.m ? in.wpos[e] - 1u : in.wpos[in.m - 1];
+}
+
+// The row that holds pair p.
+__device__ uint32_t row_of_pair(const PivotInput& in, uint32_t p) {
+  uint32_t lo = 0, hi = in.n;  // the last row whose first pair is <= p (empty rows share their successor's)
+  while (hi - lo > 1) {
+    const uint32_t mid = lo + ((hi - lo) >> 1);
+    if (row_pair(in, mid) <= p) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// The pivots (8 words each, see PivotGraph) and, after the last, one whose e0
+// is ~0.  When every id exceeds its row's, all in-edges of v lie in tasks that
+// meet row v and no id of row v lies below v's part.  Otherwise the tasks
+// (i, j, k) with j = part(v), i <= j <= k meet only in-edges from parts up to
+// j (the entries are in source order) and ids from cuts[j] on (the reference's
+// tiles ab = (i, j), ac = (i, k), bc = (j, k),
+// src/triangle_counting/gpu_sparse_kernel.cu:25-46).
+__global__ void k_pivots(PivotInput in, CutVec cuts, const uint2* __restrict__ rec, uint4* __restrict__ piv,
+                         uint32_t* __restrict__ flags) {
+  if (flags[kFlagBad]) return;
+  const bool plain = flags[kFlagUnoriented] == 0;
+  const IsPivot is{in.first, in.end, in.indptr};
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < in.n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = (uint32_t)t;
+    const uint32_t k = in.pos[v];
+    const uint32_t some = is(v);
+    if (v == in.n - 1) {
+      flags[kFlagPivots] = k + some;
+      piv[2 * (uint64_t)(k + some)] = make_uint4(~0u, ~0u, 0, 0);
+      piv[2 * (uint64_t)(k + some) + 1] = make_uint4(0, 0, 0, 0);
+    }
+    if (!some) continue;
+    uint32_t a = in.indptr[v], b = in.indptr[v + 1], e0 = in.first[v], e1 = in.end[v], mask0 = FULLMASK;
+    if (!plain) {
+      const uint32_t part = part_of(cuts.c, cuts.P, v);
+      a = lower_bound_range(in.indices, a, b, cuts.c[part]);
+      if (a < b) mask0 <<= in.indices[a] & 31;
+      uint32_t lo = e0, hi = e1;  // first entry from a later part
+      while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (row_of_pair(in, rec[mid].x) < cuts.c[part + 1]) lo = mid + 1; else hi = mid;
+      }
+      e1 = lo;
+    }
+    uint32_t ws = 0, wn = 0, fw = 0, span = 0;
+    if (a < b) {
+      ws = in.wpos[a] - 1u;
+      wn = row_pair(in, v + 1) - ws;
+      fw = in.indices[a] >> 5;
+      span = (in.indices[b - 1] >> 5) - fw + 1;
+    }
+    piv[2 * (uint64_t)k] = make_uint4(e0, e1, ws, wn);
+    piv[2 * (uint64_t)k + 1] = make_uint4(fw, span, mask0, v);
+  }
+}
+
+// First pair of the record of entry (u, v): the streamed side is row u from
+// the first pair whose word can hold a kept id of row v (first kept id L).
+// When L lies in v's word or above -- always, when every id exceeds its row's
+// -- that is the pair `p` holding v itself; otherwise the pair is searched in
+// row u's pairs before p.
+__device__ __forceinline__ uint32_t record_start(const PivotInput& in, uint32_t v, uint32_t lo, uint32_t p) {
+  const uint32_t a = in.indptr[v], b = in.indptr[v + 1];
+  const uint32_t k = lower_bound_range(in.indices, a, b, lo);
+  if (k >= b) return p;  // no kept id
+  const uint32_t lw = in.indices[k] >> 5;
+  if (lw >= (v >> 5)) return p;
+  uint32_t lo_p = row_pair(in, row_of_pair(in, p)), hi_p = p;  // the row holds v, so the answer is at or before p
+  while (lo_p < hi_p) {
+    const uint32_t mid = lo_p + ((hi_p - lo_p) >> 1);
+    if (in.words[mid].x < lw) lo_p = mid + 1; else hi_p = mid;
+  }
+  return lo_p;
+}
+
+// Four consecutive batches of 32 entries with this many pivots or more count as sparse.
+constexpr uint32_t kSparsePivots = 8;
+
+// crow, and the records' first pairs when the CSR is not oriented upwards.
+__global__ void k_entry_index(PivotInput in, CutVec cuts, const uint4* __restrict__ piv, uint32_t* __restrict__ crow,
+                              uint2* __restrict__ rec, uint32_t* __restrict__ flags) {
+  if (flags[kFlagBad]) return;
+  const bool plain = flags[kFlagUnoriented] == 0;
+  const IsPivot is{in.first, in.end, in.indptr};
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint64_t q = t0; 32 * q < in.m; q += stride) {
+    const uint32_t v = in.keys[32 * q];
+    uint32_t k = in.pos[v];
+    if (is(v) && 32 * q >= piv[2 * (uint64_t)k].y) k++;  // past the entries that it keeps
+    crow[q] = k;
+    // batches with four pivots or more among this one and the next three
+    const uint64_t ahead = 32 * q + 128;
+    if (ahead < in.m && in.pos[in.keys[ahead]] - in.pos[v] >= kSparsePivots)
+      atomicMax(&flags[kFlagSparse], (uint32_t)(q + 4));
+  }
+  if (plain) return;
+  for (uint64_t q = t0; q < in.m; q += stride) {
+    const uint32_t v = in.keys[q];
+    rec[q].x = record_start(in, v, cuts.c[part_of(cuts.c, cuts.P, v)], rec[q].x);
+  }
+}
+
+// Row id of every edge of a CSR that meets the contract, one warp per row.
+__global__ void k_row_ids(const uint32_t* __restrict__ indptr, uint32_t n, uint32_t* __restrict__ rows) {
+  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t u = warp; u < n; u += nwarps) {
+    const uint32_t b = indptr[u + 1];
+    for (uint64_t e = (uint64_t)indptr[u] + lane; e < b; e += 32) rows[e] = (uint32_t)u;
   }
 }
 
@@ -132,8 +360,7 @@ __global__ void k_expand_check(const uint32_t* __restrict__ indptr, const uint32
 __global__ void k_entry_count(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
                               const uint32_t* __restrict__ rows, uint64_t m, const uint32_t* __restrict__ cuts_g,
                               uint32_t P, const uint64_t* __restrict__ rp_off, uint32_t* __restrict__ counts,
-                              uint32_t* __restrict__ runs, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
+                              uint32_t* __restrict__ runs) {
   __shared__ uint32_t cuts[kMaxParts + 1];
   for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) cuts[t] = cuts_g[t];
   __syncthreads();
@@ -181,8 +408,7 @@ __global__ void k_zero_ranges(ZeroRanges z) {
 __global__ void k_localize_stats(uint32_t* __restrict__ rp, const uint32_t* __restrict__ scanned,
                                  const uint32_t* __restrict__ cuts_g, uint32_t P,
                                  const uint64_t* __restrict__ part_off, uint64_t len, uint32_t* __restrict__ maxdeg,
-                                 uint32_t* __restrict__ nerows, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
+                                 uint32_t* __restrict__ nerows) {
   __shared__ uint32_t cuts[kMaxParts + 1];
   __shared__ uint64_t poff[kMaxParts + 1];
   for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) {
@@ -232,8 +458,8 @@ __global__ void k_localize_stats(uint32_t* __restrict__ rp, const uint32_t* __re
 // shuffles (launched as one block of 32 threads).
 __global__ void k_tile_offsets(const uint32_t* __restrict__ rp, const uint64_t* __restrict__ rp_off,
                                const uint32_t* __restrict__ cuts, uint32_t P, uint32_t* __restrict__ nnz,
-                               uint64_t* __restrict__ col_off, const uint32_t* __restrict__ bad) {
-  if (blockIdx.x != 0 || threadIdx.x >= 32 || *bad) return;
+                               uint64_t* __restrict__ col_off) {
+  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
   const uint32_t lane = threadIdx.x;
   const uint32_t T = P * P;
   uint64_t cur = 0;
@@ -265,9 +491,9 @@ __global__ void k_tile_offsets(const uint32_t* __restrict__ rp, const uint64_t* 
 // exactly one non-empty row, so each slot has one writer.  blockIdx.y = tile.
 __global__ void k_row_index(const uint32_t* __restrict__ rp, const uint64_t* __restrict__ rp_off,
                             const uint32_t* __restrict__ cuts, uint32_t P, const uint64_t* __restrict__ col_off,
-                            uint32_t* __restrict__ erow, const uint32_t* __restrict__ bad) {
+                            uint32_t* __restrict__ erow) {
   const uint32_t t = blockIdx.y;
-  if (*bad || col_off[t] == kNoSegment) return;
+  if (col_off[t] == kNoSegment) return;
   const uint32_t x = t / P;
   const uint32_t H = cuts[x + 1] - cuts[x];
   const uint32_t* __restrict__ r = rp + rp_off[t];
@@ -279,50 +505,11 @@ __global__ void k_row_index(const uint32_t* __restrict__ rp, const uint64_t* __r
   }
 }
 
-// First pair of a reversed entry's record.  The entry (row v of part x,
-// column c) stands for forward edge c -> v; the tasks (i, x, k >= x) count the
-// common neighbours w of c and v with w >= cuts[x] (the reference's tiles
-// ac = (i, k), bc = (x, k), src/triangle_counting/gpu_sparse_kernel.cu:25-46).
-// The pivot side of v keeps only N+(v) ∩ [cuts[x], ∞), whose first id is L;
-// the streamed side is row c from the first pair whose word can hold an id
-// >= L.  When L lies in v's word or above -- always for a CSR oriented from
-// lower to higher ids, where every id of N+(v) exceeds v -- that is the pair
-// holding v itself (`p`); otherwise the pair is searched in row c's pairs
-// before p.  Any CSR that meets the input contract counts the reference's
-// task sum this way.
-__device__ __forceinline__ uint32_t record_start(const uint32_t* __restrict__ fptr, const uint32_t* __restrict__ fidx,
-                                                 const uint2* __restrict__ words, const uint32_t* __restrict__ wptr,
-                                                 uint32_t v, uint32_t c, uint32_t lo, uint32_t p) {
-  const uint32_t a = fptr[v], b = fptr[v + 1];
-  if (a >= b) return p;  // no pivot: the kernel skips the row
-  uint32_t L = fidx[a];
-  if (L < lo) {
-    const uint32_t k = lower_bound_range(fidx, a, b, lo);
-    if (k >= b) return p;  // no pivot id in the task columns
-    L = fidx[k];
-  }
-  const uint32_t lw = L >> 5;
-  if (lw >= (v >> 5)) return p;
-  uint32_t lo_p = wptr[c], hi_p = p;  // row c holds v, so the answer is at or before p
-  while (lo_p < hi_p) {
-    const uint32_t mid = lo_p + ((hi_p - lo_p) >> 1);
-    if (words[mid].x < lw) lo_p = mid + 1; else hi_p = mid;
-  }
-  return lo_p;
-}
-
-// Scatter tile-local column ids (and, for the reversed graph, the records of
-// the forward edges) into the column pool.  For the reversed graph
-// `fptr` / `fidx` / `words` are the oriented CSR and its word-compressed rows.
+// Scatter tile-local column ids into the column pool.
 __global__ void k_entry_scatter(const uint32_t* __restrict__ runs, const uint32_t* __restrict__ indices,
                                 const uint32_t* __restrict__ rows, uint64_t m, const uint32_t* __restrict__ cuts_g,
                                 uint32_t P, const uint64_t* __restrict__ rp_off, const uint64_t* __restrict__ col_off,
-                                const uint32_t* __restrict__ rp, uint32_t* __restrict__ col,
-                                const uint32_t* __restrict__ eids, const uint32_t* __restrict__ wpos,
-                                const uint32_t* __restrict__ wptr, uint2* __restrict__ rec,
-                                const uint32_t* __restrict__ fptr, const uint32_t* __restrict__ fidx,
-                                const uint2* __restrict__ words, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
+                                const uint32_t* __restrict__ rp, uint32_t* __restrict__ col) {
   __shared__ uint32_t cuts[kMaxParts + 1];
   for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) cuts[t] = cuts_g[t];
   __syncthreads();
@@ -336,89 +523,12 @@ __global__ void k_entry_scatter(const uint32_t* __restrict__ runs, const uint32_
     const uint32_t run = runs[e];  // first edge of this (row, tile) run
     const uint64_t pos = col_off[t] + rp[rp_off[t] + (u - cuts[x])] + ((uint32_t)e - run);
     col[pos] = c - cuts[y];
-    if (rec) {
-      // forward edge fe = (c -> u) of this reversed entry: the pairs of row c
-      // from the record's first pair to the row's end
-      const uint32_t fe = eids[e];
-      rec[pos] = make_uint2(record_start(fptr, fidx, words, wptr, u, c, cuts[x], wpos[fe] - 1u), wptr[c + 1]);
-    }
   }
 }
 
-// Word-compressed rows: each row's ids grouped by 32-id word into (word, bit
-// mask) pairs.  flags[e] = 1 when edge e opens a new word of its row
-// (k_expand_check); wpos = their inclusive scan, so edge e lands in pair
-// wpos[e] - 1.  A warp takes 32 consecutive edges; a pair's edges are
-// consecutive, so a segmented suffix OR by shuffles (five steps, no
-// divergence) gives the first lane of each pair in the chunk the bits of the
-// pair's edges in the chunk.  The lane of the edge that opens a pair stores
-// it, after ORing in the bits of its edges past the chunk (at most 31 more,
-// only for the chunk's last pair); a pair that opened in an earlier chunk is
-// that chunk's to store.  So each pair has one writer and no atomics.  Pairs
-// W = wpos[m - 1] .. m + 1 (the array's unused tail) are zeroed.  Needs m > 0.
-__global__ void k_word_fill(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ flags,
-                            const uint32_t* __restrict__ wpos, uint64_t m, uint2* __restrict__ words,
-                            const uint32_t* __restrict__ bad) {
-  if (*bad) return;
-  const uint64_t W = wpos[m - 1];
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;  // a multiple of 32: warps keep their chunks aligned
-  for (uint64_t e = t0; e - lane < m; e += stride) {
-    const bool valid = e < m;
-    const uint32_t x = valid ? indices[e] : 0u;
-    const uint32_t p = valid ? wpos[e] - 1u : 0xffffffffu;
-    uint32_t v = valid ? 1u << (x & 31) : 0u;
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-      const uint32_t o = __shfl_down_sync(FULLMASK, v, d);
-      const uint32_t po = __shfl_down_sync(FULLMASK, p, d);
-      if (lane + d < 32 && po == p) v |= o;
-    }
-    const uint32_t p_prev = __shfl_up_sync(FULLMASK, p, 1);
-    const uint32_t p_last = __shfl_sync(FULLMASK, p, 31);
-    if (!valid) continue;
-    if (e >= W) words[e] = make_uint2(0, 0);
-    if ((lane > 0 && p_prev == p) || !flags[e]) continue;  // not the opening edge of its pair
-    if (p_last == p) {  // the pair reaches the chunk's last edge: it may go on past the chunk
-      for (uint64_t k = e - lane + 32; k < m && !flags[k]; k++) v |= 1u << (indices[k] & 31);
-    }
-    words[p] = make_uint2(x >> 5, v);
-  }
-  if (t0 < 2) words[m + t0] = make_uint2(0, 0);
-}
-
-// wptr[u] = first pair of row u (u in [0, n]); a row's first edge opens a pair.
-// desc[u]: the fused kernel's view of row u as a pivot, in one 16-byte load.
-__global__ void k_word_rowptr(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
-                              const uint32_t* __restrict__ wpos, uint32_t n, uint64_t m, uint32_t* __restrict__ wptr,
-                              uint4* __restrict__ desc, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u <= n; u += gridDim.x * blockDim.x) {
-    const uint32_t e = indptr[u];
-    const uint32_t w = (uint64_t)e < m ? wpos[e] - 1u : (m ? wpos[m - 1] : 0u);
-    wptr[u] = w;
-    // pivot descriptor: row start, pair start, first and last id (0, 0 for an empty row)
-    const bool has = u < n && indptr[u + 1] > e;
-    desc[u] = make_uint4(e, w, has ? indices[e] : 0u, has ? indices[indptr[u + 1] - 1] : 0u);
-  }
-}
-
-// The reversed graph from the (column, forward edge id) pairs sorted by
-// column, in two passes (the row pointers' searches run with the whole
-// GPU's parallelism, not behind the gather in one grid-stride loop):
-// rev_cols[q] = source row of forward edge eids[q] (q < m) ...
-__global__ void k_gather(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ eids, uint64_t m,
-                         uint32_t* __restrict__ rev_cols, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) rev_cols[e] = rows[eids[e]];
-}
-
-// ... and rev_indptr[v] = first position of key v in the sorted keys (v <= n).
+// rev_indptr[v] = first position of key v in the sorted keys (v <= n).
 __global__ void k_rev_indptr(const uint32_t* __restrict__ keys, uint64_t m, uint32_t n,
-                             uint32_t* __restrict__ rev_indptr, const uint32_t* __restrict__ bad) {
-  if (*bad) return;
+                             uint32_t* __restrict__ rev_indptr) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += stride) {
     uint64_t lo = 0, hi = m;
@@ -498,14 +608,11 @@ int launch_layout(const bbtc_ctx* ctx, void (*kernel)(KArgs...), dim3 grid, dim3
 }
 
 // Build one block CSR (forward or reversed) from a CSR in device memory whose
-// per-edge row ids are `rows`.  With `eids` the reversed build also writes the
-// forward-edge records.  The tile statistics land in `st` (device, 4*P*P words)
-// and are copied to the host by the caller.
+// per-edge row ids are `rows`.  The tile statistics land in d_stats (device,
+// 4*P*P words) and are copied to the host by the caller.
 int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const uint32_t* d_indices,
                 const uint32_t* d_rows, uint32_t n, uint64_t m, const std::vector<uint32_t>& cuts,
-                const uint32_t* d_cuts, const uint32_t* eids, const uint32_t* wpos, const uint32_t* wptr,
-                const uint32_t* fptr, const uint32_t* fidx, const uint2* words, uint32_t* d_stats,
-                uint64_t* d_coloff, const uint32_t* d_bad, int grid) {
+                const uint32_t* d_cuts, uint32_t* d_stats, uint64_t* d_coloff, int grid) {
   const uint32_t P = (uint32_t)cuts.size() - 1;
   const uint32_t T = P * P;
   cudaStream_t s = ctx->stream;
@@ -526,9 +633,8 @@ int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const u
   {
     cudaError_t e1 = dev_malloc(&bt.d_rp, bt.rp_len * sizeof(uint32_t), s);
     cudaError_t e2 = dev_malloc(&bt.d_col, bt.col_len * sizeof(uint32_t), s);
-    cudaError_t e3 = eids ? dev_malloc(&bt.d_rec, bt.col_len * sizeof(uint2), s) : cudaSuccess;
     cudaError_t e4 = dev_malloc(&bt.d_erow, bt.erow_len * sizeof(uint32_t), s);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
+    if (e1 != cudaSuccess || e2 != cudaSuccess || e4 != cudaSuccess) {
       cudaGetLastError();
       bt.release(s);
       return fail(BBTC_ERR_NOMEM, "device allocation of the block-CSR pools failed");
@@ -542,8 +648,8 @@ int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const u
   uint64_t* d_rp_off = offs.as<uint64_t>();
   uint64_t* d_part_off = d_rp_off + T;
   {
-    // through this block CSR's own pinned region: it is not written again before the build's final sync
-    uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOff[eids ? 1 : 0]);
+    // through a pinned region that is not written again before the build's final sync
+    uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOff);
     std::memcpy(h, bt.rp_off.data(), T * sizeof(uint64_t));
     std::memcpy(h + T, part_off.data(), (P + 1) * sizeof(uint64_t));
     BBTC_CUDA(cudaMemcpyAsync(d_rp_off, h, (T + P + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
@@ -557,7 +663,7 @@ int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const u
   }
   if (m > 0) {
     BBTC_TRY(launch_layout(ctx, k_entry_count, grid, 256, s, d_indptr, d_indices, d_rows, m, d_cuts, P, d_rp_off,
-                           counts.as<uint32_t>(), runs.as<uint32_t>(), d_bad));
+                           counts.as<uint32_t>(), runs.as<uint32_t>()));
     size_t rb = 0;
     BBTC_CUDA(cub::DeviceScan::InclusiveScan(nullptr, rb, runs.as<uint32_t>(), runs.as<uint32_t>(), cub::Max(),
                                              (int64_t)m, s));
@@ -578,55 +684,34 @@ int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const u
   uint32_t* st_max = d_stats + T;
   uint32_t* st_ne = d_stats + 2 * T;
   BBTC_TRY(launch_layout(ctx, k_localize_stats, grid, 256, s, bt.d_rp, counts.as<uint32_t>(), d_cuts, P, d_part_off,
-                         part_off[P], st_max, st_ne, d_bad));
-  BBTC_TRY(launch_layout(ctx, k_tile_offsets, 1, 32, s, bt.d_rp, d_rp_off, d_cuts, P, st_nnz, d_coloff, d_bad));
+                         part_off[P], st_max, st_ne));
+  BBTC_TRY(launch_layout(ctx, k_tile_offsets, 1, 32, s, bt.d_rp, d_rp_off, d_cuts, P, st_nnz, d_coloff));
   {
     uint32_t maxH = 1;
     for (uint32_t x = 0; x < P; x++) maxH = std::max(maxH, cuts[x + 1] - cuts[x]);
     const uint32_t gx = std::min<uint32_t>(64, (maxH + 255) / 256);
-    BBTC_TRY(launch_layout(ctx, k_row_index, dim3(gx, T), 256, s, bt.d_rp, d_rp_off, d_cuts, P, d_coloff, bt.d_erow,
-                           d_bad));
+    BBTC_TRY(launch_layout(ctx, k_row_index, dim3(gx, T), 256, s, bt.d_rp, d_rp_off, d_cuts, P, d_coloff,
+                           bt.d_erow));
   }
   if (m > 0) {
     BBTC_TRY(launch_layout(ctx, k_entry_scatter, grid, 256, s, runs.as<uint32_t>(), d_indices, d_rows, m, d_cuts, P,
-                           d_rp_off, d_coloff, bt.d_rp, bt.d_col, eids, wpos, wptr,
-                           reinterpret_cast<uint2*>(bt.d_rec), fptr, fidx, words, d_bad));
+                           d_rp_off, d_coloff, bt.d_rp, bt.d_col));
   }
   return BBTC_OK;
 }
 
-// Read back the tile statistics of one or two block CSRs (a may be null) with
-// one sync; with `d_bad`, also the input-contract flags (into *h_bad), and
-// when any is set the statistics are left unread.
-int fetch_stats(bbtc_ctx* ctx, BlockTiles* a, BlockTiles& b, const uint32_t* d_stats_a, const uint64_t* d_coloff_a,
-                const uint32_t* d_stats_b, const uint64_t* d_coloff_b, cudaStream_t s,
-                const uint32_t* d_bad = nullptr, uint32_t* h_bad = nullptr) {
-  const uint32_t T = b.P * b.P;
-  // pinned staging: [coloff a | coloff b | stats a | stats b]
-  uint64_t* hc = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageStats);
-  uint32_t* hs = reinterpret_cast<uint32_t*>(hc + 2 * T);
-  if (a) {
-    BBTC_CUDA(cudaMemcpyAsync(hc, d_coloff_a, T * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    BBTC_CUDA(cudaMemcpyAsync(hs, d_stats_a, 3 * T * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  }
-  BBTC_CUDA(cudaMemcpyAsync(hc + T, d_coloff_b, T * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  BBTC_CUDA(cudaMemcpyAsync(hs + 3 * T, d_stats_b, 3 * T * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  uint32_t* hb = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageBad);
-  if (d_bad) BBTC_CUDA(cudaMemcpyAsync(hb, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+// Read back a block CSR's tile statistics (synchronises the stream).
+int fetch_stats(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_stats, const uint64_t* d_coloff, cudaStream_t s) {
+  const uint32_t T = bt.P * bt.P;
+  uint64_t* hc = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageStats);  // pinned staging: column offsets, statistics
+  uint32_t* hs = reinterpret_cast<uint32_t*>(hc + T);
+  BBTC_CUDA(cudaMemcpyAsync(hc, d_coloff, T * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  BBTC_CUDA(cudaMemcpyAsync(hs, d_stats, 3 * T * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   BBTC_CUDA(cudaStreamSynchronize(s));
-  if (d_bad) {
-    *h_bad = *hb;
-    if (*hb) return BBTC_OK;  // the statistics are void
-  }
-  for (BlockTiles* p : {a, &b}) {
-    if (!p) continue;
-    const uint64_t* c = p == a ? hc : hc + T;
-    const uint32_t* h = p == a ? hs : hs + 3 * T;
-    p->col_off.assign(c, c + T);
-    p->nnz.assign(h, h + T);
-    p->maxdeg.assign(h + T, h + 2 * T);
-    p->nerows.assign(h + 2 * T, h + 3 * T);
-  }
+  bt.col_off.assign(hc, hc + T);
+  bt.nnz.assign(hs, hs + T);
+  bt.maxdeg.assign(hs + T, hs + 2 * T);
+  bt.nerows.assign(hs + 2 * T, hs + 3 * T);
   return BBTC_OK;
 }
 
@@ -639,8 +724,12 @@ int layout_grid(const bbtc_ctx* ctx, uint32_t n, uint64_t m, uint32_t P) {
                                  std::max<uint64_t>(ctx->sms, (span + 2047) / 2048));
 }
 
-uint64_t block_bytes(const BlockTiles& t, bool rec) {
-  return (t.rp_len + t.col_len + t.erow_len) * sizeof(uint32_t) + (rec ? t.col_len * sizeof(uint2) : 0);
+uint64_t block_bytes(const BlockTiles& t) { return (t.rp_len + t.col_len + t.erow_len) * sizeof(uint32_t); }
+
+int key_bits(uint64_t n) {
+  int b = 1;
+  while (b < 32 && (1ull << b) < n) b++;
+  return b;
 }
 
 }  // namespace
@@ -648,10 +737,8 @@ uint64_t block_bytes(const BlockTiles& t, bool rec) {
 void BlockTiles::release(cudaStream_t s) {
   if (d_rp) cudaFreeAsync(d_rp, s);
   if (d_col) cudaFreeAsync(d_col, s);
-  if (d_rec) cudaFreeAsync(d_rec, s);
   if (d_erow) cudaFreeAsync(d_erow, s);
   d_rp = d_col = d_erow = nullptr;
-  d_rec = nullptr;
 }
 
 DevTile dev_tile(const BlockTiles& t, const std::vector<uint32_t>& cuts, uint32_t x, uint32_t y) {
@@ -664,17 +751,15 @@ DevTile dev_tile(const BlockTiles& t, const std::vector<uint32_t>& cuts, uint32_
   if (d.nnz) {
     d.rp = t.d_rp + t.rp_off[id];
     d.col = t.d_col + t.col_off[id];
-    d.rec = t.d_rec ? reinterpret_cast<const uint2*>(t.d_rec) + t.col_off[id] : nullptr;
     d.erow = t.d_erow + t.col_off[id] / 32 + id;
   } else {
     d.rp = d.col = d.erow = nullptr;
-    d.rec = nullptr;
   }
   return d;
 }
 
 // Layout scratch a context keeps between builds: the temporaries of a graph
-// of up to about five million edges (about 45 bytes per edge); a larger
+// of up to about nine million edges (about 28 bytes per edge); a larger
 // build allocates its own and frees them at its end.
 constexpr size_t kScratchKeep = 256ull << 20;
 
@@ -719,22 +804,12 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
   ScratchScope scratch(ctx, s);
   const uint32_t n = g->n;
   const uint64_t m = g->m;
-  const uint32_t P = g->P;
-  const uint32_t T = P * P;
-  const int grid = layout_grid(ctx, n, m, P);
-  cudaEvent_t ev0, ev1;
-  BBTC_CUDA(cudaEventCreate(&ev0));
-  BBTC_CUDA(cudaEventCreate(&ev1));
-  struct EvGuard {
-    cudaEvent_t a, b;
-    ~EvGuard() {
-      cudaEventDestroy(a);
-      cudaEventDestroy(b);
-    }
-  } evg{ev0, ev1};
-  BBTC_CUDA(cudaEventRecord(ev0, s));
+  const int grid = layout_grid(ctx, n, m, 1);
+  for (cudaEvent_t& ev : ctx->ev_layout)
+    if (!ev) BBTC_CUDA(cudaEventCreate(&ev));
+  BBTC_CUDA(cudaEventRecord(ctx->ev_layout[0], s));
 
-  // the graph keeps its own copy of the oriented CSR: the fused task rows probe it
+  // the graph keeps its own copy of the oriented CSR
   {
     cudaError_t e1 = dev_malloc(&g->d_indptr, ((size_t)n + 1) * sizeof(uint32_t), s);
     cudaError_t e2 = dev_malloc(&g->d_indices, std::max<uint64_t>(m, 1) * sizeof(uint32_t) + 16, s);
@@ -802,132 +877,120 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
   const uint32_t* d_indptr = g->d_indptr;
   const uint32_t* d_indices = g->d_indices;
 
-  DevBuf d_cuts, rows, stats_r, coloff_r, wflags, wpos, eids_in;
-  BBTC_TRY(dalloc(wflags, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(wpos, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(d_cuts, (g->cuts.size() + 1) * sizeof(uint32_t), s));  // the cuts, then the contract flags
-  BBTC_TRY(dalloc(rows, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(stats_r, 4 * T * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(coloff_r, T * sizeof(uint64_t), s));
-  BBTC_TRY(dalloc(eids_in, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-  uint32_t* d_bad = d_cuts.as<uint32_t>() + g->cuts.size();
+  const uint64_t mm = std::max<uint64_t>(m, 1);
+  const uint64_t nheads = mm / 32 + 1;
+  const uint64_t npiv_max = std::min<uint64_t>(n, m);
+  g->nentry_rows = mm / 32 + 1;
   {
-    // one copy: the cut vector and a zero flags word
-    uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageCuts);
-    std::memcpy(h, g->cuts.data(), g->cuts.size() * sizeof(uint32_t));
-    h[g->cuts.size()] = 0;
-    BBTC_CUDA(cudaMemcpyAsync(d_cuts.p, h, (g->cuts.size() + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  }
-  // The contract check runs first; its flags are read back with the tile
-  // statistics at the end, and every kernel between that indexes by the input
-  // returns at once when they are set, so no host round trip splits the build.
-  if (n > 0) {
-    BBTC_TRY(launch_layout(ctx, k_expand_check, grid, 256, s, d_indptr, d_indices, n, m, rows.as<uint32_t>(), d_bad,
-                           wflags.as<uint32_t>(), eids_in.as<uint32_t>()));
-  } else if (m > 0) {
-    BBTC_CUDA(cudaMemsetAsync(d_bad, 0xff, sizeof(uint32_t), s));  // edges without rows
-  }
-
-  // the forward block CSR waits until something needs it (ensure_fwd): the
-  // fused task rows read only the reversed one
-
-  // word-compressed rows (the fused task rows stream these); k_expand_check wrote the flags
-  {
-    cudaError_t e1 = dev_malloc(&g->d_words, std::max<uint64_t>(m, 1) * sizeof(uint2) + 16, s);
-    cudaError_t e2 = dev_malloc(&g->d_wptr, ((size_t)n + 1) * sizeof(uint32_t), s);
-    cudaError_t e3 = dev_malloc(&g->d_desc, ((size_t)n + 1) * sizeof(uint4), s);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
+    cudaError_t e1 = dev_malloc(&g->d_words, mm * sizeof(uint2), s);
+    cudaError_t e2 = dev_malloc(&g->d_rec, mm * sizeof(uint2), s);
+    cudaError_t e3 = dev_malloc(&g->d_piv, (npiv_max + 1) * 2 * sizeof(uint4), s);
+    cudaError_t e4 = dev_malloc(&g->d_crow, g->nentry_rows * sizeof(uint32_t), s);
+    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
       cudaGetLastError();
-      return fail(BBTC_ERR_NOMEM, "device allocation of the word-compressed rows failed");
+      return fail(BBTC_ERR_NOMEM, "device allocation of the word-compressed rows and pivot lists failed");
     }
-    if (m > 0) {
-      size_t tb = 0;
-      BBTC_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, wflags.as<uint32_t>(), wpos.as<uint32_t>(), (int64_t)m, s));
-      DevBuf tmp;
-      BBTC_TRY(dalloc(tmp, tb, s));
-      BBTC_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, tb, wflags.as<uint32_t>(), wpos.as<uint32_t>(), (int64_t)m, s));
-      BBTC_TRY(launch_layout(ctx, k_word_fill, grid, 256, s, d_indices, wflags.as<uint32_t>(), wpos.as<uint32_t>(), m,
-                             reinterpret_cast<uint2*>(g->d_words), d_bad));
-    } else {
-      BBTC_CUDA(cudaMemsetAsync(g->d_words, 0, sizeof(uint2) + 16, s));
-    }
-    BBTC_TRY(launch_layout(ctx, k_word_rowptr, grid, 256, s, d_indptr, d_indices, wpos.as<uint32_t>(), n, m,
-                           g->d_wptr, static_cast<uint4*>(g->d_desc), d_bad));
   }
-
-  // reversed graph: a stable sort of (column, forward edge id) by column keeps
-  // every in-list ordered by source
+  // flags, row heads and the vertices' entry bounds start at zero; the flags
+  // are read back once, at the end: every pass between stays inside its arrays
+  // whatever the input, or returns at once when the contract flag is set
+  DevBuf zeroed, wpos, rec_in, keys, pos;
+  const uint64_t nv = ((uint64_t)n + 4) & ~3ull, hw = (nheads + 3) & ~3ull;
+  BBTC_TRY(dalloc(zeroed, (kFlagWords + hw + 2 * nv) * sizeof(uint32_t), s));
+  BBTC_TRY(dalloc(wpos, mm * sizeof(uint32_t), s));
+  BBTC_TRY(dalloc(rec_in, mm * sizeof(uint2), s));
+  BBTC_TRY(dalloc(keys, mm * sizeof(uint32_t), s));
+  BBTC_TRY(dalloc(pos, nv * sizeof(uint32_t), s));
+  uint32_t* flags = zeroed.as<uint32_t>();
+  uint32_t* heads = flags + kFlagWords;
+  uint32_t* first = heads + hw;
+  uint32_t* end = first + nv;
   {
-    DevBuf keys_out, eids_out, rev_indptr, rev_cols;
-    BBTC_TRY(dalloc(keys_out, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-    BBTC_TRY(dalloc(eids_out, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-    BBTC_TRY(dalloc(rev_cols, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-    BBTC_TRY(dalloc(rev_indptr, ((size_t)n + 1) * sizeof(uint32_t), s));
-    if (m > 0) {
-      int end_bit = 1;
-      while (end_bit < 32 && (1ull << end_bit) < (uint64_t)n) end_bit++;
-      size_t tmp_bytes = 0;
-      BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_indices, keys_out.as<uint32_t>(),
-                                                eids_in.as<uint32_t>(), eids_out.as<uint32_t>(), (int64_t)m, 0,
-                                                end_bit, s));
-      DevBuf tmp;
-      BBTC_TRY(dalloc(tmp, tmp_bytes, s));
-      BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, d_indices, keys_out.as<uint32_t>(),
-                                                eids_in.as<uint32_t>(), eids_out.as<uint32_t>(), (int64_t)m, 0,
-                                                end_bit, s));
-    }
-    if (m > 0) {
-      BBTC_TRY(launch_layout(ctx, k_gather, grid, 256, s, rows.as<uint32_t>(), eids_out.as<uint32_t>(), m,
-                             rev_cols.as<uint32_t>(), d_bad));
-    }
-    BBTC_TRY(launch_layout(ctx, k_rev_indptr, grid, 256, s, keys_out.as<uint32_t>(), m, n, rev_indptr.as<uint32_t>(),
-                           d_bad));
-    // reversed entries: row = column vertex v (keys), column = source u, record of forward edge (u, v)
-    BBTC_TRY(build_block(ctx, g->rev, rev_indptr.as<uint32_t>(), rev_cols.as<uint32_t>(), keys_out.as<uint32_t>(),
-                         n, m, g->cuts, d_cuts.as<uint32_t>(), eids_out.as<uint32_t>(), wpos.as<uint32_t>(),
-                         g->d_wptr, d_indptr, d_indices, reinterpret_cast<const uint2*>(g->d_words),
-                         stats_r.as<uint32_t>(), coloff_r.as<uint64_t>(), d_bad, grid));
+    ZeroRanges z{{flags, nullptr, nullptr, nullptr}, {kFlagWords + hw + 2 * nv, 0, 0, 0}};
+    BBTC_TRY(launch_layout(ctx, k_zero_ranges, grid, 256, s, z));
   }
-  // the host needs the tile statistics and the contract flags only now: one read-back
-  uint32_t hbad = 0;
-  BBTC_TRY(fetch_stats(ctx, nullptr, g->rev, nullptr, nullptr, stats_r.as<uint32_t>(), coloff_r.as<uint64_t>(), s,
-                       d_bad, &hbad));
-  if (hbad) {
+  if (n > 0) {
+    BBTC_TRY(launch_layout(ctx, k_row_heads, grid, 256, s, d_indptr, d_indices, n, m, heads, flags));
+  } else if (m > 0) {
+    BBTC_CUDA(cudaMemsetAsync(flags, 0xff, sizeof(uint32_t), s));  // edges without rows
+  }
+  if (n > 0 && m > 0) {
+    uint2* words = static_cast<uint2*>(g->d_words);
+    uint2* rec = static_cast<uint2*>(g->d_rec);
+    uint4* piv = static_cast<uint4*>(g->d_piv);
+    const auto opens = thrust::make_transform_iterator(thrust::counting_iterator<uint64_t>(0), OpensPair{d_indices, heads});
+    const auto is_pivot = thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0),
+                                                          IsPivot{first, end, d_indptr});
+    size_t b1 = 0, b2 = 0, b3 = 0;
+    BBTC_CUDA(cub::DeviceScan::InclusiveSum(nullptr, b1, opens, wpos.as<uint32_t>(), (int64_t)m, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b2, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
+                                              (int64_t)m, 0, key_bits(n), s));
+    BBTC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b3, is_pivot, pos.as<uint32_t>(), (int64_t)n, s));
+    DevBuf tmp;
+    BBTC_TRY(dalloc(tmp, std::max(b1, std::max(b2, b3)), s));
+    BBTC_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, b1, opens, wpos.as<uint32_t>(), (int64_t)m, s));
+    BBTC_TRY(launch_layout(ctx, k_pairs, grid, 256, s, d_indices, heads, wpos.as<uint32_t>(), n, m, words,
+                           rec_in.as<uint2>(), flags));
+    // a stable sort of the records by column keeps every in-list in source order
+    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, b2, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
+                                              (int64_t)m, 0, key_bits(n), s));
+    BBTC_TRY(launch_layout(ctx, k_key_bounds, grid, 256, s, keys.as<uint32_t>(), m, n, first, end));
+    BBTC_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, b3, is_pivot, pos.as<uint32_t>(), (int64_t)n, s));
+    CutVec cuts{};
+    std::copy(g->cuts.begin(), g->cuts.end(), cuts.c);
+    cuts.P = g->P;
+    const PivotInput in{d_indptr, d_indices, wpos.as<uint32_t>(), keys.as<uint32_t>(), first, end, pos.as<uint32_t>(),
+                        words, n, m};
+    BBTC_TRY(launch_layout(ctx, k_pivots, grid, 256, s, in, cuts, rec, piv, flags));
+    BBTC_TRY(launch_layout(ctx, k_entry_index, grid, 256, s, in, cuts, piv, g->d_crow, rec, flags));
+  }
+  uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageFlags);
+  BBTC_CUDA(cudaMemcpyAsync(h, flags, kFlagWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  BBTC_CUDA(cudaEventRecord(ctx->ev_layout[1], s));
+  BBTC_CUDA(cudaStreamSynchronize(s));
+  const uint32_t bad = h[kFlagBad];
+  if (bad) {
     std::string why;
-    if (hbad == 0xffffffffu) why += " edges but no rows;";
+    if (bad == 0xffffffffu) why += " edges but no rows;";
     else {
-      if (hbad & 1) why += " indptr[0] != 0;";
-      if (hbad & 2) why += " indptr[n] != m;";
-      if (hbad & 4) why += " row pointers decrease or exceed m;";
-      if (hbad & 8) why += " a column id >= n;";
-      if (hbad & 16) why += " a row is not strictly increasing (unsorted or duplicate ids);";
+      if (bad & 1) why += " indptr[0] != 0;";
+      if (bad & 2) why += " indptr[n] != m;";
+      if (bad & 4) why += " row pointers decrease or exceed m;";
+      if (bad & 8) why += " a column id >= n;";
+      if (bad & 16) why += " a row is not strictly increasing (unsorted or duplicate ids);";
     }
     return fail(BBTC_ERR_INPUT, "CSR breaks the input contract:" + why);
   }
-  BBTC_CUDA(cudaEventRecord(ev1, s));
-  BBTC_CUDA(cudaEventSynchronize(ev1));
+  g->oriented = h[kFlagUnoriented] == 0;
+  g->npiv = h[kFlagPivots];
+  g->nwords = h[kFlagPairs];
+  g->sparse_end = h[kFlagSparse];
   float ms = 0;
-  BBTC_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
+  BBTC_CUDA(cudaEventElapsedTime(&ms, ctx->ev_layout[0], ctx->ev_layout[1]));
   g->layout_ms = ms;
-  g->device_bytes = block_bytes(g->rev, true) + ((uint64_t)n + 1 + m) * sizeof(uint32_t) + 64 * sizeof(uint64_t) +
-                    m * sizeof(uint2) + ((uint64_t)n + 1) * (sizeof(uint32_t) + sizeof(uint4));
+  g->device_bytes = ((uint64_t)n + 1 + m + g->nentry_rows) * sizeof(uint32_t) + 64 * sizeof(uint64_t) +
+                    2 * mm * sizeof(uint2) + (npiv_max + 1) * 2 * sizeof(uint4);
   return BBTC_OK;
 }
 
 namespace {
 
-int build_fwd(bbtc_graph* g) {
-  Range range("bbtc forward tiles");
+// One block CSR of the per-task kernels, from the resident CSR (which passed
+// the contract check when it was uploaded): the forward one, or the reversed
+// one from the edges sorted by column (stable, so in-lists stay in source
+// order).
+int build_tiles(bbtc_graph* g, bool reversed) {
+  Range range(reversed ? "bbtc reversed tiles" : "bbtc forward tiles");
   bbtc_ctx* ctx = g->ctx;
   cudaStream_t s = ctx->stream;
   BBTC_CUDA(cudaSetDevice(ctx->device));
   const uint32_t n = g->n, P = g->P, T = P * P;
-  const uint64_t m = g->m;
+  const uint64_t m = g->m, mm = std::max<uint64_t>(m, 1);
   const int grid = layout_grid(ctx, n, m, P);
-  DevBuf d_cuts, bad, rows, stats, coloff;
+  BlockTiles& bt = reversed ? g->rev : g->fwd;
+  DevBuf d_cuts, rows, stats, coloff, keys, sources, rev_indptr;
   BBTC_TRY(dalloc(d_cuts, g->cuts.size() * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(bad, sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(rows, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
+  BBTC_TRY(dalloc(rows, mm * sizeof(uint32_t), s));
   BBTC_TRY(dalloc(stats, 4 * T * sizeof(uint32_t), s));
   BBTC_TRY(dalloc(coloff, T * sizeof(uint64_t), s));
   {
@@ -935,40 +998,63 @@ int build_fwd(bbtc_graph* g) {
     std::memcpy(h, g->cuts.data(), g->cuts.size() * sizeof(uint32_t));
     BBTC_CUDA(cudaMemcpyAsync(d_cuts.p, h, g->cuts.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   }
-  BBTC_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s));
-  if (n > 0) {
-    // row id of every edge (the CSR passed validation when it was uploaded)
-    BBTC_TRY(launch_layout(ctx, k_expand_check, grid, 256, s, g->d_indptr, g->d_indices, n, m, rows.as<uint32_t>(),
-                           bad.as<uint32_t>(), nullptr, nullptr));
+  if (n > 0) BBTC_TRY(launch_layout(ctx, k_row_ids, grid, 256, s, g->d_indptr, n, rows.as<uint32_t>()));
+  const uint32_t* t_indptr = g->d_indptr;
+  const uint32_t* t_indices = g->d_indices;
+  const uint32_t* t_rows = rows.as<uint32_t>();
+  if (reversed) {
+    BBTC_TRY(dalloc(keys, mm * sizeof(uint32_t), s));
+    BBTC_TRY(dalloc(sources, mm * sizeof(uint32_t), s));
+    BBTC_TRY(dalloc(rev_indptr, ((size_t)n + 1) * sizeof(uint32_t), s));
+    if (m > 0) {
+      size_t tb = 0;
+      BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, g->d_indices, keys.as<uint32_t>(), rows.as<uint32_t>(),
+                                                sources.as<uint32_t>(), (int64_t)m, 0, key_bits(n), s));
+      DevBuf tmp;
+      BBTC_TRY(dalloc(tmp, tb, s));
+      BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, g->d_indices, keys.as<uint32_t>(), rows.as<uint32_t>(),
+                                                sources.as<uint32_t>(), (int64_t)m, 0, key_bits(n), s));
+    }
+    BBTC_TRY(launch_layout(ctx, k_rev_indptr, grid, 256, s, keys.as<uint32_t>(), m, n, rev_indptr.as<uint32_t>()));
+    t_indptr = rev_indptr.as<uint32_t>();
+    t_indices = sources.as<uint32_t>();
+    t_rows = keys.as<uint32_t>();
   }
-  BBTC_TRY(build_block(ctx, g->fwd, g->d_indptr, g->d_indices, rows.as<uint32_t>(), n, m, g->cuts,
-                       d_cuts.as<uint32_t>(), nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                       stats.as<uint32_t>(), coloff.as<uint64_t>(), bad.as<uint32_t>(), grid));
-  BBTC_TRY(fetch_stats(ctx, nullptr, g->fwd, nullptr, nullptr, stats.as<uint32_t>(), coloff.as<uint64_t>(), s));
-  g->fwd_built = true;
-  g->device_bytes += block_bytes(g->fwd, false);
+  BBTC_TRY(build_block(ctx, bt, t_indptr, t_indices, t_rows, n, m, g->cuts, d_cuts.as<uint32_t>(),
+                       stats.as<uint32_t>(), coloff.as<uint64_t>(), grid));
+  BBTC_TRY(fetch_stats(ctx, bt, stats.as<uint32_t>(), coloff.as<uint64_t>(), s));
+  (reversed ? g->rev_built : g->fwd_built) = true;
+  g->device_bytes += block_bytes(bt);
   return BBTC_OK;
+}
+
+int ensure(bbtc_graph* g, bool reversed) {
+  if (reversed ? g->rev_built : g->fwd_built) return BBTC_OK;
+  const int rc = build_tiles(g, reversed);
+  if (rc != BBTC_OK) {
+    // a failed build (say, out of memory half way) leaves nothing behind: the
+    // frees are stream-ordered after whatever of it was enqueued
+    BlockTiles& bt = reversed ? g->rev : g->fwd;
+    bt.release(g->ctx->stream);
+    bt = BlockTiles();
+  }
+  return rc;
 }
 
 }  // namespace
 
-int ensure_fwd(bbtc_graph* g) {
-  if (g->fwd_built) return BBTC_OK;
-  const int rc = build_fwd(g);
-  if (rc != BBTC_OK) {
-    // a failed build (say, out of memory half way) leaves nothing behind: the
-    // frees are stream-ordered after whatever of it was enqueued
-    g->fwd.release(g->ctx->stream);
-    g->fwd = BlockTiles();
-  }
-  return rc;
+int ensure_fwd(bbtc_graph* g) { return ensure(g, false); }
+
+int ensure_tiles(bbtc_graph* g) {
+  BBTC_TRY(ensure(g, false));
+  return ensure(g, true);
 }
 
 }  // namespace bbtc
 
 // Read the whole layout back and check it on the host (debug aid: it copies
 // every array, so it costs about the graph's device bytes in host memory and
-// PCIe time).  The forward block CSR is checked when it has been built.
+// PCIe time).  The block CSRs of the per-task kernels are checked when they have been built.
 int bbtc_graph_validate(const bbtc_graph* g) {
   using namespace bbtc;
   static_assert(check::kNoSeg == kNoSegment, "empty-tile marker");
@@ -985,29 +1071,33 @@ int bbtc_graph_validate(const bbtc_graph* g) {
     if (words) BBTC_CUDA(cudaMemcpyAsync(h.data(), d, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return BBTC_OK;
   };
-  std::vector<uint32_t> indptr, indices, wptr, pairs, desc;
-  BBTC_TRY(get(desc, g->d_desc, 4 * ((uint64_t)n + 1)));
+  std::vector<uint32_t> indptr, indices, pairs, rec, piv, crow;
   BBTC_TRY(get(indptr, g->d_indptr, (uint64_t)n + 1));
   BBTC_TRY(get(indices, g->d_indices, mm));
-  BBTC_TRY(get(wptr, g->d_wptr, (uint64_t)n + 1));
-  BBTC_TRY(get(pairs, g->d_words, 2 * mm));
+  BBTC_TRY(get(pairs, g->d_words, 2 * g->nwords));
+  BBTC_TRY(get(rec, g->d_rec, 2 * m));
+  BBTC_TRY(get(piv, g->d_piv, m ? 8 * ((uint64_t)g->npiv + 1) : 0));
+  BBTC_TRY(get(crow, g->d_crow, (m + 31) / 32));
   BBTC_CUDA(cudaStreamSynchronize(s));
   check::Csr c{n, m, indptr.data(), indices.data()};
-  check::Words w{wptr.data(), pairs.data(), mm};
   std::string why = check::csr(c);
-  if (why.empty()) why = check::words(c, w);
-  if (why.empty()) why = check::descs(c, w, desc.data());
-  std::vector<uint32_t> tp, tc;
+  std::vector<uint32_t> wptr((size_t)n + 1, 0), tp, tc;
+  check::Words w{wptr.data(), pairs.data(), g->nwords};
+  if (why.empty()) {
+    check::row_pairs(c, wptr.data());
+    why = check::words(c, w);
+  }
   if (why.empty()) check::transpose(c, tp, tc);
   const check::Csr tr{n, m, tp.data(), tc.data()};
+  if (why.empty() && m)
+    why = check::pivots(c, tr, w, check::Pivots{g->P, g->cuts.data(), g->npiv, piv.data(), rec.data(), crow.data()});
   for (int pass = 0; pass < 2 && why.empty(); pass++) {
     const BlockTiles& bt = pass == 0 ? g->rev : g->fwd;
-    if (pass == 1 && !g->fwd_built) break;
-    std::vector<uint32_t> rp, col, erow, rec;
+    if (!(pass == 0 ? g->rev_built : g->fwd_built)) continue;
+    std::vector<uint32_t> rp, col, erow;
     BBTC_TRY(get(rp, bt.d_rp, bt.rp_len));
     BBTC_TRY(get(col, bt.d_col, bt.col_len));
     BBTC_TRY(get(erow, bt.d_erow, bt.erow_len));
-    if (bt.d_rec) BBTC_TRY(get(rec, bt.d_rec, 2 * bt.col_len));
     BBTC_CUDA(cudaStreamSynchronize(s));
     check::Tiles t;
     t.P = g->P;
@@ -1023,9 +1113,7 @@ int bbtc_graph_validate(const bbtc_graph* g) {
     t.col_len = bt.col_len;
     t.erow = erow.data();
     t.erow_len = bt.erow_len;
-    t.rec = bt.d_rec ? rec.data() : nullptr;
-    if (pass == 0 && !t.rec) why = "reversed tiles: no forward-edge records";
-    else why = check::tiles(pass == 0 ? "reversed tiles" : "forward tiles", pass == 0 ? tr : c, t, w);
+    why = check::tiles(pass == 0 ? "reversed tiles" : "forward tiles", pass == 0 ? tr : c, t, w);
   }
   if (!why.empty()) return fail(BBTC_ERR_LAYOUT, "device layout check failed: " + why);
   return BBTC_OK;

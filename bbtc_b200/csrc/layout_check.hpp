@@ -27,6 +27,7 @@
 //     row u's pairs and its first pair: the one that contains v, or -- when
 //     the first id L of v's row at or above cuts[x] lies in a lower 32-id
 //     word than v -- the first pair of row u whose word is >= L / 32.
+//   * the pivot lists of the fused count (Pivots below).
 // Each check returns "" or a message naming the first broken rule.
 #pragma once
 
@@ -157,6 +158,79 @@ inline uint32_t record_word(const Words& w, uint32_t v, uint32_t lo) {
       if ((mask >> bit & 1) && word * 32 + bit >= lo) return word;
   }
   return ~0u;
+}
+
+// First pair of every row (n + 1 offsets) of the only word compression of g.
+inline void row_pairs(const Csr& g, uint32_t* wptr) {
+  uint32_t p = 0;
+  for (uint32_t u = 0; u < g.n; u++) {
+    wptr[u] = p;
+    for (uint32_t e = g.indptr[u]; e < g.indptr[u + 1]; e++)
+      p += e == g.indptr[u] || g.indices[e - 1] / 32 != g.indices[e] / 32;
+  }
+  wptr[g.n] = p;
+}
+
+// The pivot lists of the fused count: entries in (v, u) order of the
+// transposed CSR `tr`.  Vertex v with in-edges and a row is a pivot; it keeps
+// the in-edges from parts up to its own and the ids from its part's first on.
+struct Pivots {
+  uint32_t P = 0;
+  const uint32_t* cuts = nullptr;
+  uint32_t npiv = 0;
+  const uint32_t* piv = nullptr;   // 8 words a pivot, npiv + 1 of them
+  const uint32_t* rec = nullptr;   // 2 words an entry
+  const uint32_t* crow = nullptr;  // per 32 entries
+};
+
+inline std::string pivots(const Csr& g, const Csr& tr, const Words& w, const Pivots& p) {
+  uint32_t k = 0;
+  std::vector<uint32_t> next((size_t)(g.m + 31) / 32, ~0u);
+  for (uint32_t v = 0, part = 0; v < g.n; v++) {
+    while (v >= p.cuts[part + 1]) part++;
+    const uint32_t c0 = tr.indptr[v], c1 = tr.indptr[v + 1];
+    uint32_t e1 = c0;
+    const bool is = c1 > c0 && g.indptr[v + 1] > g.indptr[v];
+    if (is) {
+      if (k >= p.npiv) return at("a pivot is missing, vertex", v);
+      const uint32_t* d = p.piv + 8 * (uint64_t)k;
+      while (e1 < c1 && tr.indices[e1] < p.cuts[part + 1]) e1++;
+      if (d[0] != c0 || d[1] != e1 || d[7] != v) return at("pivot names the wrong entries, vertex", v);
+      uint32_t a = g.indptr[v];
+      const uint32_t b = g.indptr[v + 1];
+      while (a < b && g.indices[a] < p.cuts[part]) a++;
+      uint32_t ws = w.wptr[v];
+      if (a < b)
+        while (w.pairs[2 * (uint64_t)ws] < g.indices[a] / 32) ws++;
+      if (a == b ? d[3] != 0
+                 : d[2] != ws || d[3] != w.wptr[v + 1] - ws || d[4] != g.indices[a] / 32 ||
+                       d[5] != g.indices[b - 1] / 32 - g.indices[a] / 32 + 1)
+        return at("pivot differs from its row, vertex", v);
+      if (a < b) {
+        uint32_t kept = 0;  // ids of the first pair at or above the part's first id
+        for (uint32_t q = a; q < b && g.indices[q] / 32 == g.indices[a] / 32; q++) kept |= 1u << (g.indices[q] % 32);
+        if ((w.pairs[2 * (uint64_t)ws + 1] & d[6]) != kept) return at("pivot keeps the wrong ids, vertex", v);
+      }
+      const uint32_t lw = record_word(w, v, p.cuts[part]);
+      for (uint32_t q = c0; q < e1; q++) {
+        const uint32_t u = tr.indices[q], p0 = p.rec[2 * (uint64_t)q], p1 = p.rec[2 * (uint64_t)q + 1];
+        if (p1 != w.wptr[u + 1] || p0 < w.wptr[u] || p0 >= p1) return at("record outside the row's pairs, entry", q);
+        if (lw < v / 32) {
+          if (w.pairs[2 * (uint64_t)p0] < lw || (p0 > w.wptr[u] && w.pairs[2 * (uint64_t)(p0 - 1)] >= lw))
+            return at("record names the wrong pair, entry", q);
+        } else if (w.pairs[2 * (uint64_t)p0] != v / 32 || !(w.pairs[2 * (uint64_t)p0 + 1] >> (v % 32) & 1)) {
+          return at("record names the wrong pair, entry", q);
+        }
+      }
+    }
+    for (uint64_t x = ((uint64_t)c0 + 31) / 32; x * 32 < c1; x++) next[x] = is && x * 32 >= e1 ? k + 1 : k;
+    if (is) k++;
+  }
+  if (k != p.npiv) return at("too many pivots", p.npiv, k);
+  if (p.piv[8 * (uint64_t)k] != ~0u) return "the pivots have no end mark";
+  for (size_t x = 0; x < next.size(); x++)
+    if (next[x] != p.crow[x]) return at("entry index names the wrong pivot, entry", x * 32);
+  return "";
 }
 
 // `src` is the CSR the block CSR splits (the oriented graph for the forward

@@ -121,7 +121,7 @@ int n1d_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_indptr, uint64_t m, 
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ctx->sms * 8, (n + 255) / 256));
   k_max_row<<<grid, 256, 0, s>>>(d_indptr, n, dmax.as<uint32_t>());
   BBTC_CUDA(cudaGetLastError());
-  uint32_t* hmax = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageBad);
+  uint32_t* hmax = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageFlags);
   BBTC_CUDA(cudaMemcpyAsync(hmax, dmax.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   BBTC_CUDA(cudaStreamSynchronize(s));
   // the host's search range (partition_core.hpp: n1d_cuts)

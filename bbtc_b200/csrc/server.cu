@@ -55,16 +55,17 @@ uint64_t now_ns() {
       .count();
 }
 
-// Device bytes a graph's layout needs, while it is built (upper bound).
-uint64_t estimate_bytes(uint32_t n, uint64_t m, const std::vector<uint32_t>& cuts) {
+// Device bytes a graph's layout needs, while it is built (upper bound); with
+// `tiles`, also the block CSRs that a per-task count builds.
+uint64_t estimate_bytes(uint32_t n, uint64_t m, const std::vector<uint32_t>& cuts, bool tiles) {
+  const uint64_t csr = 4 * ((uint64_t)n + 1) + 4 * m;
+  const uint64_t lists = 16 * m + m / 8 + 32 * (std::min<uint64_t>(n, m) + 1);  // pairs, records, index, pivots
+  const uint64_t temps = 32 * m + 16 * ((uint64_t)n + 4) + (16ull << 20);
+  if (!tiles) return csr + lists + temps;
   const uint64_t P = cuts.size() - 1;
   uint64_t rp = 0;
   for (uint64_t x = 0; x < P; x++) rp += P * (((uint64_t)cuts[x + 1] - cuts[x] + 1 + 3) & ~3ull);
-  const uint64_t pools = 2 * 4 * (rp + 4) + 2 * 4 * (m + 4 * P * P + 4) + 8 * (m + 4 * P * P + 4) +
-                        2 * 4 * (m / 32 + 2 * P * P + 2);
-  const uint64_t csr = 4 * ((uint64_t)n + 1) + 4 * m;
-  const uint64_t temps = 4 * (rp + 4) + 24 * m + 4 * ((uint64_t)n + 1) + (16ull << 20);
-  return pools + csr + temps;
+  return csr + lists + temps + 3 * 4 * (rp + 4) + 2 * 4 * (m + 4 * P * P + 4) + 2 * 4 * (m / 32 + 2 * P * P + 2);
 }
 
 struct Request {
@@ -236,7 +237,7 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
     int rc = BBTC_OK;
     if (!fused) {
       for (size_t i = 0; i < batch.size(); i++) {
-        if (rc == BBTC_OK) rc = ensure_fwd(gs[i]);
+        if (rc == BBTC_OK) rc = o.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(gs[i]) : ensure_tiles(gs[i]);
         uint32_t nt = 0;
         bbtc_task_list(gs[i]->P, nullptr, 0, &nt);
         tl[i].resize(nt);
@@ -246,11 +247,11 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
     if (rc == BBTC_OK) rc = count_enqueue(ctx, gs, tl, o, fused, L.d_outs, &plan, false);
     if (rc == BBTC_OK) {
       const cudaError_t e =
-          cudaMemcpyAsync(L.h_outs, L.d_outs, batch.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost,
+          cudaMemcpyAsync(L.h_outs, L.d_outs, (batch.size() + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost,
                           ctx->stream);
       const cudaError_t e2 = e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
       if (e2 != cudaSuccess) rc = cuda_fail(e2, "server batch readback");
-      else rc = staging_status(ctx);
+      else rc = control_status(L.h_outs[batch.size()]);
     }
     const uint64_t t = now_ns();
     // stream-ordered frees: the memory returns to the pool behind this launch
@@ -456,8 +457,8 @@ int bbtc_server_create(int device, const bbtc_server_opts* opts, bbtc_server** o
       rc = set_partition_stream(s, s->load_ctx[i], (int)(i % 2), i % 2 == 0 ? mid : lo);
   }
   for (uint32_t l = 0; rc == BBTC_OK && l < 2; l++) {
-    if (dev_malloc_sync(&s->lanes[l].d_outs, s->opts.max_batch * sizeof(uint64_t)) != cudaSuccess ||
-        cudaMallocHost(&s->lanes[l].h_outs, s->opts.max_batch * sizeof(uint64_t)) != cudaSuccess) {
+    if (dev_malloc_sync(&s->lanes[l].d_outs, ((size_t)s->opts.max_batch + 1) * sizeof(uint64_t)) != cudaSuccess ||
+        cudaMallocHost(&s->lanes[l].h_outs, ((size_t)s->opts.max_batch + 1) * sizeof(uint64_t)) != cudaSuccess) {
       cudaGetLastError();
       rc = fail(BBTC_ERR_NOMEM, "allocation of the result slots failed");
     }
@@ -574,7 +575,10 @@ int bbtc_submit(bbtc_server* s, uint32_t n, const uint32_t* indptr, const uint32
   r->indptr = indptr;
   r->indices = indices;
   r->cuts.assign(cuts, cuts + P + 1);
-  r->reserved = estimate_bytes(n, m, r->cuts);
+  const bbtc_opts& co = s->opts.count;
+  const bool tiles = !(co.kernel == BBTC_KERNEL_FUSED ||
+                       (co.kernel == BBTC_KERNEL_AUTO && co.mode == BBTC_MODE_PERSISTENT));
+  r->reserved = estimate_bytes(n, m, r->cuts, tiles);
   r->t_submit = now_ns();
   std::lock_guard<std::mutex> lk(s->mu);
   if (s->stop) {

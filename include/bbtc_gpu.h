@@ -162,14 +162,14 @@ typedef enum bbtc_mode {
 
 typedef enum bbtc_kernel {
   BBTC_KERNEL_AUTO = 0,   /* persistent form over the whole task list (tasks == NULL, or every task
-                             once in any order, as the reference's driver passes it): fused task rows; otherwise
+                             once in any order, as the reference's driver passes it): fused; otherwise
                              per task: bitmap when the part fits the shared bitmap, else search */
   BBTC_KERNEL_BITMAP = 1, /* per task: pivot row of bc as a shared-memory bitmap, probes from ac */
   BBTC_KERNEL_SEARCH = 2, /* per task: pivot row of bc as a sorted shared-memory list, bisection probes */
   BBTC_KERNEL_MERGE = 3,  /* per task, the reference's row order: pivot = ac row of each ab row,
                              the bc rows it meets are searched against it */
-  BBTC_KERNEL_FUSED = 4   /* task rows: the tasks (i, j, k >= j) sharing tile ab = (i, j) in one
-                             pass (needs the whole task list: tasks == NULL, or every task once) */
+  BBTC_KERNEL_FUSED = 4   /* pivot lists: all tasks in one pass over the in-edges of every vertex (needs the
+                             whole task list: tasks == NULL, or every task once) */
 } bbtc_kernel;
 
 typedef struct bbtc_opts {
@@ -177,12 +177,12 @@ typedef struct bbtc_opts {
   int kernel;                /* bbtc_kernel */
   uint32_t bitmap_words;     /* shared bitmap / list words per warp: 0 = default (1024) */
   uint32_t warps_per_block;  /* 0 = default (8) */
-  uint32_t unit_work;        /* target probes per work unit, 0 = default (256 task rows, 8192 tasks) */
+  uint32_t unit_work;        /* target probes per work unit, 0 = default (by position in a fused count, 8192 per task) */
   uint32_t blocks_per_sm;    /* persistent grid = SMs x this, 0 = occupancy limit */
   int use_cuda_graph;        /* replay the launch sequence through a captured CUDA graph */
   int sort_tasks;            /* when tasks == NULL: 1 = cost-sorted descending (default) */
-  uint32_t occupancy;        /* persistent form: register budget for 4, 5, 6 or 8 blocks per SM (5: fused task rows only; 0: 6 for
-                                fused task rows with a bitmap of at most 1024 words, else 4) */
+  uint32_t occupancy;        /* persistent form: register budget for 4, 5, 6 or 8 blocks per SM (5: fused counts only; 0: 5 for
+                                fused counts with a buffer of at most 1024 words, else 4) */
 } bbtc_opts;
 
 void bbtc_opts_default(bbtc_opts* o);
