@@ -30,12 +30,11 @@
 // consecutive ids at a time (see probe_entries).
 #include <algorithm>
 #include <cmath>
-#include <cstddef>
 #include <cstring>
-#include <mutex>
 #include <sstream>
 
 #include "internal.h"
+#include "search.cuh"
 
 namespace bbtc {
 
@@ -95,20 +94,6 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, uint32_
   return __all_sync(FULL, done_all);
 }
 
-__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
-  uint32_t lo = 0;
-  while (n > 0) {
-    const uint32_t half = n >> 1;
-    if (a[lo + half] < x) {
-      lo += half + 1;
-      n -= half + 1;
-    } else {
-      n = half;
-    }
-  }
-  return lo;
-}
-
 struct PivotView {
   const uint32_t* row;  // global pivot row
   uint32_t len;
@@ -116,32 +101,6 @@ struct PivotView {
   uint32_t cap;   // a bit of the warp's last buffer word, which stays zero
   uint32_t first, last;
 };
-
-// First p in [from, n) with a[p] >= x (n if none) for a sorted a, given
-// a[from - 1] < x: steps of 1, 2, 4, ... from `from`, then bisection of the
-// last step.  A lane probing increasing ids of one row against a long pivot
-// row moves forward from its previous position instead of bisecting the
-// whole row again (skewed degrees: long pivot rows, short probe rows).
-__device__ __forceinline__ uint32_t gallop_lb(const uint32_t* __restrict__ a, uint32_t n, uint32_t from, uint32_t x) {
-  if (from >= n || a[from] >= x) return from;
-  uint32_t lo = from, step = 1;  // a[lo] < x
-  while (lo + step < n && a[lo + step] < x) {
-    lo += step;
-    step <<= 1;
-  }
-  uint32_t L = lo + 1;
-  uint32_t len = min(lo + step, n) - L;  // the answer is in [L, L + len]
-  while (len > 0) {
-    const uint32_t half = len >> 1;
-    if (a[L + half] < x) {
-      L += half + 1;
-      len -= half + 1;
-    } else {
-      len = half;
-    }
-  }
-  return L;
-}
 
 template <uint32_t KIND>
 __device__ __forceinline__ uint32_t member(const uint32_t* bm, const PivotView& pv, uint32_t x) {
@@ -292,29 +251,6 @@ __device__ __forceinline__ uint32_t pivot_pass(const uint32_t* __restrict__ prow
   }
   __syncwarp();
   return hits;
-}
-
-// Row b of a tile holding entry e: the largest b with rp[b] <= e.
-__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ rp, uint32_t H, uint32_t e) {
-  uint32_t lo = 0, hi = H;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (rp[mid] <= e) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
-// Next row after b with an entry at or after e (a warp-wide scan of row ends).
-__device__ __forceinline__ uint32_t next_row(const uint32_t* __restrict__ rp, uint32_t H, uint32_t b, uint32_t e,
-                                             uint32_t lane) {
-  b++;
-  while (true) {
-    const uint32_t idx = b + lane;
-    const uint32_t v = idx < H ? rp[idx + 1] : 0xffffffffu;
-    const uint32_t mask = __ballot_sync(FULL, v > e);
-    if (mask) return b + __ffs(mask) - 1;
-    b += 32;
-  }
 }
 
 // One per-task work unit: entries [unit*K, min((unit+1)*K, nnz)) of the rows tile.
@@ -619,13 +555,21 @@ static int make_pivot_plan(const bbtc_ctx* ctx, const std::vector<bbtc_graph*>& 
   return BBTC_OK;
 }
 
+// Unit sizes of the per-task kernels.  Units of 8192 probes were a few
+// thousand per request and left the chip to the last ones: half the task list
+// of R-MAT s18 / s15 / Chung-Lu 2^18 (bitmap kernel, us) 821 / 482 / 5318;
+// 1024 probes, and at least eight units a warp, 549 / 111 / 472; 512 probes
+// 587 / 112 / 481.
+constexpr uint32_t kUnitWork = 1024;  // probes of a unit
+constexpr uint32_t kUnitShare = 8;    // units per warp at least, while they hold 32 entries or more
+
 // Build the device task array for a per-task request.  A single graph keeps
 // the caller's task order (its border split); several graphs are merged into
 // one queue ordered by estimated probe work, heaviest first.
-static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<std::vector<bbtc_task>>& tasks,
-                     const bbtc_opts& o, Plan* plan) {
+static int make_plan(const bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
+                     const std::vector<std::vector<bbtc_task>>& tasks, const bbtc_opts& o, Plan* plan) {
   const uint32_t bmw = norm_bm_words(o.bitmap_words);
-  const uint32_t unit_work = o.unit_work ? o.unit_work : 8192;  // units of about 8192 probes
+  const uint32_t unit_work = o.unit_work ? o.unit_work : kUnitWork;
   std::vector<DevTask> list;
   std::vector<double> cost;
   auto add = [&](DevTask d, double avg_probe) {
@@ -667,6 +611,18 @@ static int make_plan(const std::vector<bbtc_graph*>& graphs, const std::vector<s
       const uint32_t probe_tile = u_centric ? j * P + k : i * P + k;
       const uint32_t probe_rows = std::max<uint32_t>(1, g->fwd.nerows[probe_tile]);
       add(d, (double)d.probe.nnz / probe_rows);
+    }
+  }
+  if (!o.unit_work) {
+    // no unit larger than an even share of the launch's entries -- the whole
+    // queue's, or in the plain form the task's -- over a few units per warp
+    const uint64_t warps = (uint64_t)ctx->sms * 32;
+    uint64_t entries = 0;
+    for (const DevTask& d : list) entries += d.rows.nnz;
+    for (DevTask& d : list) {
+      const uint64_t share = o.mode == BBTC_MODE_PLAIN ? d.rows.nnz / (2 * warps) : entries / (kUnitShare * warps);
+      d.unit_edges = std::min(d.unit_edges, ((uint32_t)std::min<uint64_t>(share, 16384) + 31) & ~31u);
+      d.unit_edges = std::max(d.unit_edges, 32u);
     }
   }
   std::vector<uint32_t> order(list.size());
@@ -775,7 +731,7 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
     if (plan->exec) cudaGraphExecDestroy(plan->exec);
     plan->exec = nullptr;
     if (fused) BBTC_TRY(make_pivot_plan(ctx, graphs, o, plan));
-    else BBTC_TRY(make_plan(graphs, tasks, o, plan));
+    else BBTC_TRY(make_plan(ctx, graphs, tasks, o, plan));
     // one graph's fused queue rides in the kernel's arguments; other queues are uploaded
     const size_t nt = fused && plan->pivots.size() == 1 ? 0 : plan->prefix.size() - 1;
     if (nt) {
@@ -844,213 +800,4 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
   return BBTC_OK;
 }
 
-// ---- counting without allocation --------------------------------------------
-//
-// bbtc_count_csr_noalloc counts the triangles of an oriented CSR that the
-// caller already holds in device memory, for callers that cannot allocate
-// device memory themselves or through this library: code that runs inside
-// another framework's device-memory manager (which owns the device's memory
-// and hands out only slices of its own pool), processes held to a fixed
-// device-memory quota, and paths that must not pay cudaMalloc / cudaFree's
-// implicit device synchronisation.  It is the persistent queue kernel's
-// scheme run over the CSR as one task (P = 1, the reference's row order: the
-// pivot is N+(u), the rows streamed are N+(v) for v in N+(u)); every word of
-// scratch -- the queue head, an error word, the total and one partial count
-// per work unit -- lives in the static array below, so the call allocates
-// nothing.  Limit: at most kNoAllocMaxEdges oriented edges.
-constexpr uint32_t kNoAllocUnitEdges = 256;
-constexpr uint64_t kNoAllocMaxEdges = 1ull << 24;  // 16,777,216 oriented edges
-constexpr uint32_t kNoAllocMaxUnits = (uint32_t)(kNoAllocMaxEdges / kNoAllocUnitEdges);
-
-struct NoAllocScratch {
-  uint32_t head;   // next work unit
-  uint32_t error;  // bit 0: a row pointer or id outside the CSR was met
-  unsigned long long total;
-  uint32_t pad[60];
-  unsigned long long partial[kNoAllocMaxUnits];
-};
-
-// One copy per device that loads the library, kept until the process exits
-// (about 512 KiB).  Host code must not take its address directly: the
-// device address comes from cudaGetSymbolAddress, once per device.
-static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
-
-namespace {
-
-// Row ranges of a caller CSR, checked against [0, m] and ids against n.
-struct CheckedCsrSegs {
-  const uint32_t* __restrict__ col;
-  const uint32_t* __restrict__ rp;
-  uint32_t n;
-  uint64_t m;
-  uint32_t* err;
-  __device__ __forceinline__ void get(uint32_t q, uint32_t& start, uint32_t& len) const {
-    const uint32_t v = col[q];
-    start = 0;
-    len = 0;
-    if (v >= n) {
-      atomicOr(err, 1u);
-      return;
-    }
-    const uint32_t a = rp[v], b = rp[v + 1];
-    if (b < a || (uint64_t)b > m) {
-      atomicOr(err, 1u);
-      return;
-    }
-    start = a;
-    len = b - a;
-  }
-};
-
-__global__ void __launch_bounds__(256, 4) k_count_csr_static(const uint32_t* __restrict__ indptr,
-                                                             const uint32_t* __restrict__ indices, uint32_t n,
-                                                             uint64_t m, uint32_t units, NoAllocScratch* scr,
-                                                             uint32_t bm_words) {
-  extern __shared__ __align__(16) uint32_t sh[];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* bm = sh + warp * (bm_words + kSegWords);
-  uint32_t* sstart = bm + bm_words;
-  uint32_t* sbase = sstart + 33;
-  for (uint32_t i = lane; i < bm_words; i += 32) bm[i] = 0;
-  __syncwarp();
-  const CheckedCsrSegs segs{indices, indptr, n, m, &scr->error};
-  while (true) {
-    uint32_t g = 0;
-    if (lane == 0) g = atomicAdd(&scr->head, 1u);
-    g = __shfl_sync(FULL, g, 0);
-    if (g >= units) break;
-    const uint32_t e0 = g * kNoAllocUnitEdges;
-    const uint64_t e1w = (uint64_t)e0 + kNoAllocUnitEdges;
-    const uint32_t e1 = (uint32_t)(e1w < m ? e1w : m);
-    uint32_t e = e0;
-    uint32_t u = row_of(indptr, n, e);  // < n (the host refuses n == 0 with m > 0)
-    unsigned long long acc = 0;
-    while (e < e1) {
-      if (u >= n) {  // no row ends after e: indptr[n] < m
-        if (lane == 0) atomicOr(&scr->error, 1u);
-        break;
-      }
-      const uint32_t a = indptr[u], b = indptr[u + 1];
-      if (b < a || (uint64_t)b > m || b <= e) {  // malformed row pointers: stop this unit
-        if (lane == 0) atomicOr(&scr->error, 1u);
-        break;
-      }
-      const uint32_t ee = min(b, e1);
-      const uint32_t pd = b - a;
-      const uint32_t* prow = indices + a;
-      // the caller's row must be strictly increasing: the bitmap is indexed by id
-      bool sorted = true;
-      for (uint32_t i = lane; i + 1 < pd; i += 32) sorted &= prow[i] < prow[i + 1];
-      if (!__all_sync(FULL, sorted)) {
-        if (lane == 0) atomicOr(&scr->error, 1u);
-        e = ee;
-        if (e < e1) u = next_row(indptr, n, u, e, lane);
-        continue;
-      }
-      const uint32_t first = prow[0], last = prow[pd - 1];
-      const uint32_t span_words = last >= first ? ((last - first) >> 5) + 1 : 0xffffffffu;
-      if (span_words < bm_words)
-        acc += pivot_pass<kPivotBitmap>(prow, pd, first, span_words, segs, e, ee, indices, bm, sstart, sbase,
-                                        lane);
-      else if (pd <= bm_words)
-        acc += pivot_pass<kPivotList>(prow, pd, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
-      else
-        acc += pivot_pass<kPivotGlobal>(prow, pd, 0, 0, segs, e, ee, indices, bm, sstart, sbase, lane);
-      e = ee;
-      if (e < e1) u = next_row(indptr, n, u, e, lane);
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) scr->partial[g] = acc;
-  }
-}
-
-// total = sum of the unit partials, in a fixed order (one block).
-__global__ void k_noalloc_total(NoAllocScratch* scr, uint32_t units) {
-  __shared__ unsigned long long part[1024];
-  unsigned long long s = 0;
-  for (uint32_t i = threadIdx.x; i < units; i += blockDim.x) s += scr->partial[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (uint32_t w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) scr->total = part[0];
-}
-
-}  // namespace
-
-namespace {
-
-// Per device, set up by the first call on it: the device address of
-// g_noalloc_scratch, the kernel's shared-memory attribute and its grid.
-std::mutex g_noalloc_mu;
-void* g_noalloc_ptr[kMaxDevices] = {};
-uint32_t g_noalloc_grid[kMaxDevices] = {};
-
-constexpr uint32_t kNoAllocBitmapWords = 1024, kNoAllocWarps = 8;
-
-int noalloc_setup(int dev, void** ptr, uint32_t* grid) {
-  std::lock_guard<std::mutex> lk(g_noalloc_mu);
-  if (!g_noalloc_ptr[dev]) {
-    // the device is current: resolve the array's device address
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-    const size_t sm = smem_bytes(kNoAllocBitmapWords, kNoAllocWarps);
-    BBTC_CUDA(cudaFuncSetAttribute(k_count_csr_static, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    int sms = 0, per_sm = 0;
-    BBTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_count_csr_static, kNoAllocWarps * 32, sm));
-    g_noalloc_grid[dev] = (uint32_t)std::max(1, sms * std::max(1, per_sm));
-    g_noalloc_ptr[dev] = p;
-  }
-  *ptr = g_noalloc_ptr[dev];
-  *grid = g_noalloc_grid[dev];
-  return BBTC_OK;
-}
-
-}  // namespace
-
 }  // namespace bbtc
-
-extern "C" int bbtc_count_csr_noalloc(const uint32_t* d_indptr, const uint32_t* d_indices, uint32_t n, uint64_t m,
-                                      uint64_t* out, void* stream) {
-  using namespace bbtc;
-  if (!d_indptr || (m && !d_indices) || !out) return fail(BBTC_ERR_ARG, "NULL argument");
-  if (n == 0xffffffffu) return fail(BBTC_ERR_ARG, "n must be below 2^32 - 1");
-  if (n == 0 && m > 0) return fail(BBTC_ERR_ARG, "a CSR with no rows cannot hold edges (n == 0, m > 0)");
-  if (m > kNoAllocMaxEdges)
-    return fail(BBTC_ERR_CAPACITY, "bbtc_count_csr_noalloc takes at most " + std::to_string(kNoAllocMaxEdges) +
-                                       " oriented edges (its static scratch has one slot per 256 edges); got " +
-                                       std::to_string(m));
-  int dev = 0;
-  BBTC_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= (int)kMaxDevices) return fail(BBTC_ERR_NODEV, "device index beyond the supported range");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  void* ptr = nullptr;
-  uint32_t grid = 0;
-  BBTC_TRY(noalloc_setup(dev, &ptr, &grid));
-  NoAllocScratch* scr = static_cast<NoAllocScratch*>(ptr);
-  // head, error and total start at zero; the partials of this call's units are all rewritten
-  BBTC_CUDA(cudaMemsetAsync(scr, 0, offsetof(NoAllocScratch, pad), s));
-  const uint32_t units = (uint32_t)((m + kNoAllocUnitEdges - 1) / kNoAllocUnitEdges);
-  if (units > 0) {
-    const size_t sm = smem_bytes(kNoAllocBitmapWords, kNoAllocWarps);
-    k_count_csr_static<<<grid, kNoAllocWarps * 32, sm, s>>>(d_indptr, d_indices, n, m, units, scr,
-                                                              kNoAllocBitmapWords);
-    BBTC_CUDA(cudaGetLastError());
-    k_noalloc_total<<<1, 1024, 0, s>>>(scr, units);
-    BBTC_CUDA(cudaGetLastError());
-  }
-  struct {
-    uint32_t head, error;
-    unsigned long long total;
-  } hdr{0, 0, 0};
-  BBTC_CUDA(cudaMemcpyAsync(&hdr, scr, sizeof(hdr), cudaMemcpyDeviceToHost, s));
-  BBTC_CUDA(cudaStreamSynchronize(s));
-  if (hdr.error) return fail(BBTC_ERR_INPUT, "the CSR has a row pointer or column id outside its bounds, or an "
-                                            "unsorted row");
-  *out = hdr.total;
-  return BBTC_OK;
-}

@@ -495,6 +495,10 @@ Kernel kernel_for(uint32_t occ) {
 
 }  // namespace
 
+size_t pivots_smem(uint32_t bm_words, uint32_t warps) {
+  return (size_t)warps * (bm_words + kFrameWords) * sizeof(uint32_t);
+}
+
 int pivots_smem_optin(size_t bytes) {
   for (Kernel k : {k_count_pivots<4>, k_count_pivots<5>, k_count_pivots<6>, k_count_pivots<8>})
     BBTC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -504,7 +508,7 @@ int pivots_smem_optin(size_t bytes) {
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
                   uint32_t total_units, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts) {
   const uint32_t bmw = norm_bm_words(o.bitmap_words), wpb = norm_warps(o.warps_per_block);
-  const size_t sm = (size_t)wpb * (bmw + kFrameWords) * sizeof(uint32_t);
+  const size_t sm = pivots_smem(bmw, wpb);
   const Kernel kern = kernel_for(o.occupancy);
   int per_sm = 0;
   BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * 32, sm));

@@ -305,6 +305,7 @@ inline uint32_t norm_bm_words(uint32_t w) {
 inline uint32_t norm_warps(uint32_t w) { return w == 0 || w > 8 ? 8 : w; }
 
 // fused.cu
+size_t pivots_smem(uint32_t bm_words, uint32_t warps);
 int pivots_smem_optin(size_t bytes);
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
                   uint32_t total_units, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts);

@@ -372,13 +372,13 @@ int bbtc_server_stats_get(bbtc_server* s, bbtc_server_stats* st);
  * cudaFree.  The caller passes a degree-ordered, oriented CSR that is already
  * in device memory of the current device (d_indptr[n+1], d_indices[m], rows
  * strictly increasing) and a host pointer for the count; the call allocates
- * nothing.  Its scratch (queue head, error word, total, one partial count per
- * 256 edges) is a file-scope device array of about 512 KiB that every GPU
- * loading the library holds until the process exits, so m is limited to
- * 16,777,216 oriented edges (larger m: BBTC_ERR_CAPACITY, nothing launched).
- * The first call on a device (with that device current) looks up the array's
- * device address and the kernel's launch shape, once.  All calls share the
- * array and it keeps the last call's contents: each call clears what must
+ * nothing.  Its scratch (queue head, error word, total) is a file-scope device
+ * variable that every GPU loading the library holds until the process exits;
+ * m is limited to 16,777,216 oriented edges (larger m: BBTC_ERR_CAPACITY,
+ * nothing launched).
+ * The first call on a device (with that device current) looks up its
+ * device address and the kernel's launch shape, once.  All calls share it and
+ * it keeps the last call's contents: each call clears what must
  * start at zero, and calls that overlap on the GPU (on different streams or
  * threads) race -- serialise them.  Work is enqueued on `stream` (a
  * cudaStream_t, NULL = the legacy default stream) and the call is synchronous:
