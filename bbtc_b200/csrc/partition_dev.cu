@@ -8,10 +8,10 @@
 //  * uni: cuts[i] = i n / P.
 //  * n1d: the smallest bottleneck B for which the greedy split of the row
 //    pointer prefix into at most P stripes succeeds.  The host bisects over B
-//    with one greedy probe per step; here one kernel evaluates 1024 candidate
-//    bounds at once (a thread per bound, each a greedy probe over the device
-//    row pointers), so four rounds narrow [max(maxrow, m/P), m] to the
-//    minimum.  The cuts are the greedy probe at that minimum, as on the host.
+//    with one greedy probe per step; here one block evaluates 1024 bounds at
+//    once (a thread per bound, each a greedy probe over the device row
+//    pointers), so a few rounds narrow [max(maxrow, m/P), m] to the minimum.
+//    The cuts are the greedy probe at that minimum, as on the host.
 //  * pal: the host draws the same sample of nonzero indices (a seeded
 //    geometric-skip stream that needs only m), the GPU maps each sampled
 //    index to its (row, column), and the probe runs on that sample on the
@@ -58,34 +58,57 @@ __device__ bool n1d_feasible(const uint32_t* __restrict__ indptr, uint32_t n, ui
   return true;
 }
 
-__global__ void k_n1d_candidates(const uint32_t* __restrict__ indptr, uint32_t n, uint32_t P, uint64_t lo,
-                                 uint64_t step, uint64_t hi, uint8_t* __restrict__ ok) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= kCandidates) return;
-  const uint64_t B = lo + (uint64_t)c * step;
-  ok[c] = B <= hi ? (n1d_feasible(indptr, n, P, B) ? 1 : 0) : 2;  // 2: beyond the range
-}
-
-__global__ void k_n1d_cuts(const uint32_t* __restrict__ indptr, uint32_t n, uint32_t P, uint64_t B,
-                           uint32_t* __restrict__ cuts) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  uint32_t start = 0, k = 0;
-  cuts[0] = 0;
-  while (start < n && k < P) {
-    const uint64_t limit = (uint64_t)indptr[start] + B;
-    uint32_t lo = start, hi = n;
-    while (lo < hi) {
-      const uint32_t mid = lo + (hi - lo + 1) / 2;
-      if ((uint64_t)indptr[mid] <= limit) lo = mid; else hi = mid - 1;
+// The minimum feasible bound and its cuts, in one block: every round tests
+// kCandidates bounds spread over [lo, hi] (a thread each) and narrows the
+// range to the gap below the first feasible one, as the host's bisection does
+// (partition_core.hpp: n1d_cuts).  One launch instead of a launch and a host
+// round trip per round; what it costs is the chain of dependent row-pointer
+// loads of a probe (about 20 per stripe).
+__global__ void __launch_bounds__(kCandidates) k_n1d(const uint32_t* __restrict__ indptr, uint32_t n, uint64_t m,
+                                                     uint32_t P, const uint32_t* __restrict__ max_row,
+                                                     uint32_t* __restrict__ cuts) {
+  __shared__ uint32_t first;
+  uint64_t lo = max((uint64_t)*max_row, (m + P - 1) / P);
+  uint64_t hi = max(m, lo);  // feasible
+  while (lo < hi) {
+    const uint64_t step = max((uint64_t)1, (hi - lo + kCandidates) / kCandidates);
+    if (threadIdx.x == 0) first = kCandidates;
+    __syncthreads();
+    const uint64_t B = lo + threadIdx.x * step;
+    if (B <= hi && n1d_feasible(indptr, n, P, B)) atomicMin(&first, threadIdx.x);
+    __syncthreads();
+    const uint32_t f = first;
+    __syncthreads();
+    if (f == kCandidates) {  // only hi itself, past the last candidate
+      lo = lo + (hi - lo) / step * step + 1;
+    } else {
+      const uint64_t b = lo + f * step;
+      if (f > 0) lo = b - step + 1;
+      hi = b;
     }
-    uint32_t end = lo;
-    if (end <= start) end = start + 1;
-    start = end;
-    k++;
-    cuts[k] = start;
   }
-  for (uint32_t t = k + 1; t <= P; t++) cuts[t] = n;
-  cuts[P] = n;
+  // the greedy split at the bound: one warp, 32-way searches
+  if (threadIdx.x >= 32) return;
+  const uint32_t lane = threadIdx.x;
+  uint32_t start = 0, k = 0;
+  if (lane == 0) cuts[0] = 0;
+  while (start < n && k < P) {
+    const uint64_t limit = (uint64_t)indptr[start] + lo;
+    uint32_t a = start, b = n + 1;  // last index in [start, n] with indptr <= limit
+    while (b - a > 1) {
+      const uint32_t step = (b - a + 31) / 32;
+      const uint64_t at = a + (uint64_t)(lane + 1) * step;
+      const uint32_t below = __ballot_sync(0xffffffffu, at < b && (uint64_t)indptr[at] <= limit);
+      a += __popc(below) * step;
+      b = min(b - a, step) + a;
+    }
+    start = a <= start ? start + 1 : a;
+    k++;
+    if (lane == 0) cuts[k] = start;
+  }
+  for (uint32_t t = k + 1 + lane; t <= P; t += 32) cuts[t] = n;
+  __syncwarp();
+  if (lane == 0) cuts[P] = n;
 }
 
 // (row, column) of every sampled nonzero index.
@@ -113,47 +136,14 @@ struct HostPinned {
 
 int n1d_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_indptr, uint64_t m, uint32_t P, uint32_t* cuts) {
   cudaStream_t s = ctx->stream;
-  DevBuf dmax, ok, dcuts;
+  DevBuf dmax, dcuts;
   BBTC_TRY(dalloc(dmax, sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(ok, kCandidates, s));
   BBTC_TRY(dalloc(dcuts, (P + 1) * sizeof(uint32_t), s));
   BBTC_CUDA(cudaMemsetAsync(dmax.p, 0, sizeof(uint32_t), s));
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ctx->sms * 8, (n + 255) / 256));
   k_max_row<<<grid, 256, 0, s>>>(d_indptr, n, dmax.as<uint32_t>());
   BBTC_CUDA(cudaGetLastError());
-  uint32_t* hmax = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageFlags);
-  BBTC_CUDA(cudaMemcpyAsync(hmax, dmax.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  BBTC_CUDA(cudaStreamSynchronize(s));
-  // the host's search range (partition_core.hpp: n1d_cuts)
-  uint64_t lo = std::max<uint64_t>(*hmax, (m + P - 1) / P);
-  uint64_t hi = std::max<uint64_t>(m, lo);
-  uint8_t* hok = reinterpret_cast<uint8_t*>(ctx->h_stage + kStageOut);
-  while (lo < hi) {
-    // hi is feasible; candidates lo, lo + step, ... cover [lo, hi]
-    const uint64_t step = std::max<uint64_t>(1, (hi - lo + kCandidates) / kCandidates);
-    k_n1d_candidates<<<kCandidates / 256, 256, 0, s>>>(d_indptr, n, P, lo, step, hi, ok.as<uint8_t>());
-    BBTC_CUDA(cudaGetLastError());
-    BBTC_CUDA(cudaMemcpyAsync(hok, ok.p, kCandidates, cudaMemcpyDeviceToHost, s));
-    BBTC_CUDA(cudaStreamSynchronize(s));
-    uint32_t first = kCandidates;
-    for (uint32_t c = 0; c < kCandidates; c++)
-      if (hok[c] == 1) {
-        first = c;
-        break;
-      }
-    if (first == kCandidates) {
-      // every candidate below hi failed: the minimum lies above the last one
-      uint32_t last = 0;
-      for (uint32_t c = 0; c < kCandidates; c++)
-        if (hok[c] == 0) last = c;
-      lo = lo + (uint64_t)last * step + 1;
-    } else {
-      const uint64_t B = lo + (uint64_t)first * step;
-      if (first > 0) lo = lo + (uint64_t)(first - 1) * step + 1;
-      hi = B;
-    }
-  }
-  k_n1d_cuts<<<1, 32, 0, s>>>(d_indptr, n, P, lo, dcuts.as<uint32_t>());
+  k_n1d<<<1, kCandidates, 0, s>>>(d_indptr, n, m, P, dmax.as<uint32_t>(), dcuts.as<uint32_t>());
   BBTC_CUDA(cudaGetLastError());
   uint32_t* hc = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageCuts);
   BBTC_CUDA(cudaMemcpyAsync(hc, dcuts.p, (P + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -68,22 +68,55 @@ __global__ void k_rmat(int scale, uint64_t m, double a, double ab, double abc, u
   }
 }
 
-// (min, max) as one 64-bit key; self-loops and ids >= n become the largest key.
+// (min, max) as one key of 2 b bits, b bits an end; self-loops and ids >= n
+// become (n, n), the largest key, and are reported.
 __global__ void k_canon(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m, uint32_t n,
-                        uint64_t* __restrict__ keys) {
+                        int b, uint64_t* __restrict__ keys, uint32_t* __restrict__ dropped) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  bool some = false;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
     const uint32_t u = src[e], v = dst[e];
-    keys[e] = (u == v || u >= n || v >= n) ? ~0ull : ((uint64_t)min(u, v) << 32) | max(u, v);
+    const bool drop = u == v || u >= n || v >= n;
+    some |= drop;
+    keys[e] = drop ? (uint64_t)n << b | n : (uint64_t)min(u, v) << b | max(u, v);
+  }
+  if (some) *dropped = 1u;
+}
+
+// The lower ends are sorted: a run's last edge adds its length to its vertex.
+// The upper ends go to an array that is sorted for the same purpose.
+__global__ void k_ends(const uint64_t* __restrict__ keys, uint64_t m, int b, uint32_t* __restrict__ first,
+                       uint32_t* __restrict__ upper) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t low = (1ull << b) - 1;
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
+    const uint64_t k = keys[e];
+    const uint32_t u = (uint32_t)(k >> b);
+    if (e == 0 || (uint32_t)(keys[e - 1] >> b) != u) first[u] = (uint32_t)e;
+    upper[e] = (uint32_t)(k & low);
   }
 }
 
-__global__ void k_degrees(const uint64_t* __restrict__ keys, uint64_t m, uint32_t* __restrict__ deg) {
+// Degrees from the runs of the sorted lower ends (in the keys) and of the
+// sorted upper ends.  An atomic per end instead took 0.86 ms for 15 M edges of
+// an R-MAT graph (its hubs' counters serialise); both sorts and passes 0.3 ms.
+__global__ void k_degrees(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ upper, uint64_t m, int b,
+                          const uint32_t* __restrict__ first_lower, uint32_t* __restrict__ deg_lower,
+                          uint32_t* __restrict__ first_upper) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
-    const uint64_t k = keys[e];
-    atomicAdd(&deg[k >> 32], 1u);
-    atomicAdd(&deg[k & 0xffffffffull], 1u);
+    const uint32_t u = (uint32_t)(keys[e] >> b), v = upper[e];
+    if (e + 1 == m || (uint32_t)(keys[e + 1] >> b) != u) deg_lower[u] = (uint32_t)e + 1u - first_lower[u];
+    if (e == 0 || upper[e - 1] != v) first_upper[v] = (uint32_t)e;
+  }
+}
+
+__global__ void k_add_upper(const uint32_t* __restrict__ upper, uint64_t m, const uint32_t* __restrict__ first_upper,
+                            uint32_t* __restrict__ deg) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
+    const uint32_t v = upper[e];
+    if (e + 1 == m || upper[e + 1] != v) deg[v] += (uint32_t)e + 1u - first_upper[v];  // one writer a vertex
   }
 }
 
@@ -96,29 +129,32 @@ __global__ void k_rank(const uint32_t* __restrict__ order, uint32_t n, uint32_t*
 }
 
 // relabel both ends and orient from the lower to the higher new id
-__global__ void k_relabel(const uint64_t* __restrict__ keys, uint64_t m, const uint32_t* __restrict__ rank,
+__global__ void k_relabel(const uint64_t* __restrict__ keys, uint64_t m, const uint32_t* __restrict__ rank, int b,
                           uint64_t* __restrict__ out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t low = (1ull << b) - 1;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
     const uint64_t k = keys[e];
-    const uint32_t a = rank[k >> 32], b = rank[k & 0xffffffffull];
-    out[e] = ((uint64_t)min(a, b) << 32) | max(a, b);
+    const uint32_t x = rank[k >> b], y = rank[k & low];
+    out[e] = (uint64_t)min(x, y) << b | max(x, y);
   }
 }
 
-__global__ void k_split(const uint64_t* __restrict__ keys, uint64_t m, uint32_t* __restrict__ indices) {
+__global__ void k_split(const uint64_t* __restrict__ keys, uint64_t m, int b, uint32_t* __restrict__ indices) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t low = (1ull << b) - 1;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride)
-    indices[e] = (uint32_t)(keys[e] & 0xffffffffull);
+    indices[e] = (uint32_t)(keys[e] & low);
 }
 
 // indptr[r] = first edge whose row is >= r
-__global__ void k_indptr(const uint64_t* __restrict__ keys, uint64_t m, uint32_t n, uint32_t* __restrict__ indptr) {
+__global__ void k_indptr(const uint64_t* __restrict__ keys, uint64_t m, uint32_t n, int b,
+                         uint32_t* __restrict__ indptr) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += gridDim.x * blockDim.x) {
     uint64_t lo = 0, hi = m;
     while (lo < hi) {
       const uint64_t mid = (lo + hi) >> 1;
-      if ((keys[mid] >> 32) < r) lo = mid + 1; else hi = mid;
+      if ((keys[mid] >> b) < r) lo = mid + 1; else hi = mid;
     }
     indptr[r] = (uint32_t)lo;
   }
@@ -178,34 +214,32 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   BBTC_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
   const int grid = ctx->sms * 8;
-  const int key_bits = 32 + bits_for(n);
-  Buf keys, keys2, uniq, nsel, deg, ids, ids2, deg2, rank, tmp;
-  BBTC_TRY(balloc(keys, std::max<uint64_t>(m_raw, 1) * 8, s));
-  BBTC_TRY(balloc(keys2, std::max<uint64_t>(m_raw, 1) * 8, s));
-  BBTC_TRY(balloc(nsel, 8, s));
+  const int b = bits_for((uint64_t)n + 1);  // bits of an end: n itself marks the dropped pairs
+  const uint64_t mm = std::max<uint64_t>(m_raw, 1);
+  Buf keys, keys2, sel, ends, firsts, deg, ids, ids2, deg2, rank, tmp;
+  BBTC_TRY(balloc(keys, mm * 8, s));
+  BBTC_TRY(balloc(keys2, mm * 8, s));
+  BBTC_TRY(balloc(sel, 16, s));  // distinct pairs, "some were dropped"
+  BBTC_CUDA(cudaMemsetAsync(sel.p, 0, 16, s));
   uint64_t m_und = 0;
   if (m_raw) {
-    k_canon<<<grid, 256, 0, s>>>(d_src, d_dst, m_raw, n, keys.as<uint64_t>());
+    k_canon<<<grid, 256, 0, s>>>(d_src, d_dst, m_raw, n, b, keys.as<uint64_t>(), sel.as<uint32_t>() + 2);
     BBTC_CUDA(cudaGetLastError());
     size_t tb = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys.as<uint64_t>(), keys2.as<uint64_t>(), (int64_t)m_raw,
-                                             0, 64, s));
+                                             0, 2 * b, s));
     size_t tu = 0;
-    BBTC_CUDA(cub::DeviceSelect::Unique(nullptr, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(),
-                                        nsel.as<uint64_t>(), (int64_t)m_raw, s));
+    BBTC_CUDA(cub::DeviceSelect::Unique(nullptr, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), sel.as<uint64_t>(),
+                                        (int64_t)m_raw, s));
     BBTC_TRY(balloc(tmp, std::max(tb, tu), s));
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb, keys.as<uint64_t>(), keys2.as<uint64_t>(), (int64_t)m_raw, 0,
-                                             64, s));
-    BBTC_CUDA(cub::DeviceSelect::Unique(tmp.p, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), nsel.as<uint64_t>(),
+                                             2 * b, s));
+    BBTC_CUDA(cub::DeviceSelect::Unique(tmp.p, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), sel.as<uint64_t>(),
                                         (int64_t)m_raw, s));
-    uint64_t sel = 0, last = 0;
-    BBTC_CUDA(cudaMemcpyAsync(&sel, nsel.p, 8, cudaMemcpyDeviceToHost, s));
+    uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageFlags);
+    BBTC_CUDA(cudaMemcpyAsync(h, sel.p, 16, cudaMemcpyDeviceToHost, s));
     BBTC_CUDA(cudaStreamSynchronize(s));
-    if (sel) {
-      BBTC_CUDA(cudaMemcpyAsync(&last, keys.as<uint64_t>() + sel - 1, 8, cudaMemcpyDeviceToHost, s));
-      BBTC_CUDA(cudaStreamSynchronize(s));
-    }
-    m_und = (sel && last == ~0ull) ? sel - 1 : sel;  // the dropped pairs sort last
+    m_und = h[0] - ((uint32_t)h[1] ? 1 : 0);  // the dropped pairs' key sorts last
   }
   if (m_und >= (1ull << 32)) return fail(BBTC_ERR_UNSUPPORTED, "more than 2^32 - 1 edges after cleaning");
   BBTC_TRY(balloc(deg, ((size_t)n + 1) * 4, s));
@@ -215,20 +249,36 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   BBTC_TRY(balloc(rank, ((size_t)n + 1) * 4, s));
   BBTC_CUDA(cudaMemsetAsync(deg.p, 0, ((size_t)n + 1) * 4, s));
   if (m_und) {
-    k_degrees<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, deg.as<uint32_t>());
+    BBTC_TRY(balloc(firsts, 2 * ((size_t)n + 1) * 4, s));
+    BBTC_TRY(balloc(ends, 2 * m_und * 4, s));
+    uint32_t* upper = ends.as<uint32_t>();
+    uint32_t* upper_sorted = upper + m_und;
+    uint32_t* first_lower = firsts.as<uint32_t>();
+    uint32_t* first_upper = first_lower + n + 1;
+    k_ends<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, b, first_lower, upper);
+    BBTC_CUDA(cudaGetLastError());
+    size_t te = 0;
+    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, te, upper, upper_sorted, (int64_t)m_und, 0, b, s));
+    Buf tmp4;
+    BBTC_TRY(balloc(tmp4, te, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp4.p, te, upper, upper_sorted, (int64_t)m_und, 0, b, s));
+    k_degrees<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), upper_sorted, m_und, b, first_lower, deg.as<uint32_t>(),
+                                   first_upper);
+    BBTC_CUDA(cudaGetLastError());
+    k_add_upper<<<grid, 256, 0, s>>>(upper_sorted, m_und, first_upper, deg.as<uint32_t>());
     BBTC_CUDA(cudaGetLastError());
   }
   if (n) {
     k_iota32<<<grid, 256, 0, s>>>(ids.as<uint32_t>(), n);
     BBTC_CUDA(cudaGetLastError());
-    // stable sort of ids by degree: ties keep id order
+    // stable sort of ids by degree (below n): ties keep id order
     size_t tr = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tr, deg.as<uint32_t>(), deg2.as<uint32_t>(), ids.as<uint32_t>(),
-                                              ids2.as<uint32_t>(), (int64_t)n, 0, 32, s));
+                                              ids2.as<uint32_t>(), (int64_t)n, 0, b, s));
     Buf tmp2;
     BBTC_TRY(balloc(tmp2, tr, s));
     BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp2.p, tr, deg.as<uint32_t>(), deg2.as<uint32_t>(), ids.as<uint32_t>(),
-                                              ids2.as<uint32_t>(), (int64_t)n, 0, 32, s));
+                                              ids2.as<uint32_t>(), (int64_t)n, 0, b, s));
     k_rank<<<grid, 256, 0, s>>>(ids2.as<uint32_t>(), n, rank.as<uint32_t>());
     BBTC_CUDA(cudaGetLastError());
   }
@@ -241,19 +291,19 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     return fail(BBTC_ERR_NOMEM, "device allocation of the oriented CSR failed");
   }
   if (m_und) {
-    k_relabel<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, rank.as<uint32_t>(), keys2.as<uint64_t>());
+    k_relabel<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, rank.as<uint32_t>(), b, keys2.as<uint64_t>());
     BBTC_CUDA(cudaGetLastError());
     size_t tb = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), (int64_t)m_und, 0,
-                                             key_bits, s));
+                                             2 * b, s));
     Buf tmp3;
     BBTC_TRY(balloc(tmp3, tb, s));
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp3.p, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), (int64_t)m_und, 0,
-                                             key_bits, s));
-    k_split<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, d_indices);
+                                             2 * b, s));
+    k_split<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, b, d_indices);
     BBTC_CUDA(cudaGetLastError());
   }
-  k_indptr<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, n, d_indptr);
+  k_indptr<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, n, b, d_indptr);
   BBTC_CUDA(cudaGetLastError());
   BBTC_CUDA(cudaStreamSynchronize(s));
   out->indptr = d_indptr;
