@@ -31,8 +31,6 @@
 // walks a whole row.
 #include <cub/cub.cuh>
 #include <cuda.h>
-#include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cstring>
@@ -98,8 +96,19 @@ struct CutVec {
   uint32_t P;
 };
 
-// Words of the flags block that the build leaves for the host.
-enum : uint32_t { kFlagBad = 0, kFlagUnoriented = 1, kFlagPivots = 2, kFlagPairs = 3, kFlagSparse = 4, kFlagWords = 8 };
+// Words of the flags block: what the build leaves for the host, and the tile
+// tickets of the two single-pass kernels.
+enum : uint32_t {
+  kFlagBad = 0,
+  kFlagUnoriented = 1,
+  kFlagPivots = 2,
+  kFlagPairs = 3,
+  kFlagSparse = 4,
+  kFlagTicketPairs = 5,
+  kFlagTicketPivots = 6,
+  kFlagWords = 8
+};
+constexpr uint32_t kBadWait = 1u << 30;  // in kFlagBad: a wait for an earlier tile ran out
 
 // Row part of the input contract, a thread per row: row pointers start at 0,
 // never decrease and end at m.  Sets the bit of every edge that starts a row
@@ -120,124 +129,391 @@ __global__ void k_row_heads(const uint32_t* __restrict__ indptr, const uint32_t*
   }
 }
 
-__device__ __forceinline__ bool is_head(const uint32_t* __restrict__ heads, uint64_t e) {
-  return (heads[e >> 5] >> (e & 31)) & 1u;
+// ---- single-pass tiles --------------------------------------------------------
+// The two passes below number things (pairs, pivots) across the whole edge
+// array in one read of it: a block takes the next tile by ticket, counts in
+// it, publishes the count, and adds up the tiles before it from what they have
+// published -- their own counts, or from some tile on the sum up to it.  A
+// tile's word is (state << 62 | value): 0 nothing yet, 1 the tile's own, 2 up
+// to and including it.  Tickets follow the order in which blocks start, so the
+// tiles waited for are running or done; the waits are bounded all the same.
+// Tiles are small (8 warps of 8 chunks of 32) while few of them would leave
+// SMs idle, and large (16 warps of 16 chunks) where the sum over earlier tiles
+// would bound the pass.  Small and large, us: k_pairs R-MAT s12 7.2 / 12.4,
+// s18 45 / 32, s22 570 / 420; k_pivots 8.8 / 16.9, 36 / 42, 371 / 276.
+constexpr uint32_t kSmallWarps = 8, kSmallChunks = 8, kLargeWarps = 16, kLargeChunks = 16;
+constexpr uint64_t kLargePairs = 1ull << 20, kLargePivots = 4ull << 20;  // edges from which tiles are large
+inline uint64_t tile_size(bool large) {
+  return 32 * (large ? (uint64_t)kLargeWarps * kLargeChunks : (uint64_t)kSmallWarps * kSmallChunks);
+}
+constexpr uint64_t kOwn = 1ull << 62, kUpTo = 2ull << 62;
+constexpr uint32_t kTilePolls = 1u << 22;
+
+__device__ __forceinline__ uint64_t tile_load(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tile_store(uint64_t* p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// 1 for an edge that opens a new (word, mask) pair of its row: the input of the pair positions' scan.
-struct OpensPair {
-  const uint32_t* indices;
-  const uint32_t* heads;
-  __device__ __forceinline__ uint32_t operator()(uint64_t e) const {
-    return e == 0 || (indices[e] >> 5) != (indices[e - 1] >> 5) || is_head(heads, e) ? 1u : 0u;
-  }
+// What the tiles before tile i (in ticket order) hold together.  `a` carries
+// counts; with HEADS, `b` carries for each tile the count from its first head
+// on (0: no head) -- the counts run towards the tiles before, so the nearest
+// tile with a head gives the count up to it.  Called by one warp.
+struct TileSum {
+  uint32_t count, head;
 };
+template <bool HEADS>
+__device__ __forceinline__ TileSum tiles_before(const uint64_t* a, const uint64_t* b, uint32_t i, uint32_t* bad) {
+  const uint32_t lane = threadIdx.x & 31;
+  TileSum out{0, 0};
+  uint32_t polls = 0;
+  for (int64_t j = (int64_t)i - 1; j >= 0; j -= 32) {
+    const int64_t at = j - lane;
+    uint64_t va = kUpTo, vb = kUpTo;  // before the first tile: nothing
+    bool ok;
+    do {
+      if (at >= 0) {
+        va = tile_load(a + at);
+        vb = HEADS ? tile_load(b + at) : va;
+      }
+      ok = va >> 62 != 0 && va >> 62 == vb >> 62;  // both words of one publication
+      if (!ok && ++polls > kTilePolls) {
+        atomicOr(bad, kBadWait);
+        va = vb = kUpTo;
+        ok = true;
+      }
+    } while (!__all_sync(FULLMASK, ok));
+    const uint32_t sums = __ballot_sync(FULLMASK, va >> 62 == 2);
+    const uint32_t last = sums ? __ffs(sums) - 1 : 32;  // the nearest tile with a sum
+    const uint32_t own = lane < last ? (uint32_t)va : 0u;
+    if (HEADS && out.head == 0) {
+      const uint32_t some = __ballot_sync(FULLMASK, lane < last && (uint32_t)vb != 0);
+      if (some) {  // the tiles between that head and here are in out.count and before it in the window
+        const uint32_t f = __ffs(some) - 1;
+        out.head = __shfl_sync(FULLMASK, (uint32_t)vb, f) + __reduce_add_sync(FULLMASK, lane > f ? own : 0u);
+      } else if (last < 32) {
+        out.head = __shfl_sync(FULLMASK, (uint32_t)vb, last);
+        out.count += __reduce_add_sync(FULLMASK, own) + __shfl_sync(FULLMASK, (uint32_t)va, last);
+        return out;
+      }
+    } else if (HEADS) {
+      out.head += __reduce_add_sync(FULLMASK, own);
+    }
+    out.count += __reduce_add_sync(FULLMASK, own);
+    if (last < 32) {
+      const uint32_t sum = __shfl_sync(FULLMASK, (uint32_t)va, last);
+      out.count += sum;
+      if (HEADS && out.head) out.head += sum;
+      return out;
+    }
+  }
+  return out;
+}
 
 // Edge part of the input contract (rows strictly increasing, ids < n), the
-// word-compressed rows and the records.  wpos = inclusive scan of OpensPair,
-// so edge e lands in pair wpos[e] - 1.  A warp takes 32 consecutive edges; a
-// pair's edges are consecutive, so a segmented suffix OR by shuffles (five
-// steps, no divergence) gives the first lane of each pair in the chunk the
-// bits of the pair's edges in the chunk.  The lane of the edge that opens a
-// pair stores it, after ORing in the bits of its edges past the chunk (at most
-// 31 more, only for the chunk's last pair); a pair that opened in an earlier
-// chunk is that chunk's to store.  So each pair has one writer and no atomics.
-// Record of edge e: its own pair and the end of its row's pairs, which is the
-// pair of the next row's first edge -- in the chunk, or (one search a chunk)
-// after it.  Needs m > 0.
-__global__ void k_pairs(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ heads,
-                        const uint32_t* __restrict__ wpos, uint32_t n, uint64_t m, uint2* __restrict__ words,
-                        uint2* __restrict__ rec, uint32_t* __restrict__ flags) {
-  const uint32_t W = wpos[m - 1];
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t nheads = (m + 31) / 32;
-  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;  // a multiple of 32: warps keep their chunks aligned
-  if (t0 == 0) flags[kFlagPairs] = W;
-  for (uint64_t e = t0; e - lane < m; e += stride) {
-    const bool valid = e < m;
-    const uint32_t hw = heads[e >> 5];
-    const uint32_t x = valid ? indices[e] : 0u;
-    const uint32_t p = valid ? wpos[e] - 1u : 0xffffffffu;
-    uint32_t prev = __shfl_up_sync(FULLMASK, x, 1);
-    if (lane == 0) prev = e > 0 ? indices[e - 1] : 0u;
-    const bool head = e == 0 || ((hw >> lane) & 1u);
-    uint32_t v = valid ? 1u << (x & 31) : 0u;
+// word-compressed rows and the records, in one read of the ids.  Pairs are
+// numbered from the end of the array, pair p = m - (pairs opened from it on),
+// so tiles run from the last edges to the first and the end of an edge's row
+// -- the pair of the next row's first edge -- is known when the edge is
+// reached.  A pair's edges are consecutive and their bits distinct, so its
+// mask is a difference of running sums; the lane of the edge that opens it
+// writes it.  head_pair[e] is written for edges that start a row.  Needs m > 0.
+//
+// It replaces a scan of the openings and a pass that read its result and
+// searched the row ends: R-MAT s22 0.94 ms before, 0.42 now (1.3 GB moved: the
+// shuffles and population counts of a chunk bound it, not memory), s12 20 us
+// in three launches before, 7 in one.
+template <uint32_t kTileWarps, uint32_t kTileChunks, int MINB>
+__global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pairs(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ heads,
+                                               uint32_t n, uint64_t m, uint2* __restrict__ words,
+                                               uint2* __restrict__ rec, uint32_t* __restrict__ head_pair,
+                                               uint64_t* __restrict__ sums, uint64_t* __restrict__ head_sums,
+                                               uint32_t* __restrict__ flags) {
+  __shared__ uint32_t s_tile, s_count[kTileWarps], s_head[kTileWarps];
+  __shared__ TileSum s_before;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr uint32_t kTile = kTileWarps * kTileChunks * 32;
+  const uint32_t ntiles = (uint32_t)((m + kTile - 1) / kTile);
+  while (true) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&flags[kFlagTicketPairs], 1u);
+    __syncthreads();
+    const uint32_t i = s_tile;
+    if (i >= ntiles) return;
+    const uint64_t base = (uint64_t)(ntiles - 1 - i) * kTile + warp * (kTileChunks * 32);
+    uint32_t x[kTileChunks];
 #pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-      const uint32_t o = __shfl_down_sync(FULLMASK, v, d);
-      const uint32_t po = __shfl_down_sync(FULLMASK, p, d);
-      if (lane + d < 32 && po == p) v |= o;
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      const uint64_t e = base + 32 * c + lane;
+      x[c] = e < m ? __ldg(indices + e) : 0u;
     }
-    const uint32_t p_last = __shfl_sync(FULLMASK, p, 31);
-    // the end of this edge's row: the next head's pair
-    const uint32_t later = lane < 31 ? hw & (FULLMASK << (lane + 1)) : 0u;
-    const uint32_t end = __shfl_sync(FULLMASK, p, later ? __ffs(later) - 1 : 0);
-    uint32_t far = W;  // the first head after the chunk
-    for (uint64_t c = (e >> 5) + 1; c < nheads; c += 32) {
-      const uint32_t o = c + lane < nheads ? heads[c + lane] : 0u;
-      const uint32_t some = __ballot_sync(FULLMASK, o != 0);
-      if (!some) continue;
-      const uint32_t src = __ffs(some) - 1;
-      const uint32_t word = __shfl_sync(FULLMASK, o, src);
-      const uint64_t at = (c + src) * 32 + (__ffs(word) - 1);
-      if (at < m) far = wpos[at] - 1u;
-      break;
+    // lane c: the words of chunk c -- edges that start a row, edges that open a pair
+    uint32_t my_heads = 0, my_opens = 0, bad = 0;
+    if (lane < kTileChunks && base + 32 * lane < m) my_heads = __ldg(heads + (base >> 5) + lane);
+    if (base == 0 && lane == 0) my_heads |= 1u;
+    uint32_t before = base > 0 && base < m ? __ldg(indices + base - 1) : 0u;
+#pragma unroll
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      const bool valid = base + 32 * c + lane < m;
+      const bool head = (__shfl_sync(FULLMASK, my_heads, c) >> lane) & 1u;
+      uint32_t prev = __shfl_up_sync(FULLMASK, x[c], 1);
+      if (lane == 0) prev = before;
+      before = __shfl_sync(FULLMASK, x[c], 31);
+      if (valid && x[c] >= n) bad |= 8u;
+      if (valid && !head && prev >= x[c]) bad |= 16u;
+      const uint32_t o = __ballot_sync(FULLMASK, valid && (head || (prev ^ x[c]) >> 5 != 0));
+      if (lane == c) my_opens = o;
     }
-    if (!valid) continue;
-    if (x >= n) atomicOr(&flags[kFlagBad], 8u);
-    if (!head && prev >= x) atomicOr(&flags[kFlagBad], 16u);
-    rec[e] = make_uint2(p, later ? end : far);
-    if (!head && (prev >> 5) == (x >> 5)) continue;  // not the opening edge of its pair
-    if (p_last == p) {  // the pair reaches the chunk's last edge: it may go on past the chunk
-      const uint64_t far_k = min(e - lane + 63, m);
-      for (uint64_t k = e - lane + 32; k < far_k && wpos[k] - 1u == p; k++) v |= 1u << (indices[k] & 31);
+    if (bad) atomicOr(&flags[kFlagBad], bad);
+    // the warp's pairs, and from its first head on
+    const uint32_t count = __reduce_add_sync(FULLMASK, __popc(my_opens));
+    {
+      const uint32_t some = __ballot_sync(FULLMASK, my_heads != 0);
+      uint32_t from = 0;
+      if (some) {
+        const uint32_t c = __ffs(some) - 1;
+        from = __reduce_add_sync(FULLMASK, lane < c ? 0u
+                                           : lane == c ? __popc(my_opens & (FULLMASK << (__ffs(my_heads) - 1)))
+                                                       : __popc(my_opens));
+      }
+      if (lane == 0) {
+        s_count[warp] = count;
+        s_head[warp] = from;
+      }
     }
-    words[p] = make_uint2(x >> 5, v);
+    __syncthreads();
+    // later warps of the tile, then the tiles before this one (they hold the later edges)
+    uint32_t C = 0, H = 0, tile_C = 0, tile_H = 0;
+    for (int w = kTileWarps - 1; w >= 0; w--) {
+      if (w == (int)warp) {
+        C = tile_C;
+        H = tile_H;
+      }
+      if (s_head[w]) tile_H = tile_C + s_head[w];
+      tile_C += s_count[w];
+    }
+    if (warp == 0) {
+      if (lane == 0 && i > 0) {
+        tile_store(sums + i, kOwn | tile_C);
+        tile_store(head_sums + i, kOwn | tile_H);
+      }
+      const TileSum b = tiles_before<true>(sums, head_sums, i, &flags[kFlagBad]);
+      if (lane == 0) {
+        tile_store(sums + i, kUpTo | (b.count + tile_C));
+        tile_store(head_sums + i, kUpTo | (tile_H ? b.count + tile_H : b.head));
+        s_before = b;
+        if (i == ntiles - 1) flags[kFlagPairs] = b.count + tile_C;
+      }
+    }
+    __syncthreads();
+    if (H) H += s_before.count; else H = s_before.head;
+    C += s_before.count;
+    // bits of the edges after the warp's that belong to its last pair
+    uint32_t tail = 0;
+    if (base + kTileChunks * 32 < m) {
+      const uint64_t e = base + kTileChunks * 32 + lane;
+      const uint32_t y = e < m ? __ldg(indices + e) : 0u;
+      uint32_t prev = __shfl_up_sync(FULLMASK, y, 1);
+      if (lane == 0) prev = before;
+      const uint32_t hw = __ldg(heads + (e >> 5));
+      const uint32_t o = __ballot_sync(FULLMASK, e >= m || ((hw >> lane) & 1u) || (prev ^ y) >> 5 != 0);
+      const uint32_t f = o ? __ffs(o) - 1 : 32;
+      tail = __reduce_or_sync(FULLMASK, lane < f ? 1u << (y & 31) : 0u);
+    }
+#pragma unroll
+    for (int c = kTileChunks - 1; c >= 0; c--) {
+      const uint64_t e = base + 32 * c + lane;
+      const bool valid = e < m;
+      const uint32_t o = __shfl_sync(FULLMASK, my_opens, c), hw = __shfl_sync(FULLMASK, my_heads, c);
+      const uint32_t bit = valid ? 1u << (x[c] & 31) : 0u;
+      uint32_t run = bit;  // running sum of the bits (modulo 2^32: only differences are used)
+#pragma unroll
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULLMASK, run, d);
+        if (lane >= d) run += v;
+      }
+      const uint32_t above = lane < 31 ? FULLMASK << (lane + 1) : 0u;
+      const uint32_t next = o & above, next_head = hw & above;
+      const uint32_t run_end = __shfl_sync(FULLMASK, run, next ? __ffs(next) - 2 : 31);
+      const uint32_t p = (uint32_t)m - (C + __popc(next) + 1);
+      if (valid) {
+        const uint32_t end = next_head ? C + __popc(o & (FULLMASK << (__ffs(next_head) - 1))) : H;
+        rec[e] = make_uint2(p, (uint32_t)m - end);
+        if ((o >> lane) & 1u) {
+          uint32_t mask = run_end - (run - bit);
+          if (!next) mask |= tail;
+          words[p] = make_uint2(x[c] >> 5, mask);
+          if ((hw >> lane) & 1u) head_pair[e] = p;
+        }
+      }
+      const uint32_t f = o ? __ffs(o) - 1 : 32;
+      const uint32_t open_bits = __reduce_or_sync(FULLMASK, lane < f ? bit : 0u);
+      tail = o ? open_bits : open_bits | tail;
+      if (hw) H = C + __popc(o & (FULLMASK << (__ffs(hw) - 1)));
+      C += __popc(o);
+    }
+    __syncthreads();
   }
 }
-
-// First and end position of every key in the sorted keys (both arrays start at zero).
-__global__ void k_key_bounds(const uint32_t* __restrict__ keys, uint64_t m, uint32_t n, uint32_t* __restrict__ first,
-                             uint32_t* __restrict__ end) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride) {
-    const uint32_t k = keys[q];
-    if (k >= n) continue;  // a refused input
-    if (q == 0 || keys[q - 1] != k) first[k] = (uint32_t)q;
-    if (q == m - 1 || keys[q + 1] != k) end[k] = (uint32_t)(q + 1);
-  }
-}
-
-// A vertex is a pivot when it has in-edges and a row.
-struct IsPivot {
-  const uint32_t* first;
-  const uint32_t* end;
-  const uint32_t* indptr;
-  __device__ __forceinline__ uint32_t operator()(uint32_t v) const {
-    return end[v] > first[v] && indptr[v + 1] > indptr[v] ? 1u : 0u;
-  }
-};
 
 // What the passes after the sort read.
 struct PivotInput {
   const uint32_t* indptr;
   const uint32_t* indices;
-  const uint32_t* wpos;
-  const uint32_t* keys;   // entries' vertices, sorted
-  const uint32_t* first;  // per vertex, its entries [first, end)
-  const uint32_t* end;
-  const uint32_t* pos;    // exclusive scan of IsPivot
+  const uint32_t* head_pair;  // at every edge that starts a row: the row's first pair
+  const uint32_t* keys;       // entries' vertices, sorted
   const uint2* words;
   uint32_t n;
   uint64_t m;
 };
 
-// First pair of row u (u <= n).
+// First pair of row u (u <= n; an empty row's is its successor's).
 __device__ __forceinline__ uint32_t row_pair(const PivotInput& in, uint32_t u) {
   const uint32_t e = in.indptr[u];
-  return (uint64_t)e < in.m ? in.wpos[e] - 1u : in.wpos[in.m - 1];
+  return (uint64_t)e < in.m ? in.head_pair[e] : (uint32_t)in.m;
 }
+
+// Four consecutive batches of 32 entries with this many pivots or more count as sparse.
+constexpr uint32_t kSparsePivots = 8;
+
+// The pivots (8 words each, see PivotGraph), after the last one whose e0 is ~0,
+// and crow, in one read of the sorted keys: a vertex is a pivot when it has
+// in-edges and a row.  An entry whose key differs from the one before starts
+// its vertex's in-edges and ends the previous vertex's.  It replaces four
+// passes and five launches (R-MAT s22 0.32 ms, s12 23 us; now 0.28 ms and 9
+// us).  (For a CSR with ids
+// below their rows, k_fix_pivots and k_fix_entries go over the result.)
+template <uint32_t kTileWarps, uint32_t kTileChunks, int MINB>
+__global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pivots(PivotInput in, uint32_t* __restrict__ piv, uint32_t* __restrict__ crow,
+                                                uint64_t* __restrict__ sums, uint32_t* __restrict__ flags) {
+  if (flags[kFlagBad]) return;
+  __shared__ uint32_t s_tile, s_count[kTileWarps], s_before;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t m = in.m;
+  constexpr uint32_t kTile = kTileWarps * kTileChunks * 32;
+  const uint32_t ntiles = (uint32_t)((m + kTile - 1) / kTile);
+  auto has_row = [&](uint32_t v) { return __ldg(in.indptr + v + 1) > __ldg(in.indptr + v); };
+  while (true) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&flags[kFlagTicketPivots], 1u);
+    __syncthreads();
+    const uint32_t i = s_tile;
+    if (i >= ntiles) return;
+    const uint64_t base = (uint64_t)i * kTile + warp * (kTileChunks * 32);
+    uint32_t key[kTileChunks];
+#pragma unroll
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      const uint64_t e = base + 32 * c + lane;
+      key[c] = e < m ? __ldg(in.keys + e) : ~0u;
+    }
+    const uint32_t last_before = base > 0 && base < m ? __ldg(in.keys + base - 1) : ~0u;
+    uint32_t start_bits = 0;  // bit c: this lane's entry of chunk c starts a vertex
+    uint32_t r0[kTileChunks], r1[kTileChunks];  // and that vertex's row pointers, all asked for before any is looked at
+#pragma unroll
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      uint32_t prev = __shfl_up_sync(FULLMASK, key[c], 1);
+      const uint32_t left = c ? __shfl_sync(FULLMASK, key[c ? c - 1 : 0], 31) : last_before;
+      if (lane == 0) prev = left;
+      const bool start = base + 32 * c + lane < m && prev != key[c];
+      start_bits |= start ? 1u << c : 0u;
+      r0[c] = r1[c] = 0;
+      if (start || (c == 0 && lane == 0 && base < m)) {
+        r0[c] = __ldg(in.indptr + key[c]);
+        r1[c] = __ldg(in.indptr + key[c] + 1);
+      }
+    }
+    // lane c: of chunk c, the entries that start a vertex, those that start a
+    // pivot, and whether its first entry's vertex is one
+    uint32_t my_starts = 0, my_pivots = 0, my_first = 0;
+    uint32_t row = 0;  // whether the vertex that is open has a row
+#pragma unroll
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      const uint32_t starts = __ballot_sync(FULLMASK, (start_bits >> c) & 1u);
+      uint32_t rows = 0;
+      if (starts || c == 0) rows = __ballot_sync(FULLMASK, r1[c] > r0[c]);
+      if (c == 0 || (starts & 1u)) row = rows & 1u;
+      if (lane == c) {
+        my_starts = starts;
+        my_pivots = starts & rows;
+        my_first = row;
+      }
+      if (starts) row = (rows >> (31 - __clz(starts))) & 1u;
+    }
+    const uint32_t mine = __popc(my_pivots);
+    uint32_t incl = mine;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULLMASK, incl, d);
+      if (lane >= d) incl += v;
+    }
+    {
+      const uint32_t ahead = __shfl_sync(FULLMASK, incl - mine, (lane + 4) & 31);
+      const bool sparse = lane + 4 < kTileChunks && ahead - (incl - mine) >= kSparsePivots;
+      const uint32_t some = __ballot_sync(FULLMASK, sparse);
+      if (lane == 0 && some) atomicMax(&flags[kFlagSparse], (uint32_t)(base >> 5) + 35 - __clz(some));
+    }
+    if (lane == 31) s_count[warp] = incl;
+    __syncthreads();
+    uint32_t C = 0, tile_C = 0;
+    for (uint32_t w = 0; w < kTileWarps; w++) {
+      if (w == warp) C = tile_C;
+      tile_C += s_count[w];
+    }
+    if (warp == 0) {
+      if (lane == 0 && i > 0) tile_store(sums + i, kOwn | tile_C);
+      const TileSum b = tiles_before<false>(sums, sums, i, &flags[kFlagBad]);
+      if (lane == 0) {
+        tile_store(sums + i, kUpTo | (b.count + tile_C));
+        s_before = b.count;
+        if (i == ntiles - 1) {
+          const uint32_t k = b.count + tile_C;
+          flags[kFlagPivots] = k;
+          uint4* end = reinterpret_cast<uint4*>(piv + 8 * (uint64_t)k);
+          end[0] = make_uint4(~0u, ~0u, 0, 0);
+          end[1] = make_uint4(0, 0, 0, 0);
+        }
+      }
+    }
+    __syncthreads();
+    C += s_before;
+    if (lane < kTileChunks && base + 32 * lane < m)
+      crow[(base >> 5) + lane] = C + (incl - mine) + (my_first ? (my_pivots & 1u) - 1u : 0u);
+#pragma unroll
+    for (uint32_t c = 0; c < kTileChunks; c++) {
+      const uint32_t starts = __shfl_sync(FULLMASK, my_starts, c), pivots = __shfl_sync(FULLMASK, my_pivots, c);
+      if (starts == 0) continue;
+      const uint64_t e = base + 32 * c + lane;
+      uint32_t prev = __shfl_up_sync(FULLMASK, key[c], 1);
+      const uint32_t left = c ? __shfl_sync(FULLMASK, key[c ? c - 1 : 0], 31) : last_before;
+      if (lane == 0) prev = left;
+      if ((starts >> lane) & 1u) {
+        const uint32_t k = C + __popc(pivots & ~(FULLMASK << lane));  // pivots before this entry
+        if (e > 0 && has_row(prev)) piv[8 * (uint64_t)(k - 1) + 1] = (uint32_t)e;
+        if ((pivots >> lane) & 1u) {
+          const uint32_t v = key[c], a = __ldg(in.indptr + v), b = __ldg(in.indptr + v + 1);
+          const uint32_t ws = in.head_pair[a], we = row_pair(in, v + 1);
+          const uint32_t fw = __ldg(in.indices + a) >> 5, lw = __ldg(in.indices + b - 1) >> 5;
+          uint32_t* d = piv + 8 * (uint64_t)k;
+          d[0] = (uint32_t)e;
+          *reinterpret_cast<uint2*>(d + 2) = make_uint2(ws, we - ws);
+          *reinterpret_cast<uint4*>(d + 4) = make_uint4(fw, lw - fw + 1, FULLMASK, v);
+        }
+      }
+      C += __popc(pivots);
+    }
+    // the warp of the last entry ends its vertex
+    if (base < m && m <= base + kTileChunks * 32 && row && lane == 0) piv[8 * (uint64_t)(C - 1) + 1] = (uint32_t)m;
+    __syncthreads();
+  }
+}
+
+// ---- CSRs with ids below their rows -------------------------------------------
+// The tasks (i, j, k) with j = part(v), i <= j <= k meet only in-edges of v
+// from parts up to j (the entries are in source order) and ids of row v from
+// cuts[j] on (the reference's tiles ab = (i, j), ac = (i, k), bc = (j, k),
+// src/triangle_counting/gpu_sparse_kernel.cu:25-46).  Where every id exceeds
+// its row's, that is all of them.
 
 // The row that holds pair p.
 __device__ uint32_t row_of_pair(const PivotInput& in, uint32_t p) {
@@ -249,57 +525,41 @@ __device__ uint32_t row_of_pair(const PivotInput& in, uint32_t p) {
   return lo;
 }
 
-// The pivots (8 words each, see PivotGraph) and, after the last, one whose e0
-// is ~0.  When every id exceeds its row's, all in-edges of v lie in tasks that
-// meet row v and no id of row v lies below v's part.  Otherwise the tasks
-// (i, j, k) with j = part(v), i <= j <= k meet only in-edges from parts up to
-// j (the entries are in source order) and ids from cuts[j] on (the reference's
-// tiles ab = (i, j), ac = (i, k), bc = (j, k),
-// src/triangle_counting/gpu_sparse_kernel.cu:25-46).
-__global__ void k_pivots(PivotInput in, CutVec cuts, const uint2* __restrict__ rec, uint4* __restrict__ piv,
-                         uint32_t* __restrict__ flags) {
-  if (flags[kFlagBad]) return;
-  const bool plain = flags[kFlagUnoriented] == 0;
-  const IsPivot is{in.first, in.end, in.indptr};
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < in.n; t += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = (uint32_t)t;
-    const uint32_t k = in.pos[v];
-    const uint32_t some = is(v);
-    if (v == in.n - 1) {
-      flags[kFlagPivots] = k + some;
-      piv[2 * (uint64_t)(k + some)] = make_uint4(~0u, ~0u, 0, 0);
-      piv[2 * (uint64_t)(k + some) + 1] = make_uint4(0, 0, 0, 0);
+__global__ void k_fix_pivots(PivotInput in, CutVec cuts, const uint2* __restrict__ rec, uint32_t npiv,
+                             uint4* __restrict__ piv) {
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < npiv; k += (uint64_t)gridDim.x * blockDim.x) {
+    uint4 d0 = piv[2 * k], d1 = piv[2 * k + 1];
+    const uint32_t v = d1.w, part = part_of(cuts.c, cuts.P, v), row_end = in.indptr[v + 1];
+    const uint32_t a = lower_bound_range(in.indices, in.indptr[v], row_end, cuts.c[part]);
+    uint32_t lo = d0.x, hi = d0.y;  // first entry from a later part
+    while (lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      if (row_of_pair(in, rec[mid].x) < cuts.c[part + 1]) lo = mid + 1; else hi = mid;
     }
-    if (!some) continue;
-    uint32_t a = in.indptr[v], b = in.indptr[v + 1], e0 = in.first[v], e1 = in.end[v], mask0 = FULLMASK;
-    if (!plain) {
-      const uint32_t part = part_of(cuts.c, cuts.P, v);
-      a = lower_bound_range(in.indices, a, b, cuts.c[part]);
-      if (a < b) mask0 <<= in.indices[a] & 31;
-      uint32_t lo = e0, hi = e1;  // first entry from a later part
-      while (lo < hi) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (row_of_pair(in, rec[mid].x) < cuts.c[part + 1]) lo = mid + 1; else hi = mid;
+    d0.y = lo;
+    if (a < row_end) {  // from the pair of the first kept id on
+      const uint32_t fw = in.indices[a] >> 5, we = d0.z + d0.w;
+      uint32_t p = d0.z, end = we;
+      while (p < end) {
+        const uint32_t mid = p + ((end - p) >> 1);
+        if (in.words[mid].x < fw) p = mid + 1; else end = mid;
       }
-      e1 = lo;
+      d0.z = p;
+      d0.w = we - p;
+      d1 = make_uint4(fw, (in.indices[row_end - 1] >> 5) - fw + 1, FULLMASK << (in.indices[a] & 31), v);
+    } else {
+      d0.z = d0.w = 0;
+      d1 = make_uint4(0, 0, FULLMASK, v);
     }
-    uint32_t ws = 0, wn = 0, fw = 0, span = 0;
-    if (a < b) {
-      ws = in.wpos[a] - 1u;
-      wn = row_pair(in, v + 1) - ws;
-      fw = in.indices[a] >> 5;
-      span = (in.indices[b - 1] >> 5) - fw + 1;
-    }
-    piv[2 * (uint64_t)k] = make_uint4(e0, e1, ws, wn);
-    piv[2 * (uint64_t)k + 1] = make_uint4(fw, span, mask0, v);
+    piv[2 * k] = d0;
+    piv[2 * k + 1] = d1;
   }
 }
 
 // First pair of the record of entry (u, v): the streamed side is row u from
 // the first pair whose word can hold a kept id of row v (first kept id L).
-// When L lies in v's word or above -- always, when every id exceeds its row's
-// -- that is the pair `p` holding v itself; otherwise the pair is searched in
-// row u's pairs before p.
+// When L lies in v's word or above that is the pair `p` holding v itself;
+// otherwise the pair is searched in row u's pairs before p.
 __device__ __forceinline__ uint32_t record_start(const PivotInput& in, uint32_t v, uint32_t lo, uint32_t p) {
   const uint32_t a = in.indptr[v], b = in.indptr[v + 1];
   const uint32_t k = lower_bound_range(in.indices, a, b, lo);
@@ -314,28 +574,14 @@ __device__ __forceinline__ uint32_t record_start(const PivotInput& in, uint32_t 
   return lo_p;
 }
 
-// Four consecutive batches of 32 entries with this many pivots or more count as sparse.
-constexpr uint32_t kSparsePivots = 8;
-
-// crow, and the records' first pairs when the CSR is not oriented upwards.
-__global__ void k_entry_index(PivotInput in, CutVec cuts, const uint4* __restrict__ piv, uint32_t* __restrict__ crow,
-                              uint2* __restrict__ rec, uint32_t* __restrict__ flags) {
-  if (flags[kFlagBad]) return;
-  const bool plain = flags[kFlagUnoriented] == 0;
-  const IsPivot is{in.first, in.end, in.indptr};
+__global__ void k_fix_entries(PivotInput in, CutVec cuts, const uint4* __restrict__ piv, uint32_t* __restrict__ crow,
+                              uint2* __restrict__ rec) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (uint64_t q = t0; 32 * q < in.m; q += stride) {
-    const uint32_t v = in.keys[32 * q];
-    uint32_t k = in.pos[v];
-    if (is(v) && 32 * q >= piv[2 * (uint64_t)k].y) k++;  // past the entries that it keeps
-    crow[q] = k;
-    // batches with four pivots or more among this one and the next three
-    const uint64_t ahead = 32 * q + 128;
-    if (ahead < in.m && in.pos[in.keys[ahead]] - in.pos[v] >= kSparsePivots)
-      atomicMax(&flags[kFlagSparse], (uint32_t)(q + 4));
+    const uint32_t k = crow[q];
+    if (32 * q >= piv[2 * (uint64_t)k].y) crow[q] = k + 1;  // past the entries that it keeps
   }
-  if (plain) return;
   for (uint64_t q = t0; q < in.m; q += stride) {
     const uint32_t v = in.keys[q];
     rec[q].x = record_start(in, v, cuts.c[part_of(cuts.c, cuts.P, v)], rec[q].x);
@@ -809,6 +1055,38 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
     if (!ev) BBTC_CUDA(cudaEventCreate(&ev));
   BBTC_CUDA(cudaEventRecord(ctx->ev_layout[0], s));
 
+  const uint64_t mm = std::max<uint64_t>(m, 1);
+  const uint64_t npiv_max = std::min<uint64_t>(n, m);
+  g->nentry_rows = mm / 32 + 1;
+  {
+    cudaError_t e1 = dev_malloc(&g->d_words, mm * sizeof(uint2), s);
+    cudaError_t e2 = dev_malloc(&g->d_rec, mm * sizeof(uint2), s);
+    cudaError_t e3 = dev_malloc(&g->d_piv, (npiv_max + 1) * 2 * sizeof(uint4), s);
+    cudaError_t e4 = dev_malloc(&g->d_crow, g->nentry_rows * sizeof(uint32_t), s);
+    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
+      cudaGetLastError();
+      return fail(BBTC_ERR_NOMEM, "device allocation of the word-compressed rows and pivot lists failed");
+    }
+  }
+  // The flags, the row heads and the tiles' words start at zero; the flags are
+  // read back once, at the end: every pass between stays inside its arrays
+  // whatever the input, or returns at once when the contract flag is set.
+  // Allocated and cleared before the upload is queued, which the upload then
+  // hides.
+  const bool large_pairs = m >= kLargePairs, large_pivots = m >= kLargePivots;
+  const uint64_t pair_tiles = (mm + tile_size(large_pairs) - 1) / tile_size(large_pairs);
+  const uint64_t pivot_tiles = (mm + tile_size(large_pivots) - 1) / tile_size(large_pivots);
+  const uint64_t hw = (mm / 32 + 4) & ~3ull;
+  const uint64_t zero_words = kFlagWords + hw + 2 * (2 * pair_tiles + pivot_tiles);
+  DevBuf zeroed;
+  BBTC_TRY(dalloc(zeroed, zero_words * sizeof(uint32_t), s));
+  uint32_t* flags = zeroed.as<uint32_t>();
+  uint32_t* heads = flags + kFlagWords;
+  uint64_t* sums = reinterpret_cast<uint64_t*>(heads + hw);
+  {
+    ZeroRanges z{{flags, nullptr, nullptr, nullptr}, {zero_words, 0, 0, 0}};
+    BBTC_TRY(launch_layout(ctx, k_zero_ranges, (int)std::min<uint64_t>((uint64_t)grid, zero_words / 1024 + 1), 256, s, z));
+  }
   // the graph keeps its own copy of the oriented CSR
   {
     cudaError_t e1 = dev_malloc(&g->d_indptr, ((size_t)n + 1) * sizeof(uint32_t), s);
@@ -877,78 +1155,45 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
   const uint32_t* d_indptr = g->d_indptr;
   const uint32_t* d_indices = g->d_indices;
 
-  const uint64_t mm = std::max<uint64_t>(m, 1);
-  const uint64_t nheads = mm / 32 + 1;
-  const uint64_t npiv_max = std::min<uint64_t>(n, m);
-  g->nentry_rows = mm / 32 + 1;
-  {
-    cudaError_t e1 = dev_malloc(&g->d_words, mm * sizeof(uint2), s);
-    cudaError_t e2 = dev_malloc(&g->d_rec, mm * sizeof(uint2), s);
-    cudaError_t e3 = dev_malloc(&g->d_piv, (npiv_max + 1) * 2 * sizeof(uint4), s);
-    cudaError_t e4 = dev_malloc(&g->d_crow, g->nentry_rows * sizeof(uint32_t), s);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
-      cudaGetLastError();
-      return fail(BBTC_ERR_NOMEM, "device allocation of the word-compressed rows and pivot lists failed");
-    }
-  }
-  // flags, row heads and the vertices' entry bounds start at zero; the flags
-  // are read back once, at the end: every pass between stays inside its arrays
-  // whatever the input, or returns at once when the contract flag is set
-  DevBuf zeroed, wpos, rec_in, keys, pos;
-  const uint64_t nv = ((uint64_t)n + 4) & ~3ull, hw = (nheads + 3) & ~3ull;
-  BBTC_TRY(dalloc(zeroed, (kFlagWords + hw + 2 * nv) * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(wpos, mm * sizeof(uint32_t), s));
+  DevBuf rec_in, keys, head_pair;
   BBTC_TRY(dalloc(rec_in, mm * sizeof(uint2), s));
   BBTC_TRY(dalloc(keys, mm * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(pos, nv * sizeof(uint32_t), s));
-  uint32_t* flags = zeroed.as<uint32_t>();
-  uint32_t* heads = flags + kFlagWords;
-  uint32_t* first = heads + hw;
-  uint32_t* end = first + nv;
-  {
-    ZeroRanges z{{flags, nullptr, nullptr, nullptr}, {kFlagWords + hw + 2 * nv, 0, 0, 0}};
-    BBTC_TRY(launch_layout(ctx, k_zero_ranges, grid, 256, s, z));
-  }
+  BBTC_TRY(dalloc(head_pair, mm * sizeof(uint32_t), s));
   if (n > 0) {
     BBTC_TRY(launch_layout(ctx, k_row_heads, grid, 256, s, d_indptr, d_indices, n, m, heads, flags));
   } else if (m > 0) {
     BBTC_CUDA(cudaMemsetAsync(flags, 0xff, sizeof(uint32_t), s));  // edges without rows
   }
+  const PivotInput in{d_indptr,           d_indices, head_pair.as<uint32_t>(), keys.as<uint32_t>(),
+                      static_cast<uint2*>(g->d_words), n, m};
+  uint2* rec = static_cast<uint2*>(g->d_rec);
   if (n > 0 && m > 0) {
-    uint2* words = static_cast<uint2*>(g->d_words);
-    uint2* rec = static_cast<uint2*>(g->d_rec);
-    uint4* piv = static_cast<uint4*>(g->d_piv);
-    const auto opens = thrust::make_transform_iterator(thrust::counting_iterator<uint64_t>(0), OpensPair{d_indices, heads});
-    const auto is_pivot = thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0),
-                                                          IsPivot{first, end, d_indptr});
-    size_t b1 = 0, b2 = 0, b3 = 0;
-    BBTC_CUDA(cub::DeviceScan::InclusiveSum(nullptr, b1, opens, wpos.as<uint32_t>(), (int64_t)m, s));
-    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b2, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
-                                              (int64_t)m, 0, key_bits(n), s));
-    BBTC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b3, is_pivot, pos.as<uint32_t>(), (int64_t)n, s));
-    DevBuf tmp;
-    BBTC_TRY(dalloc(tmp, std::max(b1, std::max(b2, b3)), s));
-    BBTC_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, b1, opens, wpos.as<uint32_t>(), (int64_t)m, s));
-    BBTC_TRY(launch_layout(ctx, k_pairs, grid, 256, s, d_indices, heads, wpos.as<uint32_t>(), n, m, words,
-                           rec_in.as<uint2>(), flags));
+    auto tile_grid = [&](uint64_t tiles) { return (int)std::min<uint64_t>(tiles, (uint64_t)grid); };
+    BBTC_TRY(launch_layout(ctx,
+                           large_pairs ? k_pairs<kLargeWarps, kLargeChunks, 3> : k_pairs<kSmallWarps, kSmallChunks, 4>,
+                           tile_grid(pair_tiles), 32 * (large_pairs ? kLargeWarps : kSmallWarps), s, d_indices, heads, n,
+                           m, static_cast<uint2*>(g->d_words), rec_in.as<uint2>(), head_pair.as<uint32_t>(), sums,
+                           sums + pair_tiles, flags));
     // a stable sort of the records by column keeps every in-list in source order
-    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, b2, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
+    size_t tb = 0;
+    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
                                               (int64_t)m, 0, key_bits(n), s));
-    BBTC_TRY(launch_layout(ctx, k_key_bounds, grid, 256, s, keys.as<uint32_t>(), m, n, first, end));
-    BBTC_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, b3, is_pivot, pos.as<uint32_t>(), (int64_t)n, s));
-    CutVec cuts{};
-    std::copy(g->cuts.begin(), g->cuts.end(), cuts.c);
-    cuts.P = g->P;
-    const PivotInput in{d_indptr, d_indices, wpos.as<uint32_t>(), keys.as<uint32_t>(), first, end, pos.as<uint32_t>(),
-                        words, n, m};
-    BBTC_TRY(launch_layout(ctx, k_pivots, grid, 256, s, in, cuts, rec, piv, flags));
-    BBTC_TRY(launch_layout(ctx, k_entry_index, grid, 256, s, in, cuts, piv, g->d_crow, rec, flags));
+    DevBuf tmp;
+    BBTC_TRY(dalloc(tmp, tb, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
+                                              (int64_t)m, 0, key_bits(n), s));
+    BBTC_TRY(launch_layout(
+        ctx, large_pivots ? k_pivots<kLargeWarps, kLargeChunks, 3> : k_pivots<kSmallWarps, kSmallChunks, 4>,
+        tile_grid(pivot_tiles), 32 * (large_pivots ? kLargeWarps : kSmallWarps), s, in, static_cast<uint32_t*>(g->d_piv),
+        g->d_crow, sums + 2 * pair_tiles, flags));
   }
   uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageFlags);
   BBTC_CUDA(cudaMemcpyAsync(h, flags, kFlagWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   BBTC_CUDA(cudaEventRecord(ctx->ev_layout[1], s));
   BBTC_CUDA(cudaStreamSynchronize(s));
   const uint32_t bad = h[kFlagBad];
+  if (bad != 0xffffffffu && (bad & kBadWait))
+    return fail(BBTC_ERR_TIMEOUT, "a layout pass waited too long for an earlier tile");
   if (bad) {
     std::string why;
     if (bad == 0xffffffffu) why += " edges but no rows;";
@@ -965,6 +1210,16 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
   g->npiv = h[kFlagPivots];
   g->nwords = h[kFlagPairs];
   g->sparse_end = h[kFlagSparse];
+  if (!g->oriented && m > 0) {
+    CutVec cuts{};
+    std::copy(g->cuts.begin(), g->cuts.end(), cuts.c);
+    cuts.P = g->P;
+    uint4* piv = static_cast<uint4*>(g->d_piv);
+    BBTC_TRY(launch_layout(ctx, k_fix_pivots, grid, 256, s, in, cuts, rec, g->npiv, piv));
+    BBTC_TRY(launch_layout(ctx, k_fix_entries, grid, 256, s, in, cuts, piv, g->d_crow, rec));
+    BBTC_CUDA(cudaEventRecord(ctx->ev_layout[1], s));
+    BBTC_CUDA(cudaStreamSynchronize(s));
+  }
   float ms = 0;
   BBTC_CUDA(cudaEventElapsedTime(&ms, ctx->ev_layout[0], ctx->ev_layout[1]));
   g->layout_ms = ms;
@@ -1074,11 +1329,15 @@ int bbtc_graph_validate(const bbtc_graph* g) {
   std::vector<uint32_t> indptr, indices, pairs, rec, piv, crow;
   BBTC_TRY(get(indptr, g->d_indptr, (uint64_t)n + 1));
   BBTC_TRY(get(indices, g->d_indices, mm));
-  BBTC_TRY(get(pairs, g->d_words, 2 * g->nwords));
+  const uint32_t at = (uint32_t)(m - g->nwords);  // pairs sit at their array's end
+  BBTC_TRY(get(pairs, static_cast<const uint2*>(g->d_words) + at, 2 * g->nwords));
   BBTC_TRY(get(rec, g->d_rec, 2 * m));
   BBTC_TRY(get(piv, g->d_piv, m ? 8 * ((uint64_t)g->npiv + 1) : 0));
   BBTC_TRY(get(crow, g->d_crow, (m + 31) / 32));
   BBTC_CUDA(cudaStreamSynchronize(s));
+  for (uint32_t& p : rec) p -= at;
+  for (uint32_t k = 0; m && k < g->npiv; k++)
+    if (piv[8 * (uint64_t)k + 3]) piv[8 * (uint64_t)k + 2] -= at;
   check::Csr c{n, m, indptr.data(), indices.data()};
   std::string why = check::csr(c);
   std::vector<uint32_t> wptr((size_t)n + 1, 0), tp, tc;
