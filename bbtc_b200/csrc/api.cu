@@ -168,15 +168,18 @@ int bbtc_ctx_create(int device, bbtc_ctx** out) {
   }
   if (device < 0 || device >= count) return fail(BBTC_ERR_NODEV, "device index out of range");
   BBTC_CUDA(cudaSetDevice(device));
-  cudaDeviceProp prop;
-  BBTC_CUDA(cudaGetDeviceProperties(&prop, device));
-  if (prop.major < 10)
-    return fail(BBTC_ERR_NODEV, std::string("device ") + prop.name + " is not sm_100-class; this build targets sm_100a");
+  // single attributes: cudaGetDeviceProperties fills them all, which takes milliseconds
+  int major = 0, sms = 0, smem_optin = 0;
+  BBTC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  BBTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  BBTC_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  if (major < 10)
+    return fail(BBTC_ERR_NODEV, "device " + std::to_string(device) + " is not sm_100-class; this build targets sm_100a");
   bbtc_ctx* c = new (std::nothrow) bbtc_ctx();
   if (!c) return fail(BBTC_ERR_NOMEM, "host allocation failed");
   c->device = device;
-  c->sms = prop.multiProcessorCount;
-  c->smem_optin = prop.sharedMemPerBlockOptin;
+  c->sms = sms;
+  c->smem_optin = (size_t)smem_optin;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete c;
