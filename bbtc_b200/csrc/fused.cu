@@ -10,14 +10,15 @@
 // shared memory and streams those pairs against it.
 //
 // What bounds it: instruction issue and the L1 / shared-memory pipe (R-MAT s20:
-// issue 66 %, that pipe 72 %, DRAM 10 %): every streamed pair is one 8-byte
+// issue 65 %, that pipe 64 %, DRAM 10 %): every streamed pair is one 8-byte
 // global load and one random shared-memory read.  So the work around the pairs
 // is what the design keeps small:
 //   * no tiles: a pivot's in-edges lie together whatever the cut vector, and
 //     only vertices that are pivots are listed, so no warp walks empty row
 //     pointers (that had left the SMs idle for 30 % of the s20 count);
 //   * lanes own rows (32, or 8 side by side when rows are short), so no lane
-//     searches the row that its pair belongs to;
+//     searches the row that its pair belongs to; the batch's rows are read from
+//     shared memory, one 8-byte broadcast a row (shuffles took two);
 //   * in-lists of a few entries share one hash table per run, so 32 entries
 //     cost two rounds of loads and not two per pivot;
 //   * units of up to eight batches of 32 entries where in-lists are long (the
@@ -26,8 +27,8 @@
 //   * the state between the probe loops lives in shared memory: the loops fit
 //     48 registers (5 blocks of 8 warps on an SM) without spilling.
 // Per count, against the tiled task rows that this replaced (B200, ms): R-MAT
-// s22 7.09 -> 5.6, s20 1.86 -> 0.91, s16 0.160 -> 0.100, s12 0.095 -> 0.037,
-// Chung-Lu 2^23 17.5 -> 4.8, geometric 2^18 0.432 -> 0.17 (readback included).
+// s22 7.09 -> 5.0, s20 1.86 -> 0.86, s16 0.160 -> 0.098, s12 0.095 -> 0.036,
+// Chung-Lu 2^23 17.5 -> 4.7, geometric 2^18 0.432 -> 0.156 (readback included).
 #include <algorithm>
 #include <cstring>
 
@@ -67,6 +68,7 @@ struct Frame {
   uint32_t far;  // hash: longest displacement of an entry
   uint32_t npiv, plain;
   uint32_t pad[2];
+  uint2 entry[32];  // the batch's entries: first pair and number of pairs of each one's row
 };
 constexpr uint32_t kFrameWords = sizeof(Frame) / 4;
 
@@ -122,56 +124,71 @@ __device__ __forceinline__ uint32_t hits_of(const uint32_t* bm, const View& pv, 
   }
 }
 
-// Rows of the batch's entries [a, b) (lane l holds entry l's start and
-// length; 0 outside [a, b)), G lanes to a row, two rows and two steps of each
-// in flight.
-template <uint32_t KIND, uint32_t G>
-__device__ __forceinline__ uint32_t probe_rows(uint32_t at, uint32_t start, uint32_t len, uint32_t a, uint32_t b) {
+// Rows of the batch's entries [a, b), G lanes to a row, R rows of each lane
+// group and two steps of each in flight.  R is 4 where the loads in flight
+// decide (LONG: graphs of long in-lists, bitmap and rank pivots), else 2: the
+// registers that 4 rows take are missing in the runs of short in-lists.
+template <uint32_t KIND, bool LONG, uint32_t G>
+__device__ __forceinline__ uint32_t probe_rows(uint32_t at, uint32_t a, uint32_t b) {
   constexpr uint32_t E = 32 / G;  // rows side by side
+  constexpr uint32_t R = LONG && (KIND == kBitmap || KIND == kRank) ? 4 : 2, S = 2;
   const uint32_t lane = threadIdx.x & 31;
   const Frame* fr = frame(at);
   const uint32_t* bm = buffer(at);
   const uint2* __restrict__ words = fr->words;
   const View pv{fr->fw, fr->span, fr->cap, fr->far};
   uint32_t hits = 0;
-  for (uint32_t r = a + lane / G; r < b + lane / G; r += 2 * E) {
-    // rows past b have length 0 (an index past 31 wraps to an entry before a)
-    const uint32_t s0 = __shfl_sync(FULL, start, r), s1 = __shfl_sync(FULL, start, r + E);
-    const uint32_t l0 = __shfl_sync(FULL, len, r), l1 = __shfl_sync(FULL, len, r + E);
-    const uint32_t lm = max(l0, l1);
-    for (uint32_t i = lane & (G - 1); i < lm; i += 2 * G) {
-      uint2 x0 = make_uint2(0, 0), x1 = x0, x2 = x0, x3 = x0;
-      if (i < l0) x0 = __ldg(words + s0 + i);
-      if (i < l1) x1 = __ldg(words + s1 + i);
-      if (i + G < l0) x2 = __ldg(words + s0 + G + i);
-      if (i + G < l1) x3 = __ldg(words + s1 + G + i);
-      hits += hits_of<KIND>(bm, pv, fr, x0);
-      hits += hits_of<KIND>(bm, pv, fr, x1);
-      if (i + G < lm) {
-        hits += hits_of<KIND>(bm, pv, fr, x2);
-        hits += hits_of<KIND>(bm, pv, fr, x3);
-      }
+  for (uint32_t r = a + lane / G; r < b; r += R * E) {
+    uint2 e[R];
+    uint32_t lm = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < R; q++) {
+      e[q] = make_uint2(0, 0);
+      if (q == 0 || r + q * E < b) e[q] = fr->entry[r + q * E];
+      lm = max(lm, e[q].y);
+    }
+    for (uint32_t i = lane & (G - 1); i < lm; i += S * G) {
+      uint2 x[R][S];
+#pragma unroll
+      for (uint32_t s = 0; s < S; s++)
+#pragma unroll
+        for (uint32_t q = 0; q < R; q++) {
+          x[q][s] = make_uint2(0, 0);
+          if (i + s * G < e[q].y) x[q][s] = __ldg(words + e[q].x + s * G + i);
+        }
+#pragma unroll
+      for (uint32_t q = 0; q < R; q++) hits += hits_of<KIND>(bm, pv, fr, x[q][0]);
+#pragma unroll
+      for (uint32_t s = 1; s < S; s++)
+        if (i + s * G < lm) {
+#pragma unroll
+          for (uint32_t q = 0; q < R; q++) hits += hits_of<KIND>(bm, pv, fr, x[q][s]);
+        }
     }
   }
   return hits;
 }
 
-template <uint32_t KIND>
-__device__ __noinline__ uint32_t probe(uint32_t at, uint32_t start, uint32_t len, uint32_t a, uint32_t b) {
+// Pairs per row from which a row gets all 32 lanes (28, 36, 40 and 44 measure
+// within 1 %, 20 and 14 are 2 and 4 % slower at R-MAT s20).
+constexpr uint32_t kWholeWarp = 40;
+
+template <uint32_t KIND, bool LONG>
+__device__ __noinline__ uint32_t probe(uint32_t at, uint32_t a, uint32_t b) {
   const uint32_t lane = threadIdx.x & 31;
-  if (lane < a || lane >= b) len = 0;
-  const uint32_t total = __reduce_add_sync(FULL, len);
+  const uint32_t total = __reduce_add_sync(FULL, lane >= a && lane < b ? frame(at)->entry[lane].y : 0u);
   if (total == 0) return 0;
-  if (total >= 20 * (b - a)) return probe_rows<KIND, 32>(at, start, len, a, b);
-  return probe_rows<KIND, 8>(at, start, len, a, b);
+  if (total >= kWholeWarp * (b - a)) return probe_rows<KIND, LONG, 32>(at, a, b);
+  return probe_rows<KIND, LONG, 8>(at, a, b);
 }
 
-__device__ __forceinline__ uint32_t probe_kind(uint32_t at, uint32_t start, uint32_t len, uint32_t a, uint32_t b) {
+template <bool LONG>
+__device__ __forceinline__ uint32_t probe_kind(uint32_t at, uint32_t a, uint32_t b) {
   switch (frame(at)->kind) {
-    case kBitmap: return probe<kBitmap>(at, start, len, a, b);
-    case kRank: return probe<kRank>(at, start, len, a, b);
-    case kHash: return probe<kHash>(at, start, len, a, b);
-    default: return probe<kSearch>(at, start, len, a, b);
+    case kBitmap: return probe<kBitmap, LONG>(at, a, b);
+    case kRank: return probe<kRank, LONG>(at, a, b);
+    case kHash: return probe<kHash, LONG>(at, a, b);
+    default: return probe<kSearch, LONG>(at, a, b);
   }
 }
 
@@ -196,18 +213,21 @@ __device__ __forceinline__ uint32_t run_hits(const uint2* tab, uint32_t shift, u
 }
 
 template <uint32_t G>
-__device__ __forceinline__ uint32_t run_rows(const uint2* __restrict__ words, const uint2* tab, uint32_t shift,
-                                             uint32_t far, uint32_t start, uint32_t len, uint32_t pl, uint32_t a,
-                                             uint32_t b) {
+__device__ __forceinline__ uint32_t run_rows(const Frame* fr, const uint2* tab, uint32_t shift, uint32_t far,
+                                             uint32_t pl, uint32_t a, uint32_t b) {
+  const uint2* __restrict__ words = fr->words;
   constexpr uint32_t E = 32 / G;
   const uint32_t lane = threadIdx.x & 31;
   uint32_t hits = 0;
   for (uint32_t r = a + lane / G; r < b + lane / G; r += 2 * E) {
     const uint32_t sub = lane & (G - 1);
-    const uint2* __restrict__ p0 = words + (__shfl_sync(FULL, start, r) + sub);
-    const uint2* __restrict__ p1 = words + (__shfl_sync(FULL, start, r + E) + sub);
-    int32_t c0 = (int32_t)(__shfl_sync(FULL, len, r) - sub), c1 = (int32_t)(__shfl_sync(FULL, len, r + E) - sub);
     const uint32_t q0 = __shfl_sync(FULL, pl, r), q1 = __shfl_sync(FULL, pl, r + E);
+    uint2 e0 = make_uint2(0, 0), e1 = e0;
+    if (r < b) e0 = fr->entry[r];
+    if (r + E < b) e1 = fr->entry[r + E];
+    const uint2* __restrict__ p0 = words + (e0.x + sub);
+    const uint2* __restrict__ p1 = words + (e1.x + sub);
+    int32_t c0 = (int32_t)(e0.y - sub), c1 = (int32_t)(e1.y - sub);
     while (max(c0, c1) > 0) {
       uint2 x0, x1;
       if (c0 > 0) x0 = __ldg(p0);
@@ -223,8 +243,8 @@ __device__ __forceinline__ uint32_t run_rows(const uint2* __restrict__ words, co
   return hits;
 }
 
-__device__ __noinline__ uint32_t run(uint32_t at, uint32_t start, uint32_t len, uint32_t pl, uint32_t ws,
-                                     uint32_t excl, uint32_t total, uint32_t j, uint32_t j2, uint32_t a, uint32_t b) {
+__device__ __noinline__ uint32_t run(uint32_t at, uint32_t pl, uint32_t ws, uint32_t excl, uint32_t total, uint32_t j,
+                                     uint32_t j2, uint32_t a, uint32_t b) {
   const uint32_t lane = threadIdx.x & 31;
   const uint2* __restrict__ words = frame(at)->words;
   const uint32_t shift = __clz(max(64u, kRunSlots * total) - 1);  // slots: a power of two, at least kRunSlots a pair
@@ -254,11 +274,11 @@ __device__ __noinline__ uint32_t run(uint32_t at, uint32_t start, uint32_t len, 
   }
   far = __reduce_max_sync(FULL, far);
   __syncwarp();
-  if (lane < a || lane >= b) len = 0;
-  const uint32_t sum = __reduce_add_sync(FULL, len);
+  const Frame* fr = frame(at);
+  const uint32_t sum = __reduce_add_sync(FULL, lane >= a && lane < b ? fr->entry[lane].y : 0u);
   uint32_t hits;
-  if (sum >= 20 * (b - a)) hits = run_rows<32>(words, tab, shift, far, start, len, pl, a, b);
-  else hits = run_rows<8>(words, tab, shift, far, start, len, pl, a, b);
+  if (sum >= kWholeWarp * (b - a)) hits = run_rows<32>(fr, tab, shift, far, pl, a, b);
+  else hits = run_rows<8>(fr, tab, shift, far, pl, a, b);
   __syncwarp();
   uint4* q = reinterpret_cast<uint4*>(tab);
   for (uint32_t i = lane; 2 * i <= cap; i += 32) q[i] = make_uint4(0, 0, 0, 0);
@@ -350,9 +370,9 @@ __device__ __forceinline__ void load_pivot(uint32_t at, uint32_t k, uint32_t lan
 
 // A batch [base, be) that is not wholly the built pivot's: its pivots, one a
 // lane; one that goes on past the batch stays built (it is the batch's last).
-// Returns this lane's hits; lane l holds entry l's pairs.
-__device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t start, uint32_t len, uint32_t base,
-                                       uint32_t be) {
+// Returns this lane's hits.
+template <bool LONG>
+__device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t base, uint32_t be) {
   const uint32_t lane = threadIdx.x & 31;
   Frame* fr = frame(at);
   const uint32_t room = (1u << (31 - __clz(bm_words))) / (2 * kRunSlots);  // pairs of a run
@@ -380,7 +400,7 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
           load_pivot(at, k + j, lane);
           build(at, bm_words);
         }
-        if ((int32_t)(bj - aj) > 0) hits += probe_kind(at, start, len, aj, bj);
+        if ((int32_t)(bj - aj) > 0) hits += probe_kind<LONG>(at, aj, bj);
         more = fr->p1 > be;
         if (!more) clear(at);
         j++;
@@ -391,10 +411,13 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
         const uint32_t j2 = stop ? (uint32_t)__ffs(stop) - 1 : np;
         const uint32_t starts = __reduce_or_sync(FULL, lane >= j && lane < j2 ? 1u << a : 0u);
         const uint32_t pl = j + __popc(starts & (FULL >> (31 - lane))) - 1;  // this entry's pivot
-        const uint32_t lend = __shfl_sync(FULL, b, pl);
-        hits += run(at, start, lane < lend ? len : 0u, pl, d.z, cum - d.w - before,
-                    __shfl_sync(FULL, cum, j2 - 1) - before, j, j2, __shfl_sync(FULL, a, j),
-                    __shfl_sync(FULL, b, j2 - 1));
+        // entries between the run's pivots belong to vertices without a row
+        const uint32_t own_end = __shfl_sync(FULL, b, pl), run_start = __shfl_sync(FULL, a, j),
+                       run_end = __shfl_sync(FULL, b, j2 - 1);
+        if (lane >= own_end && lane > run_start && lane < run_end) fr->entry[lane].y = 0;
+        __syncwarp();
+        const uint32_t total = __shfl_sync(FULL, cum, j2 - 1) - before;
+        hits += run(at, pl, d.z, cum - d.w - before, total, j, j2, run_start, run_end);
         j = j2;
       }
     }
@@ -407,7 +430,7 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
   return hits;
 }
 
-template <int MINB>
+template <int MINB, bool LONG>
 __global__ void __launch_bounds__(256, MINB)
     k_count_pivots(const __grid_constant__ PivotGraph one, const PivotGraph* __restrict__ many,
                    const uint32_t* __restrict__ prefix, uint32_t ng, uint32_t total_units,
@@ -461,18 +484,17 @@ __global__ void __launch_bounds__(256, MINB)
     while (true) {
       const uint32_t e1 = fr->e1;
       const uint32_t be = e1 - base > 32 ? base + 32 : e1;
-      uint32_t start = 0, len = 0;
-      if (base + lane < be) {
-        const uint2 r = __ldg(fr->rec + base + lane);
-        start = r.x;
-        len = r.y - r.x;
-      }
+      uint2 r = make_uint2(0, 0);
+      if (base + lane < be) r = __ldg(fr->rec + base + lane);
+      fr->entry[lane] = make_uint2(r.x, r.y - r.x);
+      __syncwarp();
       if (fr->kind != kNone && fr->p1 > be)
-        acc += probe_kind(at, start, len, 0, be - base);
+        acc += probe_kind<LONG>(at, 0, be - base);
       else
-        acc += mixed(at, bm_words, start, len, base, be);
+        acc += mixed<LONG>(at, bm_words, base, be);
       if (be == e1) break;
       base = be;
+      __syncwarp();
     }
     if (fr->kind != kNone) clear(at);
     const uint32_t slot = fr->slot;
@@ -489,8 +511,11 @@ __global__ void __launch_bounds__(256, MINB)
 using Kernel = void (*)(const PivotGraph, const PivotGraph*, const uint32_t*, uint32_t, uint32_t, unsigned long long*,
                         uint32_t, uint32_t);
 
-Kernel kernel_for(uint32_t occ) {
-  return occ >= 8 ? k_count_pivots<8> : (occ >= 6 ? k_count_pivots<6> : (occ == 5 ? k_count_pivots<5> : k_count_pivots<4>));
+Kernel kernel_for(uint32_t occ, bool long_lists) {
+  if (occ >= 8) return k_count_pivots<8, false>;
+  if (occ >= 6) return k_count_pivots<6, false>;
+  if (occ == 5) return long_lists ? k_count_pivots<5, true> : k_count_pivots<5, false>;
+  return k_count_pivots<4, false>;
 }
 
 }  // namespace
@@ -500,16 +525,17 @@ size_t pivots_smem(uint32_t bm_words, uint32_t warps) {
 }
 
 int pivots_smem_optin(size_t bytes) {
-  for (Kernel k : {k_count_pivots<4>, k_count_pivots<5>, k_count_pivots<6>, k_count_pivots<8>})
+  for (Kernel k : {k_count_pivots<4, false>, k_count_pivots<5, false>, k_count_pivots<5, true>, k_count_pivots<6, false>,
+                   k_count_pivots<8, false>})
     BBTC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return BBTC_OK;
 }
 
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
-                  uint32_t total_units, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts) {
+                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts) {
   const uint32_t bmw = norm_bm_words(o.bitmap_words), wpb = norm_warps(o.warps_per_block);
   const size_t sm = pivots_smem(bmw, wpb);
-  const Kernel kern = kernel_for(o.occupancy);
+  const Kernel kern = kernel_for(o.occupancy, long_lists);
   int per_sm = 0;
   BBTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * 32, sm));
   per_sm = std::max(1, per_sm);

@@ -147,6 +147,7 @@ struct Plan {
   uint32_t total_units = 0;
   uint32_t launches = 0;
   bool fused = false;              // pivot lists (fused.cu)
+  bool long_lists = false;         // with many in-edges per pivot
   cudaGraphExec_t exec = nullptr;
   bool captured = false;
   uint32_t stage_polls = 0;        // the context's staging test hook when the launch was captured
@@ -308,6 +309,6 @@ inline uint32_t norm_warps(uint32_t w) { return w == 0 || w > 8 ? 8 : w; }
 size_t pivots_smem(uint32_t bm_words, uint32_t warps);
 int pivots_smem_optin(size_t bytes);
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
-                  uint32_t total_units, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts);
+                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts);
 
 }  // namespace bbtc
