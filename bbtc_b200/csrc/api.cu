@@ -98,7 +98,7 @@ int finish_upload(bbtc_ctx* ctx, uint32_t n, const uint32_t* indptr, const uint3
   g->m = m;
   g->P = P;
   g->cuts.assign(cuts, cuts + P + 1);
-  if (dev_malloc(&g->d_count, 64 * sizeof(uint64_t), ctx->stream) != cudaSuccess) {
+  if (dev_malloc(&g->d_count, kCountWords * sizeof(uint64_t), ctx->stream) != cudaSuccess) {
     cudaGetLastError();
     delete g;
     return fail(BBTC_ERR_NOMEM, "device allocation of the result slot failed");
@@ -407,13 +407,15 @@ static int count_async_impl(bbtc_ctx* ctx, bbtc_graph* g, const bbtc_task* tasks
     }
     it = g->plans.emplace(key, std::make_unique<Plan>()).first;
   }
-  const int rc = count_enqueue(ctx, gs, tl, o, fused, g->d_count, it->second.get(), reuse);
+  const Delivery to{g->d_count + 2, g->d_count, reinterpret_cast<uint64_t*>(ctx->h_stage + kStageCount)};
+  const int rc = count_enqueue(ctx, gs, tl, o, fused, g->d_count, it->second.get(), reuse, &to);
   if (rc != BBTC_OK) {
     it->second->release();
     g->plans.erase(it);
     return rc;
   }
   g->last_launches = it->second->launches;
+  g->delivered = it->second->delivers ? ++ctx->delivered : 0;
   return BBTC_OK;
 }
 
@@ -426,8 +428,10 @@ int bbtc_count_wait(bbtc_ctx* ctx, bbtc_graph* g, uint64_t* out) {
   Range range("bbtc count wait");
   if (!ctx || !g || !out) return fail(BBTC_ERR_ARG, "NULL argument");
   BBTC_CUDA(cudaSetDevice(ctx->device));
-  uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut);
-  BBTC_CUDA(cudaMemcpyAsync(h, g->d_count, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  // the context's last delivered count is in its staging already; an earlier one, or one of a plain launch, is copied
+  const bool here = g->delivered && g->ctx == ctx && g->delivered == ctx->delivered;
+  uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + (here ? kStageCount : kStageOut));
+  if (!here) BBTC_CUDA(cudaMemcpyAsync(h, g->d_count, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
   BBTC_CUDA(cudaStreamSynchronize(ctx->stream));
   BBTC_TRY(control_status(h[1]));
   *out = h[0];
@@ -535,7 +539,8 @@ int bbtc_count_batch(bbtc_ctx* ctx, bbtc_graph* const* graphs, uint32_t ng, cons
   }
   uint64_t* d_outs = nullptr;
   const size_t bytes = ((size_t)ng + 1) * sizeof(uint64_t);  // the counts and the control word
-  BBTC_CUDA(dev_malloc(&d_outs, bytes, ctx->stream));
+  const size_t acc_bytes = ((size_t)ng + kDeliverWords) * sizeof(uint64_t);
+  BBTC_CUDA(dev_malloc(&d_outs, acc_bytes, ctx->stream));
   struct F {
     uint64_t* p;
     cudaStream_t s;
@@ -543,16 +548,21 @@ int bbtc_count_batch(bbtc_ctx* ctx, bbtc_graph* const* graphs, uint32_t ng, cons
   } guard{d_outs, ctx->stream};
   Plan plan;
   o.use_cuda_graph = 0;
-  // one queue for all graphs, heaviest first
-  int rc = count_enqueue(ctx, gs, tl, o, fused, d_outs, &plan, false);
+  // one queue for all graphs, heaviest first; its counts go to the staging if they fit there
+  const bool staged = bytes <= kStageBytes - kStageOut;
+  const Delivery to{d_outs, nullptr, reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut)};
+  int rc = BBTC_OK;
+  if (staged) BBTC_CUDA(cudaMemsetAsync(d_outs, 0, acc_bytes, ctx->stream));
+  rc = count_enqueue(ctx, gs, tl, o, fused, d_outs, &plan, false, staged ? &to : nullptr);
   if (rc == BBTC_OK) {
     std::vector<uint64_t> big;
     uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOut);
-    if (bytes > kStageBytes - kStageOut) {
+    if (!staged) {
       big.resize(ng + 1);
       h = big.data();
     }
-    cudaError_t e = cudaMemcpyAsync(h, d_outs, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaSuccess;
+    if (!plan.delivers) e = cudaMemcpyAsync(h, d_outs, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "batch readback");
     else rc = control_status(h[ng]);

@@ -33,6 +33,7 @@
 #include <cstring>
 #include <sstream>
 
+#include "deliver.cuh"
 #include "internal.h"
 #include "search.cuh"
 
@@ -412,14 +413,15 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) k_count_queue(const DevTask* __restrict__ tasks,
                                                         const uint32_t* __restrict__ prefix, uint32_t ntasks,
-                                                        uint32_t total_units, uint32_t* __restrict__ head,
-                                                        unsigned long long* __restrict__ outs, uint32_t bm_words,
-                                                        uint32_t dbg) {
+                                                        uint32_t total_units, unsigned long long* __restrict__ outs,
+                                                        uint32_t nouts, uint64_t* __restrict__ dev,
+                                                        uint64_t* __restrict__ host, uint32_t bm_words, uint32_t dbg) {
   extern __shared__ __align__(16) uint32_t sh[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t* bm = sh + warp * (bm_words + kSegWords);
   uint32_t* sstart = bm + bm_words;
   uint32_t* sbase = sstart + 33;
+  uint32_t* head = reinterpret_cast<uint32_t*>(outs + nouts);
   uint32_t* err = head + 1;  // set when a staging copy gave up
   for (uint32_t i = lane; i < bm_words; i += 32) bm[i] = 0;
   staging_init(bm, bm_words, lane);
@@ -439,6 +441,7 @@ __global__ void __launch_bounds__(256, MINB) k_count_queue(const DevTask* __rest
     if (lane == 0 && c) atomicAdd(&outs[tk.slot], c);
     if (staging_dead(bm, bm_words)) break;
   }
+  if (host) deliver(outs, nouts, dev, host);
 }
 
 // Plain form: one task per launch; warps stride over the task's units.
@@ -662,31 +665,37 @@ void Plan::release() {
   cap = 0;
 }
 
-static int enqueue_launches(bbtc_ctx* ctx, Plan* plan, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts) {
+static int enqueue_launches(bbtc_ctx* ctx, Plan* plan, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts,
+                            const Delivery* to) {
   cudaStream_t s = ctx->stream;
   const uint32_t bmw = norm_bm_words(o.bitmap_words);
   const uint32_t wpb = norm_warps(o.warps_per_block);
   const size_t sm = smem_bytes(bmw, wpb);
-  auto* outs = reinterpret_cast<unsigned long long*>(d_outs);
-  // the counts and, after them, the control word: queue head, staging flag
-  BBTC_CUDA(cudaMemsetAsync(d_outs, 0, (nouts + 1) * sizeof(uint64_t), s));
-  uint32_t* ctrl = reinterpret_cast<uint32_t*>(d_outs + nouts);
   plan->launches = 0;
   const uint32_t ntasks = (uint32_t)plan->prefix.size() - 1;
+  if ((!plan->fused && o.mode == BBTC_MODE_PLAIN) || ntasks == 0) to = nullptr;
+  plan->delivers = to != nullptr;
+  // the counts and, after them, the control word: queue head, staging flag
+  if (!to) BBTC_CUDA(cudaMemsetAsync(d_outs, 0, (nouts + 1) * sizeof(uint64_t), s));
+  uint64_t* acc = to ? to->acc : d_outs;
+  uint64_t* dev = to ? to->dev : nullptr;
+  uint64_t* host = to ? to->host : nullptr;
   if (ntasks == 0) return BBTC_OK;
   const uint32_t* d_prefix = reinterpret_cast<const uint32_t*>(static_cast<const char*>(plan->d_queue) + plan->prefix_at);
   if (plan->fused) {
     BBTC_TRY(pivots_launch(ctx, plan->pivots[0], static_cast<const PivotGraph*>(plan->d_queue), d_prefix, ntasks,
-                           plan->total_units, plan->long_lists, o, d_outs, nouts));
+                           plan->total_units, plan->long_lists, o, acc, nouts, dev, host));
     plan->launches = 1;
     return BBTC_OK;
   }
   const DevTask* d_tasks = static_cast<const DevTask*>(plan->d_queue);
   if (o.mode == BBTC_MODE_PLAIN) {
+    uint32_t* err = reinterpret_cast<uint32_t*>(d_outs + nouts) + 1;
     for (uint32_t t = 0; t < ntasks; t++) {
       const uint32_t units = plan->prefix[t + 1] - plan->prefix[t];
       const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((units + wpb - 1) / wpb, ctx->sms * 8));
-      k_count_task<<<grid, wpb * 32, sm, s>>>(d_tasks + t, units, outs, bmw, ctrl + 1, ctx->debug_stage_polls);
+      k_count_task<<<grid, wpb * 32, sm, s>>>(d_tasks + t, units, reinterpret_cast<unsigned long long*>(d_outs), bmw,
+                                               err, ctx->debug_stage_polls);
       BBTC_CUDA(cudaGetLastError());
       plan->launches++;
     }
@@ -702,7 +711,8 @@ static int enqueue_launches(bbtc_ctx* ctx, Plan* plan, const bbtc_opts& o, uint6
     // leaves the rest of the GPU to other streams)
     const uint64_t want = ((uint64_t)plan->total_units + wpb - 1) / wpb;
     const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * per_sm, want));
-    qkern<<<grid, wpb * 32, sm, s>>>(d_tasks, d_prefix, ntasks, plan->total_units, ctrl, outs, bmw,
+    qkern<<<grid, wpb * 32, sm, s>>>(d_tasks, d_prefix, ntasks, plan->total_units,
+                                     reinterpret_cast<unsigned long long*>(acc), nouts, dev, host, bmw,
                                      ctx->debug_stage_polls);
     BBTC_CUDA(cudaGetLastError());
     plan->launches = 1;
@@ -731,7 +741,7 @@ static bbtc_opts resolve_opts(const bbtc_opts& in, bool fused) {
 
 int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
                   const std::vector<std::vector<bbtc_task>>& tasks, const bbtc_opts& in, bool fused,
-                  uint64_t* d_outs, Plan* plan, bool reuse) {
+                  uint64_t* d_outs, Plan* plan, bool reuse, const Delivery* to) {
   Range range("bbtc count enqueue");
   cudaStream_t s = ctx->stream;
   const bbtc_opts o = resolve_opts(in, fused);
@@ -789,11 +799,12 @@ int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
   // less host time than a graph launch), and so is any plan's first count:
   // capturing and instantiating a graph pays only on replays, so the capture
   // waits for the plan's second count.
-  if (!o.use_cuda_graph || !reuse || plan->fused || o.mode != BBTC_MODE_PLAIN) return enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size());
+  if (!o.use_cuda_graph || !reuse || plan->fused || o.mode != BBTC_MODE_PLAIN)
+    return enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size(), to);
   if (!plan->captured) {
     cudaGraph_t graph = nullptr;
     BBTC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size());
+    const int rc = enqueue_launches(ctx, plan, o, d_outs, (uint32_t)graphs.size(), nullptr);
     const cudaError_t ec = cudaStreamEndCapture(s, &graph);
     if (rc != BBTC_OK) {
       if (graph) cudaGraphDestroy(graph);

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "deliver.cuh"
 #include "internal.h"
 
 namespace bbtc {
@@ -434,7 +435,8 @@ template <int MINB, bool LONG>
 __global__ void __launch_bounds__(256, MINB)
     k_count_pivots(const __grid_constant__ PivotGraph one, const PivotGraph* __restrict__ many,
                    const uint32_t* __restrict__ prefix, uint32_t ng, uint32_t total_units,
-                   unsigned long long* __restrict__ outs, uint32_t nouts, uint32_t bm_words) {
+                   unsigned long long* __restrict__ outs, uint32_t nouts, uint64_t* __restrict__ dev,
+                   uint64_t* __restrict__ host, uint32_t bm_words) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t at = (threadIdx.x >> 5) * (bm_words + kFrameWords);
   Frame* fr = frame(at);
@@ -506,10 +508,11 @@ __global__ void __launch_bounds__(256, MINB)
     }
     __syncwarp();
   }
+  if (host) deliver(outs, nouts, dev, host);
 }
 
 using Kernel = void (*)(const PivotGraph, const PivotGraph*, const uint32_t*, uint32_t, uint32_t, unsigned long long*,
-                        uint32_t, uint32_t);
+                        uint32_t, uint64_t*, uint64_t*, uint32_t);
 
 Kernel kernel_for(uint32_t occ, bool long_lists) {
   if (occ >= 8) return k_count_pivots<8, false>;
@@ -532,7 +535,8 @@ int pivots_smem_optin(size_t bytes) {
 }
 
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
-                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts) {
+                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts,
+                  uint64_t* dev, uint64_t* host) {
   const uint32_t bmw = norm_bm_words(o.bitmap_words), wpb = norm_warps(o.warps_per_block);
   const size_t sm = pivots_smem(bmw, wpb);
   const Kernel kern = kernel_for(o.occupancy, long_lists);
@@ -545,7 +549,7 @@ int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many
   const uint64_t want = ((uint64_t)total_units + wpb - 1) / wpb;
   const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * per_sm, want));
   kern<<<grid, wpb * 32, sm, ctx->stream>>>(one, d_many, d_prefix, ng, total_units,
-                                            reinterpret_cast<unsigned long long*>(d_outs), nouts, bmw);
+                                            reinterpret_cast<unsigned long long*>(d_outs), nouts, dev, host, bmw);
   BBTC_CUDA(cudaGetLastError());
   return BBTC_OK;
 }

@@ -150,6 +150,7 @@ struct Plan {
   bool long_lists = false;         // with many in-edges per pivot
   cudaGraphExec_t exec = nullptr;
   bool captured = false;
+  bool delivers = false;           // the last launch put its counts where its Delivery says
   uint32_t stage_polls = 0;        // the context's staging test hook when the launch was captured
   void release();
 };
@@ -175,6 +176,7 @@ struct bbtc_ctx {
   // waited for a long kernel on its stream held up the copies of all other
   // threads; copies from pinned memory wait only for their own stream.
   char* h_stage = nullptr;
+  uint64_t delivered = 0;  // counts delivered to h_stage (Delivery) so far; the last one is there
   // Pinned staging of the task queues' uploads, kept across plans.
   char* h_plan = nullptr;
   size_t h_plan_cap = 0;
@@ -237,10 +239,13 @@ inline int dalloc(DevBuf& b, size_t bytes, cudaStream_t s) {
   return BBTC_OK;
 }
 
+constexpr uint32_t kCountWords = 6;  // of bbtc_graph::d_count
+
 // Regions of bbtc_ctx::h_stage (one graph build or count at a time per context).
 constexpr size_t kStageBytes = 1u << 20;
 constexpr size_t kStageCuts = 0;          // cut vector, <= (64 + 2) x 4 bytes
 constexpr size_t kStageFlags = 3072;      // contract flags and totals of a layout build; small read-backs
+constexpr size_t kStageCount = 3584;      // the last delivered count and its control word
 constexpr size_t kStageOff = 4096;        // tile + part row offsets of a block CSR (<= 33,288 bytes)
 constexpr size_t kStageStats = 81920;     // its tile statistics (<= 81,920 bytes)
 constexpr size_t kStageOut = 262144;      // counts read back (<= 98,304 of them)
@@ -264,7 +269,8 @@ struct bbtc_graph {
   uint32_t sparse_end = 0;        // 32-entry batches up to which pivots have few in-edges
   bool oriented = false;          // every id exceeds its row's
   bbtc::BlockTiles fwd, rev;      // tiles of the per-task kernels, built on first use
-  uint64_t* d_count = nullptr;  // the count and its control word
+  uint64_t* d_count = nullptr;  // kCountWords: a count and its control word; then a queue kernel's accumulators
+  uint64_t delivered = 0;       // which of the context's delivered counts the last one is, 0 = none
   uint64_t device_bytes = 0;
   double layout_ms = 0;
   bool fwd_built = false;         // the forward block CSR is built on first use (task-list counting, tile stats)
@@ -286,10 +292,23 @@ int ensure_fwd(bbtc_graph* g);
 int ensure_tiles(bbtc_graph* g);
 DevTile dev_tile(const BlockTiles& t, const std::vector<uint32_t>& cuts, uint32_t x, uint32_t y);
 
+// Where a queue kernel's last warp writes the counts (deliver.cuh): `host`
+// (page-locked) and, unless NULL, `dev`, each with the control word after the
+// counts.  `acc` is what the warps add to, kDeliverWords longer than the
+// counts; it is zero before the launch and again after it.
+constexpr uint32_t kDeliverWords = 2;
+struct Delivery {
+  uint64_t* acc = nullptr;
+  uint64_t* dev = nullptr;
+  uint64_t* host = nullptr;
+};
+
 // count.cu
+// With a Delivery, a queue of at least one unit puts its counts there instead
+// of d_outs (plan->delivers), which saves the clearing and the copy.
 int count_enqueue(bbtc_ctx* ctx, const std::vector<bbtc_graph*>& graphs,
                   const std::vector<std::vector<bbtc_task>>& tasks, const bbtc_opts& o, bool fused,
-                  uint64_t* d_outs, Plan* plan, bool reuse);
+                  uint64_t* d_outs, Plan* plan, bool reuse, const Delivery* to = nullptr);
 int kernel_smem_optin(bbtc_ctx* ctx, const bbtc_opts& o);
 // Every launch of count_enqueue leaves a control word after its counts
 // (d_outs[graphs.size()]): BBTC_ERR_TIMEOUT if a shared-memory staging copy
@@ -309,6 +328,7 @@ inline uint32_t norm_warps(uint32_t w) { return w == 0 || w > 8 ? 8 : w; }
 size_t pivots_smem(uint32_t bm_words, uint32_t warps);
 int pivots_smem_optin(size_t bytes);
 int pivots_launch(bbtc_ctx* ctx, const PivotGraph& one, const PivotGraph* d_many, const uint32_t* d_prefix, uint32_t ng,
-                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts);
+                  uint32_t total_units, bool long_lists, const bbtc_opts& o, uint64_t* d_outs, uint32_t nouts,
+                  uint64_t* dev, uint64_t* host);
 
 }  // namespace bbtc

@@ -1084,7 +1084,7 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
   uint32_t* heads = flags + kFlagWords;
   uint64_t* sums = reinterpret_cast<uint64_t*>(heads + hw);
   {
-    ZeroRanges z{{flags, nullptr, nullptr, nullptr}, {zero_words, 0, 0, 0}};
+    ZeroRanges z{{flags, reinterpret_cast<uint32_t*>(g->d_count), nullptr, nullptr}, {zero_words, 2 * kCountWords, 0, 0}};
     BBTC_TRY(launch_layout(ctx, k_zero_ranges, (int)std::min<uint64_t>((uint64_t)grid, zero_words / 1024 + 1), 256, s, z));
   }
   // the graph keeps its own copy of the oriented CSR

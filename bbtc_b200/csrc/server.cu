@@ -244,11 +244,13 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
         bbtc_task_list(gs[i]->P, tl[i].data(), nt, &nt);
       }
     }
-    if (rc == BBTC_OK) rc = count_enqueue(ctx, gs, tl, o, fused, L.d_outs, &plan, false);
+    const Delivery to{L.d_outs, nullptr, L.h_outs};  // d_outs: cleared at creation, and by each launch
+    if (rc == BBTC_OK) rc = count_enqueue(ctx, gs, tl, o, fused, L.d_outs, &plan, false, &to);
     if (rc == BBTC_OK) {
-      const cudaError_t e =
-          cudaMemcpyAsync(L.h_outs, L.d_outs, (batch.size() + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost,
-                          ctx->stream);
+      cudaError_t e = cudaSuccess;
+      if (!plan.delivers)
+        e = cudaMemcpyAsync(L.h_outs, L.d_outs, (batch.size() + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                            ctx->stream);
       const cudaError_t e2 = e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
       if (e2 != cudaSuccess) rc = cuda_fail(e2, "server batch readback");
       else rc = control_status(L.h_outs[batch.size()]);
@@ -457,7 +459,9 @@ int bbtc_server_create(int device, const bbtc_server_opts* opts, bbtc_server** o
       rc = set_partition_stream(s, s->load_ctx[i], (int)(i % 2), i % 2 == 0 ? mid : lo);
   }
   for (uint32_t l = 0; rc == BBTC_OK && l < 2; l++) {
-    if (dev_malloc_sync(&s->lanes[l].d_outs, ((size_t)s->opts.max_batch + 1) * sizeof(uint64_t)) != cudaSuccess ||
+    if (dev_malloc_sync(&s->lanes[l].d_outs, ((size_t)s->opts.max_batch + kDeliverWords) * sizeof(uint64_t)) != cudaSuccess ||
+        cudaMemset(s->lanes[l].d_outs, 0, ((size_t)s->opts.max_batch + kDeliverWords) * sizeof(uint64_t)) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess ||
         cudaMallocHost(&s->lanes[l].h_outs, ((size_t)s->opts.max_batch + 1) * sizeof(uint64_t)) != cudaSuccess) {
       cudaGetLastError();
       rc = fail(BBTC_ERR_NOMEM, "allocation of the result slots failed");

@@ -61,3 +61,32 @@ def test_entry_counts_around_a_batch(ctx, m):
     finally:
         st.free()
         two.free()
+
+
+@pytest.mark.parametrize("first,second", [({}, {}), ({}, {"kernel": "merge"}), ({"kernel": "search"}, {}),
+                                          ({"kernel": "search", "mode": "plain"}, {}),
+                                          ({"kernel": "bitmap"}, {"kernel": "merge", "mode": "plain"})])
+def test_counts_in_flight_keep_apart(ctx, first, second):
+    """Two graphs and an empty one counted before any is waited for: each wait
+    returns its graph's last count, whichever was launched last."""
+    csrs = [wide_rows(3000, 40, 20, seed=1), wide_rows(3000, 50, 30, seed=2)]
+    want = [oracle.count(g.n, g.indptr, g.indices, graphs.cuts(g, 4, "n1d")) for g in csrs] + [0]
+    assert want[0] != want[1]
+    csrs.append(graphs.OrientedCSR(7, np.zeros(8, np.uint32), np.zeros(0, np.uint32)))
+    sts = [Graph.from_csr(ctx, g, graphs.cuts(g, 4, "n1d")) for g in csrs]
+    a, b = options(**first), options(**second)
+    try:
+        for order in ((0, 1, 2), (2, 1, 0), (1, 2, 0)):
+            for i in order:
+                sts[i].count_async(opts=a)
+            for i in (0, 1, 2, 1, 0):
+                assert sts[i].count_wait() == want[i], (order, i)
+            for i in order:
+                sts[i].count_async(opts=b)
+                sts[i].count_async(opts=a)
+                sts[i].count_async(opts=b)
+            assert [st.count_wait() for st in sts] == want, order
+            assert count_batch(ctx, sts, a) == want
+    finally:
+        for st in sts:
+            st.free()
