@@ -27,8 +27,8 @@
 //   * the state between the probe loops lives in shared memory: the loops fit
 //     48 registers (5 blocks of 8 warps on an SM) without spilling.
 // Per count, against the tiled task rows that this replaced (B200, ms): R-MAT
-// s22 7.09 -> 5.0, s20 1.86 -> 0.86, s16 0.160 -> 0.098, s12 0.095 -> 0.036,
-// Chung-Lu 2^23 17.5 -> 4.7, geometric 2^18 0.432 -> 0.156 (readback included).
+// s22 7.09 -> 4.95, s20 1.86 -> 0.82, s16 0.160 -> 0.077, s12 0.095 -> 0.032,
+// Chung-Lu 2^23 17.5 -> 4.17, geometric 2^18 0.432 -> 0.115 (readback included).
 #include <algorithm>
 #include <cstring>
 
@@ -42,9 +42,12 @@ constexpr uint32_t FULL = 0xffffffffu;
 
 // Membership structures of a pivot, chosen per pivot by its span and length.
 // A pivot with this many entries in a batch of 32 gets a structure of its own;
-// consecutive shorter ones share a hash table (run).  8, 12 and 16 measure
-// alike at R-MAT s22 and 10 % apart on the smallest graphs.
-constexpr uint32_t kAlone = 8;
+// consecutive shorter ones share a hash table (run).  Where in-lists are short
+// (8 / 12 / 16 / 24, ms: Chung-Lu 2^23 4.42 / 4.30 / 4.27 / 4.27, geometric
+// 2^18 0.143 / 0.125 / 0.120 / 0.119) building costs more than probing; where
+// they are long (R-MAT s22 4.96 / 5.00 / 5.02 / 5.03) the own structure, mostly
+// a bitmap, is cheaper to probe.
+constexpr uint32_t kAlone = 16, kAloneLong = 8;
 constexpr uint32_t kRunSlots = 4;  // hash slots per pair of a run: chains stay short (2 measured 1-2 % slower)
 
 enum PivotKind : uint32_t {
@@ -213,11 +216,13 @@ __device__ __forceinline__ uint32_t run_hits(const uint2* tab, uint32_t shift, u
   return 0;
 }
 
-template <uint32_t G>
+// Always 8 lanes a row: a second path of 32 lanes cost every run 2 to 3 %
+// (Chung-Lu 2^23 4.25 -> 4.17 ms without it, geometric 2^18 0.119 -> 0.115),
+// and so do paths of 4 or 16, or 4 rows in flight.
 __device__ __forceinline__ uint32_t run_rows(const Frame* fr, const uint2* tab, uint32_t shift, uint32_t far,
                                              uint32_t pl, uint32_t a, uint32_t b) {
   const uint2* __restrict__ words = fr->words;
-  constexpr uint32_t E = 32 / G;
+  constexpr uint32_t G = 8, E = 32 / G;
   const uint32_t lane = threadIdx.x & 31;
   uint32_t hits = 0;
   for (uint32_t r = a + lane / G; r < b + lane / G; r += 2 * E) {
@@ -275,11 +280,7 @@ __device__ __noinline__ uint32_t run(uint32_t at, uint32_t pl, uint32_t ws, uint
   }
   far = __reduce_max_sync(FULL, far);
   __syncwarp();
-  const Frame* fr = frame(at);
-  const uint32_t sum = __reduce_add_sync(FULL, lane >= a && lane < b ? fr->entry[lane].y : 0u);
-  uint32_t hits;
-  if (sum >= kWholeWarp * (b - a)) hits = run_rows<32>(fr, tab, shift, far, pl, a, b);
-  else hits = run_rows<8>(fr, tab, shift, far, pl, a, b);
+  const uint32_t hits = run_rows(frame(at), tab, shift, far, pl, a, b);
   __syncwarp();
   uint4* q = reinterpret_cast<uint4*>(tab);
   for (uint32_t i = lane; 2 * i <= cap; i += 32) q[i] = make_uint4(0, 0, 0, 0);
@@ -361,6 +362,15 @@ __device__ __noinline__ void clear(uint32_t at) {
   __syncwarp();
 }
 
+// Start fetching a row of pairs [r.x, r.y) into L2: its first and its last
+// line.  Chung-Lu 2^23 4.62 -> 4.40 ms (first line only: 4.52; the rows of a
+// batch that other warps reach later: no more than its own).
+__device__ __forceinline__ void touch_row(const uint2* words, uint2 r) {
+  if (r.y <= r.x) return;
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(words + r.x));
+  if (((r.y - 1) ^ r.x) & ~15u) asm volatile("prefetch.global.L2 [%0];" ::"l"(words + (r.y - 1)));
+}
+
 // The frame's next pivot: two lanes copy its 32 bytes.
 __device__ __forceinline__ void load_pivot(uint32_t at, uint32_t k, uint32_t lane) {
   Frame* fr = frame(at);
@@ -385,7 +395,7 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
     if (k + lane < fr->npiv) d = __ldg(fr->piv + 2 * (uint64_t)(k + lane));
     np = __popc(__ballot_sync(FULL, d.x < be));
     const uint32_t a = max(d.x, base) - base, b = min(d.y, be) - base;
-    const bool alone = d.x >= be || b <= a || b - a >= kAlone || d.y > be || d.w > room || !fr->plain || lane == 31 ||
+    const bool alone = d.x >= be || b <= a || b - a >= (LONG ? kAloneLong : kAlone) || d.y > be || d.w > room || !fr->plain || lane == 31 ||
                        (lane == 0 && fr->kind != kNone);
     const uint32_t single = __ballot_sync(FULL, alone);
     uint32_t cum = alone ? 0u : d.w;
@@ -488,6 +498,7 @@ __global__ void __launch_bounds__(256, MINB)
       const uint32_t be = e1 - base > 32 ? base + 32 : e1;
       uint2 r = make_uint2(0, 0);
       if (base + lane < be) r = __ldg(fr->rec + base + lane);
+      if (!LONG) touch_row(fr->words, r);  // while the pivots are read and their table is built
       fr->entry[lane] = make_uint2(r.x, r.y - r.x);
       __syncwarp();
       if (fr->kind != kNone && fr->p1 > be)
