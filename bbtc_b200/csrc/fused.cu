@@ -24,11 +24,12 @@
 //   * units of up to eight batches of 32 entries where in-lists are long (the
 //     pivot is rebuilt per unit), of one batch where they are short or the
 //     queue ends;
-//   * the state between the probe loops lives in shared memory: the loops fit
-//     48 registers (5 blocks of 8 warps on an SM) without spilling.
+//   * the state between the probe loops lives in shared memory, and what is one
+//     call's is inlined: the loops fit 48 registers (5 blocks of 8 warps on an
+//     SM) without spilling, and few registers are saved around them.
 // Per count, against the tiled task rows that this replaced (B200, ms): R-MAT
-// s22 7.09 -> 4.95, s20 1.86 -> 0.82, s16 0.160 -> 0.077, s12 0.095 -> 0.032,
-// Chung-Lu 2^23 17.5 -> 4.17, geometric 2^18 0.432 -> 0.115 (readback included).
+// s22 7.09 -> 4.85, s20 1.86 -> 0.78, s16 0.160 -> 0.074, s12 0.095 -> 0.032,
+// Chung-Lu 2^23 17.5 -> 3.68, geometric 2^18 0.432 -> 0.105 (result included).
 #include <algorithm>
 #include <cstring>
 
@@ -178,12 +179,28 @@ __device__ __forceinline__ uint32_t probe_rows(uint32_t at, uint32_t a, uint32_t
 constexpr uint32_t kWholeWarp = 40;
 
 template <uint32_t KIND, bool LONG>
-__device__ __noinline__ uint32_t probe(uint32_t at, uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t probe_here(uint32_t at, uint32_t a, uint32_t b) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t total = __reduce_add_sync(FULL, lane >= a && lane < b ? frame(at)->entry[lane].y : 0u);
   if (total == 0) return 0;
   if (total >= kWholeWarp * (b - a)) return probe_rows<KIND, LONG, 32>(at, a, b);
   return probe_rows<KIND, LONG, 8>(at, a, b);
+}
+
+// Where in-lists are long the four loops are functions, each with the whole
+// register budget for its rows in flight; a pivot is probed over many entries
+// per call.  Where they are short a call's saved registers cost more than the
+// loops' spills (Chung-Lu 2^23: 3.97 ms as functions, 3.72 inlined; R-MAT s22:
+// 4.84 and 5.20).
+template <uint32_t KIND, bool LONG>
+__device__ __noinline__ uint32_t probe_call(uint32_t at, uint32_t a, uint32_t b) {
+  return probe_here<KIND, LONG>(at, a, b);
+}
+
+template <uint32_t KIND, bool LONG>
+__device__ __forceinline__ uint32_t probe(uint32_t at, uint32_t a, uint32_t b) {
+  if constexpr (LONG) return probe_call<KIND, LONG>(at, a, b);
+  else return probe_here<KIND, LONG>(at, a, b);
 }
 
 template <bool LONG>
@@ -249,8 +266,8 @@ __device__ __forceinline__ uint32_t run_rows(const Frame* fr, const uint2* tab, 
   return hits;
 }
 
-__device__ __noinline__ uint32_t run(uint32_t at, uint32_t pl, uint32_t ws, uint32_t excl, uint32_t total, uint32_t j,
-                                     uint32_t j2, uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t run_here(uint32_t at, uint32_t pl, uint32_t ws, uint32_t excl, uint32_t total,
+                                             uint32_t j, uint32_t j2, uint32_t a, uint32_t b) {
   const uint32_t lane = threadIdx.x & 31;
   const uint2* __restrict__ words = frame(at)->words;
   const uint32_t shift = __clz(max(64u, kRunSlots * total) - 1);  // slots: a power of two, at least kRunSlots a pair
@@ -288,11 +305,25 @@ __device__ __noinline__ uint32_t run(uint32_t at, uint32_t pl, uint32_t ws, uint
   return hits;
 }
 
+// A function or not, as probe (batch of 96: 0.294 ms as a function, 0.285
+// inlined; R-MAT s20: 0.78 and 0.80).
+__device__ __noinline__ uint32_t run_call(uint32_t at, uint32_t pl, uint32_t ws, uint32_t excl, uint32_t total,
+                                          uint32_t j, uint32_t j2, uint32_t a, uint32_t b) {
+  return run_here(at, pl, ws, excl, total, j, j2, a, b);
+}
+
+template <bool LONG>
+__device__ __forceinline__ uint32_t run(uint32_t at, uint32_t pl, uint32_t ws, uint32_t excl, uint32_t total,
+                                        uint32_t j, uint32_t j2, uint32_t a, uint32_t b) {
+  if constexpr (LONG) return run_call(at, pl, ws, excl, total, j, j2, a, b);
+  else return run_here(at, pl, ws, excl, total, j, j2, a, b);
+}
+
 // Slots of a hash of wn entries: a power of two, at least four slots an entry.
 __device__ __forceinline__ uint32_t hash_slots(uint32_t wn) { return max(32u, 1u << (32 - __clz(4 * wn - 1))); }
 
 // Build the frame's pivot in the warp's all-zero buffer.
-__device__ __noinline__ void build(uint32_t at, uint32_t bm_words) {
+__device__ __forceinline__ void build(uint32_t at, uint32_t bm_words) {
   const uint32_t lane = threadIdx.x & 31;
   Frame* fr = frame(at);
   uint32_t* bm = buffer(at);
@@ -345,7 +376,7 @@ __device__ __noinline__ void build(uint32_t at, uint32_t bm_words) {
 }
 
 // Back to an all-zero buffer, and the frame to no pivot.
-__device__ __noinline__ void clear(uint32_t at) {
+__device__ __forceinline__ void clear(uint32_t at) {
   __syncwarp();
   const uint32_t lane = threadIdx.x & 31;
   Frame* fr = frame(at);
@@ -383,7 +414,7 @@ __device__ __forceinline__ void load_pivot(uint32_t at, uint32_t k, uint32_t lan
 // lane; one that goes on past the batch stays built (it is the batch's last).
 // Returns this lane's hits.
 template <bool LONG>
-__device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t base, uint32_t be) {
+__device__ __forceinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t base, uint32_t be) {
   const uint32_t lane = threadIdx.x & 31;
   Frame* fr = frame(at);
   const uint32_t room = (1u << (31 - __clz(bm_words))) / (2 * kRunSlots);  // pairs of a run
@@ -394,9 +425,9 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
     uint4 d = make_uint4(~0u, 0, 0, 0);
     if (k + lane < fr->npiv) d = __ldg(fr->piv + 2 * (uint64_t)(k + lane));
     np = __popc(__ballot_sync(FULL, d.x < be));
-    const uint32_t a = max(d.x, base) - base, b = min(d.y, be) - base;
-    const bool alone = d.x >= be || b <= a || b - a >= (LONG ? kAloneLong : kAlone) || d.y > be || d.w > room || !fr->plain || lane == 31 ||
-                       (lane == 0 && fr->kind != kNone);
+    const uint32_t a = min(max(d.x, base) - base, 32u), b = min(max(d.y, base) - base, be - base);
+    const bool alone = d.x >= be || b <= a || b - a >= (LONG ? kAloneLong : kAlone) || d.y > be || d.w > room ||
+                       !fr->plain || lane == 31 || (lane == 0 && fr->kind != kNone);
     const uint32_t single = __ballot_sync(FULL, alone);
     uint32_t cum = alone ? 0u : d.w;
 #pragma unroll
@@ -404,31 +435,34 @@ __device__ __noinline__ uint32_t mixed(uint32_t at, uint32_t bm_words, uint32_t 
       const uint32_t x = __shfl_up_sync(FULL, cum, s);
       if (lane >= s) cum += x;
     }
+    const uint32_t ws = d.z, ab = a << 8 | b;  // all that a lane keeps, with its scan, across the calls below
     for (uint32_t j = 0; j < np;) {
       if ((single >> j) & 1u) {
-        const uint32_t aj = __shfl_sync(FULL, a, j), bj = __shfl_sync(FULL, b, j);
+        const uint32_t abj = __shfl_sync(FULL, ab, j), aj = abj >> 8, bj = abj & 0xffu;
         if (fr->kind == kNone) {
           load_pivot(at, k + j, lane);
           build(at, bm_words);
         }
-        if ((int32_t)(bj - aj) > 0) hits += probe_kind<LONG>(at, aj, bj);
+        if (bj > aj) hits += probe_kind<LONG>(at, aj, bj);
         more = fr->p1 > be;
         if (!more) clear(at);
         j++;
       } else {
-        const uint32_t before = __shfl_sync(FULL, cum, j) - __shfl_sync(FULL, d.w, j);
+        uint32_t excl = __shfl_up_sync(FULL, cum, 1);  // the scan, exclusive
+        if (lane == 0) excl = 0;
+        const uint32_t before = __shfl_sync(FULL, excl, j);
         // the run ends before the first later pivot that stands alone or does not fit
-        const uint32_t stop = __ballot_sync(FULL, lane > j && (alone || cum - before > room));
+        const uint32_t stop = __ballot_sync(FULL, lane > j && (((single >> lane) & 1u) || cum - before > room));
         const uint32_t j2 = stop ? (uint32_t)__ffs(stop) - 1 : np;
-        const uint32_t starts = __reduce_or_sync(FULL, lane >= j && lane < j2 ? 1u << a : 0u);
+        const uint32_t starts = __reduce_or_sync(FULL, lane >= j && lane < j2 ? 1u << (ab >> 8) : 0u);
         const uint32_t pl = j + __popc(starts & (FULL >> (31 - lane))) - 1;  // this entry's pivot
         // entries between the run's pivots belong to vertices without a row
-        const uint32_t own_end = __shfl_sync(FULL, b, pl), run_start = __shfl_sync(FULL, a, j),
-                       run_end = __shfl_sync(FULL, b, j2 - 1);
+        const uint32_t own_end = __shfl_sync(FULL, ab, pl) & 0xffu, run_start = __shfl_sync(FULL, ab, j) >> 8,
+                       run_end = __shfl_sync(FULL, ab, j2 - 1) & 0xffu;
         if (lane >= own_end && lane > run_start && lane < run_end) fr->entry[lane].y = 0;
         __syncwarp();
         const uint32_t total = __shfl_sync(FULL, cum, j2 - 1) - before;
-        hits += run(at, pl, d.z, cum - d.w - before, total, j, j2, run_start, run_end);
+        hits += run<LONG>(at, pl, ws, excl - before, total, j, j2, run_start, run_end);
         j = j2;
       }
     }
