@@ -234,6 +234,11 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
     o.use_cuda_graph = 0;
     if (L.blocks_per_sm && (!o.blocks_per_sm || o.blocks_per_sm > L.blocks_per_sm)) o.blocks_per_sm = L.blocks_per_sm;
     const bool fused = o.kernel == BBTC_KERNEL_FUSED || (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
+    // The large lane's blocks take 40 registers a thread: with 48, three of
+    // them left no SM the registers for a small load's sort, which then waited
+    // for the large count to end (1,160 requests/s, p99 of the small ones: 7.0
+    // ms, with 40 registers 1.7; a large count's median 2.5 and 3.5 ms).
+    if (fused && L.blocks_per_sm && !o.occupancy) o.occupancy = 6;
     int rc = BBTC_OK;
     if (!fused) {
       for (size_t i = 0; i < batch.size(); i++) {
