@@ -45,16 +45,16 @@ class OrientedCSR:
         return 4 * self.m + 4 * s
 
     def fused_bytes(self, cuts) -> dict:
-        """Bytes one count by fused task rows reads at least, each byte once
+        """Bytes one fused count reads at least, each byte once
         per use (no reuse through the caches), for a CSR oriented from lower
         to higher ids:
 
         * 8 per streamed (32-id word, bit mask) pair: in-edge (u, v) streams
           the pairs of N+(u) from the one holding v to the row's end;
         * 8 per in-edge record (first pair, end pair);
-        * per pivot visit -- vertex v once per row part i that holds one of
-          its in-neighbours (reversed tile (part(v), i)) -- its word pairs
-          (8 each) and 28 bytes of row pointers and first / last ids.
+        * per pivot visit -- vertex v once per row part that holds one of its
+          in-neighbours, so once with cuts [0, n], which is what the pivot
+          lists do -- its word pairs (8 each) and 28 bytes of bounds.
 
         Returns the total and its parts."""
         n, m = self.n, self.m

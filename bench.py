@@ -233,7 +233,7 @@ class Clocks:
 
 def load_traffic(family: str, scale: int, ncut: int):
     """Per-launch DRAM bytes of the count kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_fused_queue_traffic.json")
+    path = os.path.join(ROOT, "profiles", "k_count_pivots_traffic.json")
     try:
         with open(path) as f:
             d = json.load(f)
@@ -731,7 +731,7 @@ def main():
                  "launches_per_step": plaunches // len(ptimes), "persistent_over_plain": pt / t_mean}
         # the same per-task kernel as the plain form, every task's units in one
         # persistent launch from the device queue: separates the queue's gain
-        # from the fused task rows' algorithmic gain
+        # from the fused count's algorithmic gain
         qo = options(mode="persistent", kernel="bitmap", bitmap_words=args.bitmap_words, cuda_graph=True)
         tl = st.task_list(sorted=True)
         qtimes, qcounts = [], set()
@@ -741,7 +741,7 @@ def main():
                 e0 = torch.cuda.Event(enable_timing=True)
                 e1 = torch.cuda.Event(enable_timing=True)
                 e0.record(stream)
-                st.count_async(tl, opts=qo)  # an explicit per-task kernel: the task queue, not task rows
+                st.count_async(tl, opts=qo)  # an explicit per-task kernel: the task queue, not the fused count
                 e1.record(stream)
             qcounts.add(st.count_wait())
             if i >= 2:
@@ -845,7 +845,7 @@ def main():
                                            "`bench.py --config serve --rates ...` (profiles/serving_sweep.md)"})
 
     peak, peak_kind = peaks()
-    fb = g.fused_bytes(cuts) if args.kernel in ("auto", "fused") else None
+    fb = g.fused_bytes([0, g.n]) if args.kernel in ("auto", "fused") else None
     model_bytes = fb["bytes"] if fb else balg
     achieved = model_bytes / t_mean / 1e9
     traffic, traffic_note = load_traffic(args.family, args.scale, args.ncut)
@@ -867,7 +867,7 @@ def main():
         "e2e": e2e,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                     "model_bytes": model_bytes, "model": ("fused task rows" if fb else "B_alg"),
+                     "model_bytes": model_bytes, "model": ("fused pivot lists" if fb else "B_alg"),
                      "model_parts": fb,
                      "peak_note": "of measured (MEASURED_PEAKS.json hbm_gbs)"
                      if peak_kind == "measured" else "of fallback",
@@ -875,9 +875,9 @@ def main():
                      "dram_gbs": (traffic / t_mean / 1e9) if traffic else None,
                      "dram_frac": (traffic / t_mean / 1e9 / peak) if traffic else None,
                      "note": ("achieved = model bytes / count time (CUDA events on the library's stream). Model "
-                              "(fused task rows, the default path): 8 B per streamed (32-id word, bit mask) pair "
+                              "(fused pivot lists, the default path): 8 B per streamed (32-id word, bit mask) pair "
                               "(in-edge (u, v) streams N+(u) from v's word to the row's end), 8 B per in-edge "
-                              "record, and per pivot visit its word pairs plus 28 B of row pointers and bounds -- "
+                              "record, and per pivot (once) its word pairs plus 28 B of list bounds and first word -- "
                               "each byte once per use, no cache reuse. merge_frac: the same time against B_alg = "
                               "4m + 4 sum over edges of d+(u) + d+(v), the ids a merge intersection streams, "
                               "which this kernel does not read. dram_gbs: ncu DRAM traffic of one launch over the "
