@@ -77,6 +77,7 @@ def lib() -> ctypes.CDLL:
         "bbtc_version": [],
         "bbtc_debug_fail_alloc": [c.c_int64, c.POINTER(c.c_int64)],
         "bbtc_debug_stage_timeout": [vp, u32],
+        "bbtc_debug_layout_timeout": [vp, c.c_int, u32],
         "bbtc_ctx_create": [c.c_int, c.POINTER(vp)],
         "bbtc_ctx_destroy": [vp],
         "bbtc_ctx_stream": [vp, c.POINTER(vp)],
@@ -184,6 +185,12 @@ class Context:
         not issued and each staging wait gives up after `polls` polls, so a
         count that stages returns BBTC_ERR_TIMEOUT; 0 restores normal staging."""
         check(lib().bbtc_debug_stage_timeout(self.handle, int(polls)))
+
+    def debug_layout_timeout(self, which: int, polls: int) -> None:
+        """Test hook: with polls > 0 the first tile of an upload's pair pass (1)
+        or pivot pass (2) publishes nothing and the waits for it give up after
+        `polls` polls, so an upload of several tiles returns BBTC_ERR_TIMEOUT."""
+        check(lib().bbtc_debug_layout_timeout(self.handle, int(which), int(polls)))
 
     @property
     def sm_count(self) -> int:

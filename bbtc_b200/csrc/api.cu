@@ -157,6 +157,14 @@ int bbtc_debug_stage_timeout(bbtc_ctx* ctx, uint32_t polls) {
   return BBTC_OK;
 }
 
+int bbtc_debug_layout_timeout(bbtc_ctx* ctx, int pass, uint32_t polls) {
+  if (!ctx) return fail(BBTC_ERR_ARG, "NULL argument");
+  if (polls && pass != 1 && pass != 2) return fail(BBTC_ERR_ARG, "pass must be 1 (pairs) or 2 (pivots)");
+  ctx->debug_layout_pass = (uint32_t)pass;
+  ctx->debug_layout_polls = polls;
+  return BBTC_OK;
+}
+
 int bbtc_ctx_create(int device, bbtc_ctx** out) {
   if (!out) return fail(BBTC_ERR_ARG, "out is NULL");
   *out = nullptr;

@@ -170,6 +170,8 @@ struct bbtc_ctx {
                                        // by a kernel instead of the copy engines (0 = never)
   uint32_t debug_stage_polls = 0;      // test hook (bbtc_debug_stage_timeout): > 0 = staging copies are not
                                        // issued and their waits give up after this many polls
+  uint32_t debug_layout_pass = 0;      // test hook (bbtc_debug_layout_timeout): the single-pass layout kernel (1 the
+  uint32_t debug_layout_polls = 0;     // pairs', 2 the pivots') whose first tile stays silent, and its waits' polls
   // Page-locked staging for the small control copies (cut vectors, tile
   // offsets and statistics, counts).  A copy to or from pageable memory is
   // staged by the driver through buffers every thread shares, so one that

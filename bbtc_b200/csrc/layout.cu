@@ -136,7 +136,11 @@ __global__ void k_row_heads(const uint32_t* __restrict__ indptr, const uint32_t*
 // published -- their own counts, or from some tile on the sum up to it.  A
 // tile's word is (state << 62 | value): 0 nothing yet, 1 the tile's own, 2 up
 // to and including it.  Tickets follow the order in which blocks start, so the
-// tiles waited for are running or done; the waits are bounded all the same.
+// tiles waited for are running or done; the waits are bounded all the same,
+// and a block whose wait ran out leaves without writing (a sum that lacks
+// tiles would send its writes out of range): the build fails.  With `dbg` > 0,
+// the test hook of bbtc_debug_layout_timeout, the first tile publishes nothing
+// and the waits give up after `dbg` polls.
 // Tiles are small (8 warps of 8 chunks of 32) while few of them would leave
 // SMs idle, and large (16 warps of 16 chunks) where the sum over earlier tiles
 // would bound the pass.  Small and large, us: k_pairs R-MAT s12 7.2 / 12.4,
@@ -161,31 +165,34 @@ __device__ __forceinline__ void tile_store(uint64_t* p, uint64_t v) {
 // What the tiles before tile i (in ticket order) hold together.  `a` carries
 // counts; with HEADS, `b` carries for each tile the count from its first head
 // on (0: no head) -- the counts run towards the tiles before, so the nearest
-// tile with a head gives the count up to it.  Called by one warp.
+// tile with a head gives the count up to it.  Called by one warp; false when a
+// tile has not published after `limit` polls, or another block gave up
+// waiting: there is no sum then, and the block has to leave without using one.
 struct TileSum {
   uint32_t count, head;
 };
 template <bool HEADS>
-__device__ __forceinline__ TileSum tiles_before(const uint64_t* a, const uint64_t* b, uint32_t i, uint32_t* bad) {
+__device__ __forceinline__ bool tiles_before(const uint64_t* a, const uint64_t* b, uint32_t i, uint32_t* bad,
+                                             uint32_t limit, TileSum& out) {
   const uint32_t lane = threadIdx.x & 31;
-  TileSum out{0, 0};
+  out = TileSum{0, 0};
   uint32_t polls = 0;
   for (int64_t j = (int64_t)i - 1; j >= 0; j -= 32) {
     const int64_t at = j - lane;
     uint64_t va = kUpTo, vb = kUpTo;  // before the first tile: nothing
-    bool ok;
+    bool ok, gave_up = false;
     do {
       if (at >= 0) {
         va = tile_load(a + at);
         vb = HEADS ? tile_load(b + at) : va;
       }
       ok = va >> 62 != 0 && va >> 62 == vb >> 62;  // both words of one publication
-      if (!ok && ++polls > kTilePolls) {
-        atomicOr(bad, kBadWait);
-        va = vb = kUpTo;
-        ok = true;
-      }
-    } while (!__all_sync(FULLMASK, ok));
+      if (!ok) gave_up = ++polls > limit || (polls % 1024 == 0 && (__ldcg(bad) & kBadWait));
+    } while (!__all_sync(FULLMASK, ok || gave_up));
+    if (!__all_sync(FULLMASK, ok)) {
+      if (lane == 0) atomicOr(bad, kBadWait);
+      return false;
+    }
     const uint32_t sums = __ballot_sync(FULLMASK, va >> 62 == 2);
     const uint32_t last = sums ? __ffs(sums) - 1 : 32;  // the nearest tile with a sum
     const uint32_t own = lane < last ? (uint32_t)va : 0u;
@@ -197,7 +204,7 @@ __device__ __forceinline__ TileSum tiles_before(const uint64_t* a, const uint64_
       } else if (last < 32) {
         out.head = __shfl_sync(FULLMASK, (uint32_t)vb, last);
         out.count += __reduce_add_sync(FULLMASK, own) + __shfl_sync(FULLMASK, (uint32_t)va, last);
-        return out;
+        return true;
       }
     } else if (HEADS) {
       out.head += __reduce_add_sync(FULLMASK, own);
@@ -207,10 +214,10 @@ __device__ __forceinline__ TileSum tiles_before(const uint64_t* a, const uint64_
       const uint32_t sum = __shfl_sync(FULLMASK, (uint32_t)va, last);
       out.count += sum;
       if (HEADS && out.head) out.head += sum;
-      return out;
+      return true;
     }
   }
-  return out;
+  return true;
 }
 
 // Edge part of the input contract (rows strictly increasing, ids < n), the
@@ -231,8 +238,8 @@ __global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pairs(const uint32_t*
                                                uint32_t n, uint64_t m, uint2* __restrict__ words,
                                                uint2* __restrict__ rec, uint32_t* __restrict__ head_pair,
                                                uint64_t* __restrict__ sums, uint64_t* __restrict__ head_sums,
-                                               uint32_t* __restrict__ flags) {
-  __shared__ uint32_t s_tile, s_count[kTileWarps], s_head[kTileWarps];
+                                               uint32_t* __restrict__ flags, uint32_t dbg) {
+  __shared__ uint32_t s_tile, s_summed, s_count[kTileWarps], s_head[kTileWarps];
   __shared__ TileSum s_before;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr uint32_t kTile = kTileWarps * kTileChunks * 32;
@@ -299,15 +306,20 @@ __global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pairs(const uint32_t*
         tile_store(sums + i, kOwn | tile_C);
         tile_store(head_sums + i, kOwn | tile_H);
       }
-      const TileSum b = tiles_before<true>(sums, head_sums, i, &flags[kFlagBad]);
-      if (lane == 0) {
-        tile_store(sums + i, kUpTo | (b.count + tile_C));
-        tile_store(head_sums + i, kUpTo | (tile_H ? b.count + tile_H : b.head));
+      TileSum b;
+      const bool summed = tiles_before<true>(sums, head_sums, i, &flags[kFlagBad], dbg ? dbg : kTilePolls, b);
+      if (lane == 0) s_summed = summed;
+      if (lane == 0 && summed) {
+        if (!dbg || i > 0) {
+          tile_store(sums + i, kUpTo | (b.count + tile_C));
+          tile_store(head_sums + i, kUpTo | (tile_H ? b.count + tile_H : b.head));
+        }
         s_before = b;
         if (i == ntiles - 1) flags[kFlagPairs] = b.count + tile_C;
       }
     }
     __syncthreads();
+    if (!s_summed) return;
     if (H) H += s_before.count; else H = s_before.head;
     C += s_before.count;
     // bits of the edges after the warp's that belong to its last pair
@@ -387,9 +399,10 @@ constexpr uint32_t kSparsePivots = 8;
 // below their rows, k_fix_pivots and k_fix_entries go over the result.)
 template <uint32_t kTileWarps, uint32_t kTileChunks, int MINB>
 __global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pivots(PivotInput in, uint32_t* __restrict__ piv, uint32_t* __restrict__ crow,
-                                                uint64_t* __restrict__ sums, uint32_t* __restrict__ flags) {
+                                                uint64_t* __restrict__ sums, uint32_t* __restrict__ flags,
+                                                uint32_t dbg) {
   if (flags[kFlagBad]) return;
-  __shared__ uint32_t s_tile, s_count[kTileWarps], s_before;
+  __shared__ uint32_t s_tile, s_summed, s_count[kTileWarps], s_before;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t m = in.m;
   constexpr uint32_t kTile = kTileWarps * kTileChunks * 32;
@@ -462,9 +475,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pivots(PivotInput in,
     }
     if (warp == 0) {
       if (lane == 0 && i > 0) tile_store(sums + i, kOwn | tile_C);
-      const TileSum b = tiles_before<false>(sums, sums, i, &flags[kFlagBad]);
-      if (lane == 0) {
-        tile_store(sums + i, kUpTo | (b.count + tile_C));
+      TileSum b;
+      const bool summed = tiles_before<false>(sums, sums, i, &flags[kFlagBad], dbg ? dbg : kTilePolls, b);
+      if (lane == 0) s_summed = summed;
+      if (lane == 0 && summed) {
+        if (!dbg || i > 0) tile_store(sums + i, kUpTo | (b.count + tile_C));
         s_before = b.count;
         if (i == ntiles - 1) {
           const uint32_t k = b.count + tile_C;
@@ -476,6 +491,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, MINB) k_pivots(PivotInput in,
       }
     }
     __syncthreads();
+    if (!s_summed) return;
     C += s_before;
     if (lane < kTileChunks && base + 32 * lane < m)
       crow[(base >> 5) + lane] = C + (incl - mine) + (my_first ? (my_pivots & 1u) - 1u : 0u);
@@ -1173,7 +1189,7 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
                            large_pairs ? k_pairs<kLargeWarps, kLargeChunks, 3> : k_pairs<kSmallWarps, kSmallChunks, 4>,
                            tile_grid(pair_tiles), 32 * (large_pairs ? kLargeWarps : kSmallWarps), s, d_indices, heads, n,
                            m, static_cast<uint2*>(g->d_words), rec_in.as<uint2>(), head_pair.as<uint32_t>(), sums,
-                           sums + pair_tiles, flags));
+                           sums + pair_tiles, flags, ctx->debug_layout_pass == 1 ? ctx->debug_layout_polls : 0u));
     // a stable sort of the records by column keeps every in-list in source order
     size_t tb = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, d_indices, keys.as<uint32_t>(), rec_in.as<uint2>(), rec,
@@ -1185,7 +1201,7 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
     BBTC_TRY(launch_layout(
         ctx, large_pivots ? k_pivots<kLargeWarps, kLargeChunks, 3> : k_pivots<kSmallWarps, kSmallChunks, 4>,
         tile_grid(pivot_tiles), 32 * (large_pivots ? kLargeWarps : kSmallWarps), s, in, static_cast<uint32_t*>(g->d_piv),
-        g->d_crow, sums + 2 * pair_tiles, flags));
+        g->d_crow, sums + 2 * pair_tiles, flags, ctx->debug_layout_pass == 2 ? ctx->debug_layout_polls : 0u));
   }
   uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageFlags);
   BBTC_CUDA(cudaMemcpyAsync(h, flags, kFlagWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -68,6 +68,13 @@ int bbtc_debug_fail_alloc(int64_t after, int64_t* left);
  * normal staging.  No reference counterpart (it checks no wait or error). */
 int bbtc_debug_stage_timeout(bbtc_ctx* ctx, uint32_t polls);
 
+/* The same for an upload: with polls > 0, the first tile of the layout pass
+ * that numbers the word pairs (pass = 1) or the pivots (pass = 2) publishes no
+ * count and the waits for it give up after `polls` polls.  An upload of more
+ * than one tile (2,048 edges) then returns BBTC_ERR_TIMEOUT, with nothing
+ * written out of place and nothing held.  polls = 0 restores the context. */
+int bbtc_debug_layout_timeout(bbtc_ctx* ctx, int pass, uint32_t polls);
+
 /* ---- context: device, stream, scratch ------------------------------------
  * Replaces BBTc's constructor GPU set-up and PrepareGpu
  * (src/triangle_counting/bb_tc.cpp:17-33, bb_tc_helper.cpp:53-73): one
