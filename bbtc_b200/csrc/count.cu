@@ -31,6 +31,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <sstream>
 
 #include "deliver.cuh"
@@ -477,17 +479,24 @@ size_t smem_bytes_for(const bbtc_opts& o) {
 }
 
 int kernel_smem_optin(bbtc_ctx* ctx, const bbtc_opts& o) {
-  const size_t sm = smem_bytes(norm_bm_words(o.bitmap_words), norm_warps(o.warps_per_block));
+  const uint32_t bmw = norm_bm_words(o.bitmap_words), wpb = norm_warps(o.warps_per_block);
+  const size_t sm = std::max(smem_bytes(bmw, wpb), pivots_smem(bmw, wpb));
   if (sm > ctx->smem_optin)
     return fail(BBTC_ERR_ARG, "bitmap_words x warps_per_block needs " + std::to_string(sm) +
                                   " bytes of shared memory; the device allows " + std::to_string(ctx->smem_optin));
-  if (sm <= ctx->smem_set) return BBTC_OK;
+  // A kernel has one limit per device, whichever context launches it: it is
+  // only ever raised.
+  static std::mutex mu;
+  static std::map<int, size_t> limit;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& set = limit[ctx->device];
+  if (sm <= set) return BBTC_OK;
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_CUDA(cudaFuncSetAttribute(k_count_task, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   BBTC_TRY(pivots_smem_optin(sm));
-  ctx->smem_set = sm;
+  set = sm;
   return BBTC_OK;
 }
 
