@@ -5,7 +5,8 @@
 //
 //   loader threads: take a pending request whose estimated device footprint
 //     fits the HBM budget -- the smallest, or the oldest once it has waited
-//     aging_ms -- build its device block CSR (upload + layout) on the
+//     aging_ms -- build its device layout (upload + layout, and the block
+//     CSRs where the server counts task by task) on the
 //     loader's stream for its size class (small: highest priority, a CSR in
 //     page-locked host memory read by a kernel rather than the copy
 //     engines; large: lowest priority, layout grids capped at 2 blocks per
@@ -66,6 +67,11 @@ uint64_t estimate_bytes(uint32_t n, uint64_t m, const std::vector<uint32_t>& cut
   uint64_t rp = 0;
   for (uint64_t x = 0; x < P; x++) rp += P * (((uint64_t)cuts[x + 1] - cuts[x] + 1 + 3) & ~3ull);
   return csr + lists + temps + 3 * 4 * (rp + 4) + 2 * 4 * (m + 4 * P * P + 4) + 2 * 4 * (m / 32 + 2 * P * P + 2);
+}
+
+// Do counts with these options run task by task (over the block CSRs)?
+bool counts_tasks(const bbtc_opts& o) {
+  return o.kernel != BBTC_KERNEL_FUSED && !(o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
 }
 
 struct Request {
@@ -180,8 +186,14 @@ void loader_main(bbtc_server* s, bbtc_ctx* ctx_small, bbtc_ctx* ctx_large, bool 
     // a large layout runs on a low-priority stream with its grids capped, so
     // the small ones' kernels are scheduled first and find free SMs
     bbtc_ctx* ctx = lane_of(s, r) == 0 ? ctx_small : ctx_large;
-    const int rc = bbtc_graph_upload(ctx, r->n, r->indptr, r->indices, r->m, r->cuts.data(),
-                                     (uint32_t)r->cuts.size() - 1, &g);
+    int rc = bbtc_graph_upload(ctx, r->n, r->indptr, r->indices, r->m, r->cuts.data(),
+                               (uint32_t)r->cuts.size() - 1, &g);
+    // a per-task count's block CSRs are part of what the request holds, so
+    // they are built before its reservation becomes its real size
+    if (rc == BBTC_OK && counts_tasks(s->opts.count)) {
+      rc = s->opts.count.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(g) : ensure_tiles(g);
+      if (rc != BBTC_OK) bbtc_graph_free(g);
+    }
     lk.lock();
     s->loading--;
     if (large) s->loading_large--;
@@ -233,7 +245,7 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
     bbtc_opts o = s->opts.count;
     o.use_cuda_graph = 0;
     if (L.blocks_per_sm && (!o.blocks_per_sm || o.blocks_per_sm > L.blocks_per_sm)) o.blocks_per_sm = L.blocks_per_sm;
-    const bool fused = o.kernel == BBTC_KERNEL_FUSED || (o.kernel == BBTC_KERNEL_AUTO && o.mode == BBTC_MODE_PERSISTENT);
+    const bool fused = !counts_tasks(o);
     // The large lane's blocks take 40 registers a thread: with 48, three of
     // them left no SM the registers for a small load's sort, which then waited
     // for the large count to end (1,160 requests/s, p99 of the small ones: 7.0
@@ -241,8 +253,7 @@ void launcher_main(bbtc_server* s, uint32_t lane) {
     if (fused && L.blocks_per_sm && !o.occupancy) o.occupancy = 6;
     int rc = BBTC_OK;
     if (!fused) {
-      for (size_t i = 0; i < batch.size(); i++) {
-        if (rc == BBTC_OK) rc = o.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(gs[i]) : ensure_tiles(gs[i]);
+      for (size_t i = 0; i < batch.size(); i++) {  // their block CSRs came with the load
         uint32_t nt = 0;
         bbtc_task_list(gs[i]->P, nullptr, 0, &nt);
         tl[i].resize(nt);
@@ -584,10 +595,7 @@ int bbtc_submit(bbtc_server* s, uint32_t n, const uint32_t* indptr, const uint32
   r->indptr = indptr;
   r->indices = indices;
   r->cuts.assign(cuts, cuts + P + 1);
-  const bbtc_opts& co = s->opts.count;
-  const bool tiles = !(co.kernel == BBTC_KERNEL_FUSED ||
-                       (co.kernel == BBTC_KERNEL_AUTO && co.mode == BBTC_MODE_PERSISTENT));
-  r->reserved = estimate_bytes(n, m, r->cuts, tiles);
+  r->reserved = estimate_bytes(n, m, r->cuts, counts_tasks(s->opts.count));
   r->t_submit = now_ns();
   std::lock_guard<std::mutex> lk(s->mu);
   if (s->stop) {
