@@ -402,6 +402,11 @@ static int count_async_impl(bbtc_ctx* ctx, bbtc_graph* g, const bbtc_task* tasks
     BBTC_TRY(o.kernel == BBTC_KERNEL_MERGE ? ensure_fwd(g) : ensure_tiles(g));
     if (tasks) tl[0].assign(tasks, tasks + ntasks); else tl[0] = default_tasks(g, o.sort_tasks != 0);
   }
+  // A count recorded into the caller's CUDA graph runs again without this call: from
+  // then on no call here knows which count the context's staging holds.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  BBTC_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) ctx->recorded = true;
   // border b >= 0: tasks [0, b) are queued ahead of the rest; with one device queue in list
   // order that is the list order itself, so the value only has to be in range.
   std::vector<bbtc_graph*> gs{g};
@@ -437,7 +442,7 @@ int bbtc_count_wait(bbtc_ctx* ctx, bbtc_graph* g, uint64_t* out) {
   if (!ctx || !g || !out) return fail(BBTC_ERR_ARG, "NULL argument");
   BBTC_CUDA(cudaSetDevice(ctx->device));
   // the context's last delivered count is in its staging already; an earlier one, or one of a plain launch, is copied
-  const bool here = g->delivered && g->ctx == ctx && g->delivered == ctx->delivered;
+  const bool here = !ctx->recorded && g->delivered && g->ctx == ctx && g->delivered == ctx->delivered;
   uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + (here ? kStageCount : kStageOut));
   if (!here) BBTC_CUDA(cudaMemcpyAsync(h, g->d_count, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
   BBTC_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -178,6 +178,7 @@ struct bbtc_ctx {
   // threads; copies from pinned memory wait only for their own stream.
   char* h_stage = nullptr;
   uint64_t delivered = 0;  // counts delivered to h_stage (Delivery) so far; the last one is there
+  bool recorded = false;   // a count was launched into a capture of the stream: its replays deliver there unseen
   // Pinned staging of the task queues' uploads, kept across plans.
   char* h_plan = nullptr;
   size_t h_plan_cap = 0;
