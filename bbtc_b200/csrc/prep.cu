@@ -186,6 +186,22 @@ int balloc(Buf& b, size_t bytes, cudaStream_t s) {
   return BBTC_OK;
 }
 
+// A sort's temporary: kept from one sort to the next while it is large enough.
+struct Temp {
+  Buf b;
+  size_t cap = 0;
+};
+
+int reserve(Temp& t, size_t bytes, cudaStream_t s) {
+  if (bytes <= t.cap) return BBTC_OK;
+  if (t.b.p) cudaFreeAsync(t.b.p, s);
+  t.b.p = nullptr;
+  t.cap = 0;
+  BBTC_TRY(balloc(t.b, bytes, s));
+  t.cap = bytes;
+  return BBTC_OK;
+}
+
 }  // namespace
 }  // namespace bbtc
 
@@ -216,7 +232,10 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   const int grid = ctx->sms * 8;
   const int b = bits_for((uint64_t)n + 1);  // bits of an end: n itself marks the dropped pairs
   const uint64_t mm = std::max<uint64_t>(m_raw, 1);
-  Buf keys, keys2, sel, ends, firsts, deg, ids, ids2, deg2, rank, tmp;
+  // At most 28 bytes a pair: the keys twice, a sort's temporary, the result's
+  // ids.  The degrees' arrays lie in those that are not in use yet.
+  Buf keys, keys2, sel, deg, ids, ids2, deg2, rank;
+  Temp tmp;
   BBTC_TRY(balloc(keys, mm * 8, s));
   BBTC_TRY(balloc(keys2, mm * 8, s));
   BBTC_TRY(balloc(sel, 16, s));  // distinct pairs, "some were dropped"
@@ -231,10 +250,10 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     size_t tu = 0;
     BBTC_CUDA(cub::DeviceSelect::Unique(nullptr, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), sel.as<uint64_t>(),
                                         (int64_t)m_raw, s));
-    BBTC_TRY(balloc(tmp, std::max(tb, tu), s));
-    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb, keys.as<uint64_t>(), keys2.as<uint64_t>(), (int64_t)m_raw, 0,
+    BBTC_TRY(reserve(tmp, std::max(tb, tu), s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp.b.p, tb, keys.as<uint64_t>(), keys2.as<uint64_t>(), (int64_t)m_raw, 0,
                                              2 * b, s));
-    BBTC_CUDA(cub::DeviceSelect::Unique(tmp.p, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), sel.as<uint64_t>(),
+    BBTC_CUDA(cub::DeviceSelect::Unique(tmp.b.p, tu, keys2.as<uint64_t>(), keys.as<uint64_t>(), sel.as<uint64_t>(),
                                         (int64_t)m_raw, s));
     uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageFlags);
     BBTC_CUDA(cudaMemcpyAsync(h, sel.p, 16, cudaMemcpyDeviceToHost, s));
@@ -249,19 +268,16 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   BBTC_TRY(balloc(rank, ((size_t)n + 1) * 4, s));
   BBTC_CUDA(cudaMemsetAsync(deg.p, 0, ((size_t)n + 1) * 4, s));
   if (m_und) {
-    BBTC_TRY(balloc(firsts, 2 * ((size_t)n + 1) * 4, s));
-    BBTC_TRY(balloc(ends, 2 * m_und * 4, s));
-    uint32_t* upper = ends.as<uint32_t>();
+    uint32_t* upper = keys2.as<uint32_t>();  // free until the pairs are relabelled
     uint32_t* upper_sorted = upper + m_und;
-    uint32_t* first_lower = firsts.as<uint32_t>();
-    uint32_t* first_upper = first_lower + n + 1;
+    uint32_t* first_lower = deg2.as<uint32_t>();  // free until the vertices are sorted
+    uint32_t* first_upper = ids2.as<uint32_t>();
     k_ends<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, b, first_lower, upper);
     BBTC_CUDA(cudaGetLastError());
     size_t te = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, te, upper, upper_sorted, (int64_t)m_und, 0, b, s));
-    Buf tmp4;
-    BBTC_TRY(balloc(tmp4, te, s));
-    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp4.p, te, upper, upper_sorted, (int64_t)m_und, 0, b, s));
+    BBTC_TRY(reserve(tmp, te, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp.b.p, te, upper, upper_sorted, (int64_t)m_und, 0, b, s));
     k_degrees<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), upper_sorted, m_und, b, first_lower, deg.as<uint32_t>(),
                                    first_upper);
     BBTC_CUDA(cudaGetLastError());
@@ -275,9 +291,8 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     size_t tr = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tr, deg.as<uint32_t>(), deg2.as<uint32_t>(), ids.as<uint32_t>(),
                                               ids2.as<uint32_t>(), (int64_t)n, 0, b, s));
-    Buf tmp2;
-    BBTC_TRY(balloc(tmp2, tr, s));
-    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp2.p, tr, deg.as<uint32_t>(), deg2.as<uint32_t>(), ids.as<uint32_t>(),
+    BBTC_TRY(reserve(tmp, tr, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.b.p, tr, deg.as<uint32_t>(), deg2.as<uint32_t>(), ids.as<uint32_t>(),
                                               ids2.as<uint32_t>(), (int64_t)n, 0, b, s));
     k_rank<<<grid, 256, 0, s>>>(ids2.as<uint32_t>(), n, rank.as<uint32_t>());
     BBTC_CUDA(cudaGetLastError());
@@ -296,9 +311,8 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     size_t tb = 0;
     BBTC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), (int64_t)m_und, 0,
                                              2 * b, s));
-    Buf tmp3;
-    BBTC_TRY(balloc(tmp3, tb, s));
-    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp3.p, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), (int64_t)m_und, 0,
+    BBTC_TRY(reserve(tmp, tb, s));
+    BBTC_CUDA(cub::DeviceRadixSort::SortKeys(tmp.b.p, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), (int64_t)m_und, 0,
                                              2 * b, s));
     k_split<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, b, d_indices);
     BBTC_CUDA(cudaGetLastError());

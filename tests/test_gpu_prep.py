@@ -1,4 +1,6 @@
 """Device-side preparation equals the host pipeline bit for bit."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -78,3 +80,32 @@ def test_cuts_on_device_equal_host(ctx, make):
             got = core.cuts_device(ctx, kind, g.n, ip.data_ptr(), ix.data_ptr(), g.m, P)
             want = graphs.cuts(g, P, kind)
             assert np.array_equal(got, want), (kind, P, got, want)
+
+
+def test_orient_device_memory(ctx):
+    """Preparation holds 36 bytes a pair at most: two arrays of keys (16) and a
+    sort's own copy (8) throughout, and beside them the degrees' arrays and then
+    the result (4) and the last sort's copy (8).  32 bytes a vertex; 8 MiB of
+    histograms and rounding."""
+    torch = pytest.importorskip("torch")
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool = ctypes.c_void_p()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    USED, USED_HIGH = 7, 8  # cudaMemPoolAttrUsedMemCurrent, cudaMemPoolAttrUsedMemHigh
+
+    def attr(which):
+        v = ctypes.c_uint64()
+        assert rt.cudaMemPoolGetAttribute(pool, which, ctypes.byref(v)) == 0
+        return v.value
+
+    n, m = 1 << 16, 1 << 22
+    s, d = (torch.randint(0, n, (m,), dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    before = attr(USED)
+    assert rt.cudaMemPoolSetAttribute(pool, USED_HIGH, ctypes.byref(ctypes.c_uint64(0))) == 0
+    dev = core.DeviceCSR(ctx, n, s.data_ptr(), d.data_ptr(), m)
+    peak = attr(USED_HIGH) - before
+    print(f"{peak / m:.2f} bytes a pair")
+    assert dev.m > m * 9 // 10
+    dev.free()
+    assert peak <= 36 * m + 32 * n + (8 << 20)
