@@ -297,14 +297,11 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     k_rank<<<grid, 256, 0, s>>>(ids2.as<uint32_t>(), n, rank.as<uint32_t>());
     BBTC_CUDA(cudaGetLastError());
   }
-  uint32_t* d_indptr = nullptr;
-  uint32_t* d_indices = nullptr;
-  if (dev_malloc(&d_indptr, ((size_t)n + 1) * 4, s) != cudaSuccess ||
-      dev_malloc(&d_indices, std::max<uint64_t>(m_und, 1) * 4, s) != cudaSuccess) {
-    cudaGetLastError();
-    if (d_indptr) cudaFreeAsync(d_indptr, s);
-    return fail(BBTC_ERR_NOMEM, "device allocation of the oriented CSR failed");
-  }
+  Buf out_indptr, out_indices;  // freed with the rest when a step below fails
+  BBTC_TRY(balloc(out_indptr, ((size_t)n + 1) * 4, s));
+  BBTC_TRY(balloc(out_indices, std::max<uint64_t>(m_und, 1) * 4, s));
+  uint32_t* d_indptr = out_indptr.as<uint32_t>();
+  uint32_t* d_indices = out_indices.as<uint32_t>();
   if (m_und) {
     k_relabel<<<grid, 256, 0, s>>>(keys.as<uint64_t>(), m_und, rank.as<uint32_t>(), b, keys2.as<uint64_t>());
     BBTC_CUDA(cudaGetLastError());
@@ -322,6 +319,7 @@ int bbtc_orient_device(bbtc_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   BBTC_CUDA(cudaStreamSynchronize(s));
   out->indptr = d_indptr;
   out->indices = d_indices;
+  out_indptr.p = out_indices.p = nullptr;  // the caller's now
   out->n = n;
   out->m = m_und;
   return BBTC_OK;

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle
-from bbtc_b200 import core, graphs
+from bbtc_b200 import BBTcError, core, graphs
 
 pytestmark = pytest.mark.gpu
 
@@ -109,3 +109,38 @@ def test_orient_device_memory(ctx):
     assert dev.m > m * 9 // 10
     dev.free()
     assert peak <= 36 * m + 32 * n + (8 << 20)
+
+
+def test_failed_preparation_holds_nothing(ctx):
+    """Each device allocation of a preparation fails in turn: BBTC_ERR_NOMEM, and
+    the device's pool holds what it held before."""
+    torch = pytest.importorskip("torch")
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool = ctypes.c_void_p()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def used():
+        torch.cuda.synchronize()
+        v = ctypes.c_uint64()
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(v)) == 0  # cudaMemPoolAttrUsedMemCurrent
+        return v.value
+
+    n, m = 1000, 20000
+    s, d = (torch.randint(0, n, (m,), dtype=torch.int32, device="cuda") for _ in range(2))
+    before = used()
+    try:
+        for k in range(100):
+            core.debug_fail_alloc(k)
+            try:
+                dev = core.DeviceCSR(ctx, n, s.data_ptr(), d.data_ptr(), m)
+            except BBTcError as e:
+                assert e.status == -3, (k, e.message)
+                assert used() == before, k
+                continue
+            assert core.debug_fail_alloc(-1) >= 0  # every allocation passed
+            dev.free()
+            break
+        assert 5 < k < 99
+        assert used() == before
+    finally:
+        core.debug_fail_alloc(-1)
