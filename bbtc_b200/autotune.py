@@ -1,5 +1,6 @@
 """Autotuner front end: the sweep runs in the library (bbtc_autotune), the
-winners are kept in a small JSON cache keyed by GPU name and graph statistics.
+winners are kept in a small JSON cache keyed by GPU name, graph statistics and
+the generation of the count kernels.
 
 Cache file: $BBTC_AUTOTUNE_CACHE, else ~/.cache/bbtc_b200/autotune.json.
 """
@@ -16,6 +17,10 @@ import numpy as np
 from . import core
 
 _lock = threading.Lock()
+
+# Part of a saved pick's key: a pick holds for the kernels that it was timed
+# with.  Raise it when the kernels, or what an option means to them, change.
+KERNELS = 2
 
 
 class TuneSpace(ctypes.Structure):
@@ -82,7 +87,7 @@ def sweep(graph: core.Graph, base: core.Opts | None = None, bitmap_words=None, w
 
 def tune(graph: core.Graph, use_cache: bool = True, **kw) -> tuple[core.Opts, float | None]:
     """Cached autotune: returns (options, ms) -- ms is None on a cache hit."""
-    key = f"{gpu_name(graph.ctx.device)}|{graph_key(graph)}"
+    key = f"{gpu_name(graph.ctx.device)}|{graph_key(graph)}|kernels={KERNELS}"
     path = cache_path()
     if use_cache:
         with _lock:

@@ -466,19 +466,50 @@ int bbtc_last_launches(const bbtc_graph* g, uint32_t* launches) {
 
 int bbtc_autotune(bbtc_ctx* ctx, bbtc_graph* g, const bbtc_tune_space* space, bbtc_opts* inout, double* best_ms) {
   if (!ctx || !g || !inout) return fail(BBTC_ERR_ARG, "NULL argument");
+  // The default sweep: unit sizes of 0 (by position in the queue, or by an
+  // even share) beside fixed ones, and the occupancies that have a kernel.
+  // Units of 8192 probes and 8 blocks per SM, in earlier sweeps, were best
+  // nowhere (R-MAT s14 to s22, Chung-Lu 2^20, geometric 2^17; fused, bitmap and
+  // search), while a sweep without the automatic size missed the untuned time
+  // (bitmap kernel, R-MAT s14: 0.418 ms against 0.102).
   static const uint32_t kWords[] = {256, 512, 1024, 2048, 4096};
   static const uint32_t kWarps[] = {4, 8};
-  static const uint32_t kWork[] = {256, 2048, 8192};
-  static const uint32_t kOcc[] = {4, 6, 8};
-  bbtc_tune_space sp{kWords, 5, kWarps, 2, kWork, 3, 3, kOcc, 3};
+  static const uint32_t kWork[] = {0, 256, 2048};
+  static const uint32_t kOccFused[] = {4, 5, 6}, kOccTasks[] = {4, 6};
+  const bool fused = inout->kernel == BBTC_KERNEL_FUSED ||
+                     (inout->kernel == BBTC_KERNEL_AUTO && inout->mode == BBTC_MODE_PERSISTENT);
+  const bbtc_tune_space all{kWords, 5, kWarps, 2, kWork, 3, 3, fused ? kOccFused : kOccTasks, fused ? 3u : 2u};
+  bbtc_tune_space sp = all;
+  bool chosen = false;  // the caller lists values of some option
   if (space) {
     sp = *space;
-    if (!sp.occupancy || !sp.n_occupancy) { sp.occupancy = kOcc; sp.n_occupancy = 3; }
-    if (!sp.bitmap_words || !sp.n_bitmap_words) { sp.bitmap_words = kWords; sp.n_bitmap_words = 5; }
-    if (!sp.warps_per_block || !sp.n_warps_per_block) { sp.warps_per_block = kWarps; sp.n_warps_per_block = 2; }
-    if (!sp.unit_work || !sp.n_unit_work) { sp.unit_work = kWork; sp.n_unit_work = 3; }
-    if (!sp.repeats) sp.repeats = 3;
+    auto list = [&](const uint32_t*& v, uint32_t& n, const uint32_t* dv, uint32_t dn) {
+      if (v && n) {
+        chosen = true;
+      } else {
+        v = dv;
+        n = dn;
+      }
+    };
+    list(sp.bitmap_words, sp.n_bitmap_words, all.bitmap_words, all.n_bitmap_words);
+    list(sp.warps_per_block, sp.n_warps_per_block, all.warps_per_block, all.n_warps_per_block);
+    list(sp.unit_work, sp.n_unit_work, all.unit_work, all.n_unit_work);
+    list(sp.occupancy, sp.n_occupancy, all.occupancy, all.n_occupancy);
+    if (!sp.repeats) sp.repeats = all.repeats;
   }
+  std::vector<bbtc_opts> points;
+  if (!chosen) points.push_back(*inout);  // the options as they came: the pick is not slower
+  for (uint32_t iw = 0; iw < sp.n_bitmap_words; iw++)
+    for (uint32_t ip = 0; ip < sp.n_warps_per_block; ip++)
+      for (uint32_t iu = 0; iu < sp.n_unit_work; iu++)
+        for (uint32_t io = 0; io < sp.n_occupancy; io++) {
+          bbtc_opts o = *inout;
+          o.bitmap_words = sp.bitmap_words[iw];
+          o.warps_per_block = sp.warps_per_block[ip];
+          o.unit_work = sp.unit_work[iu];
+          o.occupancy = sp.occupancy[io];
+          points.push_back(o);
+        }
   BBTC_CUDA(cudaSetDevice(ctx->device));
   cudaEvent_t a, b;
   BBTC_CUDA(cudaEventCreate(&a));
@@ -491,41 +522,33 @@ int bbtc_autotune(bbtc_ctx* ctx, bbtc_graph* g, const bbtc_tune_space* space, bb
   double best_t = 1e300;
   uint64_t ref_count = 0;
   bool have_ref = false;
-  for (uint32_t iw = 0; iw < sp.n_bitmap_words; iw++)
-    for (uint32_t ip = 0; ip < sp.n_warps_per_block; ip++)
-      for (uint32_t iu = 0; iu < sp.n_unit_work; iu++)
-      for (uint32_t io = 0; io < sp.n_occupancy; io++) {
-        bbtc_opts o = *inout;
-        o.bitmap_words = sp.bitmap_words[iw];
-        o.warps_per_block = sp.warps_per_block[ip];
-        o.unit_work = sp.unit_work[iu];
-        o.occupancy = sp.occupancy[io];
-        if (smem_bytes_for(o) > ctx->smem_optin) continue;  // does not fit this device
-        uint64_t c = 0;
-        BBTC_TRY(bbtc_count(ctx, g, nullptr, 0, -1, &o, &c));  // warm-up, builds the plan
-        std::vector<float> ts;
-        for (uint32_t r = 0; r < sp.repeats; r++) {
-          BBTC_CUDA(cudaEventRecord(a, ctx->stream));
-          BBTC_TRY(bbtc_count_async(ctx, g, nullptr, 0, -1, &o));
-          BBTC_CUDA(cudaEventRecord(b, ctx->stream));
-          BBTC_TRY(bbtc_count_wait(ctx, g, &c));
-          float ms = 0;
-          BBTC_CUDA(cudaEventElapsedTime(&ms, a, b));
-          ts.push_back(ms);
-          if (!have_ref) {
-            ref_count = c;
-            have_ref = true;
-          } else if (c != ref_count) {
-            return fail(BBTC_ERR_STATE, "autotune points disagree on the count");
-          }
-        }
-        std::sort(ts.begin(), ts.end());
-        const double med = ts[ts.size() / 2];
-        if (med < best_t) {
-          best_t = med;
-          best = o;
-        }
+  for (const bbtc_opts& o : points) {
+    if (smem_bytes_for(o) > ctx->smem_optin) continue;  // does not fit this device
+    uint64_t c = 0;
+    BBTC_TRY(bbtc_count(ctx, g, nullptr, 0, -1, &o, &c));  // warm-up, builds the plan
+    std::vector<float> ts;
+    for (uint32_t r = 0; r < sp.repeats; r++) {
+      BBTC_CUDA(cudaEventRecord(a, ctx->stream));
+      BBTC_TRY(bbtc_count_async(ctx, g, nullptr, 0, -1, &o));
+      BBTC_CUDA(cudaEventRecord(b, ctx->stream));
+      BBTC_TRY(bbtc_count_wait(ctx, g, &c));
+      float ms = 0;
+      BBTC_CUDA(cudaEventElapsedTime(&ms, a, b));
+      ts.push_back(ms);
+      if (!have_ref) {
+        ref_count = c;
+        have_ref = true;
+      } else if (c != ref_count) {
+        return fail(BBTC_ERR_STATE, "autotune points disagree on the count");
       }
+    }
+    std::sort(ts.begin(), ts.end());
+    const double med = ts[ts.size() / 2];
+    if (med < best_t) {
+      best_t = med;
+      best = o;
+    }
+  }
   if (!have_ref) return fail(BBTC_ERR_ARG, "no point of the tuning space fits this device");
   *inout = best;
   if (best_ms) *best_ms = best_t;

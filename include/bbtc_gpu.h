@@ -219,7 +219,8 @@ int bbtc_last_launches(const bbtc_graph* g, uint32_t* launches);
  * sizes (the bitmap-vs-search threshold: a pivot row becomes a bitmap when its
  * id span fits, else a sorted list), warps per block and work-unit sizes, and
  * writes the fastest into *inout (mode and kernel are kept).  Every point must
- * give the same count, else BBTC_ERR_STATE.  NULL space = the default sweep.
+ * give the same count, else BBTC_ERR_STATE.  NULL space = the default sweep,
+ * which also times the options as they came; an empty list = its default values.
  * No reference counterpart: the reference fixes its kernel choice by a width
  * test (bb_tc.cpp:98). */
 typedef struct bbtc_tune_space {
