@@ -248,8 +248,8 @@ constexpr size_t kStageBytes = 1u << 20;
 constexpr size_t kStageCuts = 0;          // cut vector, <= (64 + 2) x 4 bytes
 constexpr size_t kStageFlags = 3072;      // contract flags and totals of a layout build; small read-backs
 constexpr size_t kStageCount = 3584;      // the last delivered count and its control word
-constexpr size_t kStageOff = 4096;        // tile + part row offsets of a block CSR (<= 33,288 bytes)
-constexpr size_t kStageStats = 81920;     // its tile statistics (<= 81,920 bytes)
+constexpr size_t kStageOff[2] = {4096, 40960};      // tile offsets of the block CSRs (<= 32,768 bytes each)
+constexpr size_t kStageStats[2] = {81920, 163840};  // their tile statistics (<= 81,920 bytes each)
 constexpr size_t kStageOut = 262144;      // counts read back (<= 98,304 of them)
 
 }  // namespace bbtc

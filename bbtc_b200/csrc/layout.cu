@@ -37,6 +37,7 @@
 
 #include "internal.h"
 #include "layout_check.hpp"
+#include "search.cuh"
 
 namespace bbtc {
 
@@ -604,40 +605,98 @@ __global__ void k_fix_entries(PivotInput in, CutVec cuts, const uint4* __restric
   }
 }
 
-// Row id of every edge of a CSR that meets the contract, one warp per row.
-__global__ void k_row_ids(const uint32_t* __restrict__ indptr, uint32_t n, uint32_t* __restrict__ rows) {
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Row id of every edge of a CSR that meets the contract.  A warp takes `run`
+// consecutive edges (a multiple of 32), whatever their rows: it searches the
+// first one's row in 32-way steps and then compares the edges with the ends of
+// 32 rows at a time.  A warp per row left lanes idle (R-MAT s20, 15 edges a
+// row: 90 us; now 52).
+__global__ void k_row_ids(const uint32_t* __restrict__ indptr, uint32_t n, uint64_t m, uint32_t run,
+                          uint32_t* __restrict__ rows) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t u = warp; u < n; u += nwarps) {
-    const uint32_t b = indptr[u + 1];
-    for (uint64_t e = (uint64_t)indptr[u] + lane; e < b; e += 32) rows[e] = (uint32_t)u;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  auto row_end = [&](uint32_t u) {  // of row u + lane; past the last row: above any edge
+    return (uint64_t)u + lane < n ? __ldg(indptr + u + 1 + lane) : ~0u;
+  };
+  for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * run < m; c += warps) {
+    const uint64_t end = min(m, (c + 1) * run);
+    uint32_t u = row_of(indptr, n, (uint32_t)(c * run));
+    uint32_t ends = row_end(u);
+    for (uint64_t e0 = c * run; e0 < end; e0 += 32) {
+      const uint64_t e = e0 + lane;
+      bool done = e >= end;
+      while (true) {
+        uint32_t k = 0;  // rows of the window that end at or before e
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(FULLMASK, ends, k + step - 1) <= e) k += step;
+        const bool inside = __shfl_sync(FULLMASK, ends, k) > e;
+        if (!done && inside) {
+          rows[e] = u + k;
+          done = true;
+        }
+        const uint32_t rest = __ballot_sync(FULLMASK, !done);
+        if (!rest) break;
+        const uint32_t next = (uint32_t)(e0 + __ffs(rest) - 1);
+        u += 32;  // below n: a row past the window holds edge `next`
+        ends = row_end(u);
+        if (__shfl_sync(FULLMASK, ends, 31) <= next) {  // empty rows between, in any number
+          u = row_of(indptr, n, next);
+          ends = row_end(u);
+        }
+      }
+    }
   }
 }
 
-// Run lengths: the first edge of each (row, tile) run writes the length into
-// slot (rp_off[tile] + local row + 1) of the counts buffer.  runs[e] = e for
-// the first edge of a run, else 0: its inclusive max-scan gives every edge
-// the start of its run.
-__global__ void k_entry_count(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
-                              const uint32_t* __restrict__ rows, uint64_t m, const uint32_t* __restrict__ cuts_g,
-                              uint32_t P, const uint64_t* __restrict__ rp_off, uint32_t* __restrict__ counts,
-                              uint32_t* __restrict__ runs) {
-  __shared__ uint32_t cuts[kMaxParts + 1];
-  for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) cuts[t] = cuts_g[t];
-  __syncthreads();
+// The parts of a cut vector in a block's shared memory.  An id's part: from the
+// part of its bucket's first id on (part_of's bisection was most of the edge
+// passes' instructions); a row's: from the part of a lower row on.
+struct Parts {
+  static constexpr uint32_t kBuckets = 1024;
+  uint32_t cuts[kMaxParts + 1];
+  uint32_t shift;
+  uint8_t first[kBuckets];
+  __device__ __forceinline__ void load(const uint32_t* __restrict__ g, uint32_t P) {
+    for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) cuts[t] = g[t];
+    const uint32_t ids = g[P], bits = 32 - __clz(ids);
+    const uint32_t sh = bits > 10 ? bits - 10 : 0;  // ids < 2^bits: at most kBuckets buckets
+    if (threadIdx.x == 0) shift = sh;
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < kBuckets && (uint64_t)b << sh < ids; b += blockDim.x)
+      first[b] = (uint8_t)part_of(cuts, P, b << sh);
+    __syncthreads();
+  }
+  // `from`: the part of this id or of a lower one
+  __device__ __forceinline__ uint32_t at(uint32_t id, uint32_t from) const {
+    while (id >= cuts[from + 1]) from++;  // ends: id < cuts[P]
+    return from;
+  }
+  __device__ __forceinline__ uint32_t of(uint32_t id) const { return at(id, first[id >> shift]); }
+};
+
+// Length of every (row, tile) run, added up in slot (rp_off[tile] + local row
+// + 1) of the counts buffer, by the edges that start it or a batch of 32.  (The
+// run's end was searched from its first edge: R-MAT s20, both directions, 180
+// us; now 136, instructions bound it.)
+__global__ void k_entry_count(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ rows, uint64_t m,
+                              const uint32_t* __restrict__ cuts_g, uint32_t P, const uint64_t* __restrict__ rp_off,
+                              uint32_t* __restrict__ counts) {
+  __shared__ Parts parts;
+  parts.load(cuts_g, P);
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t x = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
-    const uint32_t u = rows[e];
-    const uint32_t c = indices[e];
-    const uint32_t y = part_of(cuts, P, c);
-    const uint32_t a = indptr[u];
-    const bool first = e == a || indices[e - 1] < cuts[y];
-    runs[e] = first ? (uint32_t)e : 0u;
-    if (!first) continue;
-    const uint32_t end = lower_bound_range(indices, (uint32_t)e, indptr[u + 1], cuts[y + 1]);
-    const uint32_t x = part_of(cuts, P, u);
-    counts[rp_off[x * P + y] + (u - cuts[x]) + 1] = end - (uint32_t)e;
+  for (uint64_t e0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; e0 < m; e0 += stride) {
+    const uint64_t e = e0 + lane;
+    const uint32_t u = e < m ? rows[e] : ~0u;  // no row's number
+    const uint32_t y = e < m ? parts.of(indices[e]) : 0u;
+    const uint32_t pu = __shfl_up_sync(FULLMASK, u, 1), py = __shfl_up_sync(FULLMASK, y, 1);
+    const bool first = lane == 0 || u != pu || y != py;
+    const uint32_t later = __ballot_sync(FULLMASK, first) & (lane < 31 ? FULLMASK << (lane + 1) : 0u);
+    if (first && e < m) {
+      x = parts.at(u, x);
+      atomicAdd(&counts[rp_off[x * P + y] + (u - parts.cuts[x]) + 1], (later ? __ffs(later) - 1 : 32u) - lane);
+    }
   }
 }
 
@@ -662,56 +721,41 @@ __global__ void k_zero_ranges(ZeroRanges z) {
   }
 }
 
-// One pass over the row-pointer pool: `scanned` is the inclusive scan of the
-// run counts, so a slot minus its tile's first slot is the tile-local row
-// pointer written to `rp`; per tile, the longest row and the number of
-// non-empty rows (a row's length is the difference of two scanned slots).
-// Lanes of one tile are combined before the atomics.
+// `scanned` is the inclusive scan of the run counts, so a slot minus its
+// tile's first slot is the tile-local row pointer written to `rp`; per tile,
+// the longest row and the number of non-empty rows (a row's length is the
+// difference of two scanned slots).  blockIdx.y = tile: a pass over the pool
+// as one array looked up every slot's tile (R-MAT s20, P 8: 63 us; now 21).
 __global__ void k_localize_stats(uint32_t* __restrict__ rp, const uint32_t* __restrict__ scanned,
-                                 const uint32_t* __restrict__ cuts_g, uint32_t P,
-                                 const uint64_t* __restrict__ part_off, uint64_t len, uint32_t* __restrict__ maxdeg,
-                                 uint32_t* __restrict__ nerows) {
-  __shared__ uint32_t cuts[kMaxParts + 1];
-  __shared__ uint64_t poff[kMaxParts + 1];
-  for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) {
-    cuts[t] = cuts_g[t];
-    poff[t] = part_off[t];
+                                 const uint32_t* __restrict__ cuts, uint32_t P, const uint64_t* __restrict__ rp_off,
+                                 uint32_t* __restrict__ maxdeg, uint32_t* __restrict__ nerows) {
+  const uint32_t t = blockIdx.y, x = t / P;
+  const uint32_t H = cuts[x + 1] - cuts[x];
+  const uint64_t slots = ((uint64_t)H + 4) & ~3ull;  // H + 1 and the padding to the next tile
+  if ((uint64_t)blockIdx.x * blockDim.x >= slots) return;
+  __shared__ uint32_t longest, nonempty;
+  if (threadIdx.x == 0) longest = nonempty = 0;
+  __syncthreads();
+  const uint64_t first = rp_off[t];
+  const uint32_t base = scanned[first];
+  uint32_t mx = 0, ne = 0;
+  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < slots; r += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = scanned[first + r];
+    rp[first + r] = v - base;
+    const uint32_t len = r < H ? scanned[first + r + 1] - v : 0u;
+    mx = max(mx, len);
+    ne += len != 0;
+  }
+  mx = __reduce_max_sync(FULLMASK, mx);
+  ne = __reduce_add_sync(FULLMASK, ne);
+  if ((threadIdx.x & 31) == 0 && ne) {
+    atomicMax(&longest, mx);
+    atomicAdd(&nonempty, ne);
   }
   __syncthreads();
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t start = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t iters = (len + stride - 1) / stride;  // the same for every lane of a warp
-  for (uint64_t it = 0; it < iters; it++) {
-    const uint64_t s = start + it * stride;
-    uint32_t tile = 0xffffffffu, rowlen = 0;
-    if (s < len) {
-      uint32_t lo = 0, hi = P;  // row part x: last x with part_off[x] <= s
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (poff[mid] <= s) lo = mid; else hi = mid;
-      }
-      const uint64_t A = (poff[lo + 1] - poff[lo]) / P;  // slots per tile of this row part
-      const uint32_t y = (uint32_t)((s - poff[lo]) / A);
-      const uint32_t r = (uint32_t)(s - poff[lo] - (uint64_t)y * A);
-      const uint32_t v = scanned[s];
-      rp[s] = v - scanned[poff[lo] + (uint64_t)y * A];
-      if (r < cuts[lo + 1] - cuts[lo]) {
-        rowlen = scanned[s + 1] - v;
-        tile = lo * P + y;
-      }
-    }
-    // a warp's 32 slots lie in one tile but at a tile's end: group lanes by
-    // tile only there (match and a per-group reduction are slow)
-    const uint32_t grp = __all_sync(FULLMASK, tile == __shfl_sync(FULLMASK, tile, 0))
-                             ? FULLMASK
-                             : __match_any_sync(FULLMASK, tile);
-    const uint32_t mx = __reduce_max_sync(grp, rowlen);
-    const uint32_t ne = __popc(grp & __ballot_sync(FULLMASK, rowlen != 0));
-    if (tile != 0xffffffffu && lane == (uint32_t)(__ffs(grp) - 1)) {
-      if (ne) atomicAdd(&nerows[tile], ne);
-      if (mx) atomicMax(&maxdeg[tile], mx);
-    }
+  if (threadIdx.x == 0 && nonempty) {
+    atomicMax(&maxdeg[t], longest);
+    atomicAdd(&nerows[t], nonempty);
   }
 }
 
@@ -747,58 +791,99 @@ __global__ void k_tile_offsets(const uint32_t* __restrict__ rp, const uint64_t* 
   }
 }
 
-// Row index of every 32nd entry: erow[t][x / 32] = the row holding entry x
-// of tile t, for x = 0, 32, 64, ... < nnz.  A work unit starting at a
-// multiple of 32 finds its first row with one load.  Every such x lies in
-// exactly one non-empty row, so each slot has one writer.  blockIdx.y = tile.
-__global__ void k_row_index(const uint32_t* __restrict__ rp, const uint64_t* __restrict__ rp_off,
-                            const uint32_t* __restrict__ cuts, uint32_t P, const uint64_t* __restrict__ col_off,
-                            uint32_t* __restrict__ erow) {
-  const uint32_t t = blockIdx.y;
-  if (col_off[t] == kNoSegment) return;
-  const uint32_t x = t / P;
-  const uint32_t H = cuts[x + 1] - cuts[x];
-  const uint32_t* __restrict__ r = rp + rp_off[t];
-  uint32_t* __restrict__ er = erow + col_off[t] / 32 + t;
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < H; b += gridDim.x * blockDim.x) {
-    const uint32_t s = r[b], e = r[b + 1];
-    // 64-bit: rounding s up to a multiple of 32 must not wrap near 2^32
-    for (uint64_t q = ((uint64_t)s + 31) & ~31ull; q < e; q += 32) er[q >> 5] = b;
+// First edge of the (row, tile) run that holds edge `base` of row u, whose ids
+// are `lo` or more: the first at or above (u, lo) in the edges' order.  Asked
+// for by a whole warp: distances of 1, 2, 4, ... back from base, then 32-way
+// steps.
+__device__ __forceinline__ uint32_t run_start(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ indices,
+                                              uint32_t base, uint32_t u, uint32_t lo) {
+  const uint32_t lane = threadIdx.x & 31;
+  auto below = [&](uint64_t e) { return rows[e] < u || (rows[e] == u && indices[e] < lo); };
+  const uint32_t before = __ballot_sync(FULLMASK, base < (1u << lane) || below(base - (1u << lane)));
+  const uint32_t k = before ? __ffs(before) - 1 : 32;  // nearest distance 2^k that is before the run
+  uint32_t hi = k == 0 ? base : base - (1u << (k - 1));
+  uint32_t at = k == 32 || base < (1u << k) ? 0 : base - (1u << k) + 1;  // the answer is in [at, hi]
+  while (at < hi) {
+    const uint32_t step = (hi - at + 31) / 32;
+    const uint64_t e = at + (uint64_t)lane * step;
+    const uint32_t n = __popc(__ballot_sync(FULLMASK, e < hi && below(e)));
+    if (n == 0) return at;
+    hi = (uint32_t)min((uint64_t)hi, at + (uint64_t)n * step);
+    at += (n - 1) * step + 1;
   }
+  return at;
 }
 
-// Scatter tile-local column ids into the column pool.
-__global__ void k_entry_scatter(const uint32_t* __restrict__ runs, const uint32_t* __restrict__ indices,
-                                const uint32_t* __restrict__ rows, uint64_t m, const uint32_t* __restrict__ cuts_g,
-                                uint32_t P, const uint64_t* __restrict__ rp_off, const uint64_t* __restrict__ col_off,
-                                const uint32_t* __restrict__ rp, uint32_t* __restrict__ col) {
-  __shared__ uint32_t cuts[kMaxParts + 1];
-  for (uint32_t t = threadIdx.x; t <= P; t += blockDim.x) cuts[t] = cuts_g[t];
-  __syncthreads();
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += stride) {
-    const uint32_t u = rows[e];
-    const uint32_t c = indices[e];
-    const uint32_t y = part_of(cuts, P, c);
-    const uint32_t x = part_of(cuts, P, u);
-    const uint32_t t = x * P + y;
-    const uint32_t run = runs[e];  // first edge of this (row, tile) run
-    const uint64_t pos = col_off[t] + rp[rp_off[t] + (u - cuts[x])] + ((uint32_t)e - run);
-    col[pos] = c - cuts[y];
-  }
-}
-
-// rev_indptr[v] = first position of key v in the sorted keys (v <= n).
-__global__ void k_rev_indptr(const uint32_t* __restrict__ keys, uint64_t m, uint32_t n,
-                             uint32_t* __restrict__ rev_indptr) {
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += stride) {
-    uint64_t lo = 0, hi = m;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if (keys[mid] < v) lo = mid + 1; else hi = mid;
+// Scatter tile-local column ids into the column pool, and the row index of
+// every 32nd entry: erow[t][x / 32] = the row that holds entry x of tile t,
+// for x = 0, 32, 64, ... < nnz, so that a work unit that starts at a multiple
+// of 32 finds its first row with one load.  A warp takes kRunEdges consecutive
+// edges.  Where a (row, tile) run starts among them its start is known; the run
+// that they begin in is searched.  The edges of a run take its place in the
+// pool from the first of them in the batch.  (The starts came from a max-scan
+// over an array of all edges, the row index from a pass over the rows: R-MAT
+// s20, both directions, 320 us; now 226.)
+constexpr uint32_t kRunEdges = 128;
+__global__ void k_entry_scatter(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ rows, uint64_t m,
+                                const uint32_t* __restrict__ cuts_g, uint32_t P, const uint64_t* __restrict__ rp_off,
+                                const uint64_t* __restrict__ col_off, const uint32_t* __restrict__ rp,
+                                uint32_t* __restrict__ col, uint32_t* __restrict__ erow) {
+  __shared__ Parts parts;
+  parts.load(cuts_g, P);
+  const uint32_t* cuts = parts.cuts;
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t x = 0;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * kRunEdges < m; w += warps) {
+    const uint32_t base = (uint32_t)(w * kRunEdges);
+    uint32_t u[kRunEdges / 32], c[kRunEdges / 32];
+#pragma unroll
+    for (uint32_t k = 0; k < kRunEdges / 32; k++) {
+      const uint64_t e = (uint64_t)base + 32 * k + lane;
+      u[k] = e < m ? rows[e] : ~0u;  // no row's number
+      c[k] = e < m ? indices[e] : 0u;
     }
-    rev_indptr[v] = (uint32_t)lo;
+    uint32_t run = 0, last_u = 0, last_y = 0;  // the run of the edges before these
+#pragma unroll
+    for (uint32_t k = 0; k < kRunEdges / 32; k++) {
+      const uint32_t e0 = base + 32 * k, y = parts.of(c[k]);
+      uint32_t pu = __shfl_up_sync(FULLMASK, u[k], 1), py = __shfl_up_sync(FULLMASK, y, 1);
+      if (lane == 0) {
+        pu = last_u;
+        py = last_y;
+      }
+      last_u = __shfl_sync(FULLMASK, u[k], 31);
+      last_y = __shfl_sync(FULLMASK, y, 31);
+      bool first = u[k] != pu || y != py;
+      if (k == 0) {
+        run = run_start(rows, indices, base, __shfl_sync(FULLMASK, u[0], 0),
+                        cuts[__shfl_sync(FULLMASK, y, 0)]);
+        if (lane == 0) first = run == base;
+      }
+      const uint32_t starts = __ballot_sync(FULLMASK, first);
+      // the first of each run's edges here looks the run's place up
+      uint64_t tile_col = 0;
+      uint32_t to = 0, index = 0, row = 0;
+      if ((first || lane == 0) && u[k] != ~0u) {
+        x = parts.at(u[k], x);
+        const uint32_t t = x * P + y;
+        row = u[k] - cuts[x];
+        tile_col = col_off[t];
+        index = (uint32_t)(tile_col / 32) + t;
+        to = rp[rp_off[t] + row] - (first ? e0 + lane : run);  // modulo 2^32: plus an edge, its entry of the tile
+      }
+      const uint32_t mine = starts & (FULLMASK >> (31 - lane)), head = mine ? 31 - __clz(mine) : 0;
+      tile_col = __shfl_sync(FULLMASK, tile_col, head);
+      to = __shfl_sync(FULLMASK, to, head);
+      index = __shfl_sync(FULLMASK, index, head);
+      row = __shfl_sync(FULLMASK, row, head);
+      if (u[k] != ~0u) {
+        const uint32_t at = to + e0 + lane;
+        col[tile_col + at] = c[k] - cuts[y];
+        if ((at & 31) == 0) erow[index + (at >> 5)] = row;
+      }
+      if (starts) run = e0 + 31 - __clz(starts);
+    }
   }
 }
 
@@ -869,27 +954,26 @@ int launch_layout(const bbtc_ctx* ctx, void (*kernel)(KArgs...), dim3 grid, dim3
   return BBTC_OK;
 }
 
-// Build one block CSR (forward or reversed) from a CSR in device memory whose
-// per-edge row ids are `rows`.  The tile statistics land in d_stats (device,
-// 4*P*P words) and are copied to the host by the caller.
-int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const uint32_t* d_indices,
-                const uint32_t* d_rows, uint32_t n, uint64_t m, const std::vector<uint32_t>& cuts,
-                const uint32_t* d_cuts, uint32_t* d_stats, uint64_t* d_coloff, int grid) {
+// Build one block CSR (forward or reversed) from the edges' ids and row ids, in
+// row order.  What the host keeps of it -- T column offsets
+// (64-bit), then nnz, longest row and non-empty rows per tile -- lands in
+// d_stats and, when the stream has run, in region `which` of the staging
+// (read_stats).
+int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indices, const uint32_t* d_rows, uint64_t m,
+                const std::vector<uint32_t>& cuts, const uint32_t* d_cuts, uint64_t* d_stats, int which, int grid) {
   const uint32_t P = (uint32_t)cuts.size() - 1;
   const uint32_t T = P * P;
   cudaStream_t s = ctx->stream;
   bt.P = P;
   bt.rp_off.assign(T, 0);
-  std::vector<uint64_t> part_off(P + 1, 0);
   uint64_t cur = 0;
   for (uint32_t x = 0; x < P; x++) {
-    part_off[x] = cur;
     const uint64_t A = align4((uint64_t)cuts[x + 1] - cuts[x] + 1);
     for (uint32_t y = 0; y < P; y++) bt.rp_off[x * P + y] = cur + y * A;
     cur += A * P;
   }
-  part_off[P] = cur;
-  bt.rp_len = cur + 4;  // a 16-byte tail keeps rounded-up reads inside the pool
+  const uint64_t slots = cur;
+  bt.rp_len = slots + 4;  // a 16-byte tail keeps rounded-up reads inside the pool
   bt.col_len = m + 4ull * T + 4;
   bt.erow_len = bt.col_len / 32 + T + 1;  // tile t's index starts at col_off[t] / 32 + t
   {
@@ -903,78 +987,62 @@ int build_block(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_indptr, const u
     }
   }
   bt.stream = s;
-  DevBuf offs, counts, runs;
-  BBTC_TRY(dalloc(runs, std::max<uint64_t>(m, 1) * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(offs, (T + P + 1) * sizeof(uint64_t), s));
+  DevBuf offs, counts;
+  BBTC_TRY(dalloc(offs, T * sizeof(uint64_t), s));
   BBTC_TRY(dalloc(counts, bt.rp_len * sizeof(uint32_t), s));
   uint64_t* d_rp_off = offs.as<uint64_t>();
-  uint64_t* d_part_off = d_rp_off + T;
   {
     // through a pinned region that is not written again before the build's final sync
-    uint64_t* h = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageOff);
+    char* h = ctx->h_stage + kStageOff[which];
     std::memcpy(h, bt.rp_off.data(), T * sizeof(uint64_t));
-    std::memcpy(h + T, part_off.data(), (P + 1) * sizeof(uint64_t));
-    BBTC_CUDA(cudaMemcpyAsync(d_rp_off, h, (T + P + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+    BBTC_CUDA(cudaMemcpyAsync(d_rp_off, h, T * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
   }
+  uint64_t* d_coloff = d_stats;
+  uint32_t* st_nnz = reinterpret_cast<uint32_t*>(d_stats + T);
+  uint32_t* st_max = st_nnz + T;
+  uint32_t* st_ne = st_nnz + 2 * T;
   {
     // run counts, column pool, tile statistics and the row-pointer pool's
     // 16-byte tail (every other slot of the pool is written below)
-    ZeroRanges z{{counts.as<uint32_t>(), bt.d_col, d_stats, bt.d_rp + part_off[P]},
-                 {bt.rp_len, bt.col_len, 4ull * T, bt.rp_len - part_off[P]}};
+    ZeroRanges z{{counts.as<uint32_t>(), bt.d_col, reinterpret_cast<uint32_t*>(d_stats), bt.d_rp + slots},
+                 {bt.rp_len, bt.col_len, 5ull * T, bt.rp_len - slots}};
     BBTC_TRY(launch_layout(ctx, k_zero_ranges, grid, 256, s, z));
   }
-  if (m > 0) {
-    BBTC_TRY(launch_layout(ctx, k_entry_count, grid, 256, s, d_indptr, d_indices, d_rows, m, d_cuts, P, d_rp_off,
-                           counts.as<uint32_t>(), runs.as<uint32_t>()));
-    size_t rb = 0;
-    BBTC_CUDA(cub::DeviceScan::InclusiveScan(nullptr, rb, runs.as<uint32_t>(), runs.as<uint32_t>(), cub::Max(),
-                                             (int64_t)m, s));
-    DevBuf rtmp;
-    BBTC_TRY(dalloc(rtmp, rb, s));
-    BBTC_CUDA(cub::DeviceScan::InclusiveScan(rtmp.p, rb, runs.as<uint32_t>(), runs.as<uint32_t>(), cub::Max(),
-                                             (int64_t)m, s));
-  }
+  if (m > 0)
+    BBTC_TRY(launch_layout(ctx, k_entry_count, grid, 256, s, d_indices, d_rows, m, d_cuts, P, d_rp_off,
+                           counts.as<uint32_t>()));
   // run counts -> their inclusive scan, in place: k_localize_stats turns it into tile-local row pointers
-  size_t tmp_bytes = 0;
-  BBTC_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, counts.as<uint32_t>(), counts.as<uint32_t>(),
-                                          (int64_t)part_off[P], s));
-  DevBuf tmp;
-  BBTC_TRY(dalloc(tmp, tmp_bytes, s));
-  BBTC_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, tmp_bytes, counts.as<uint32_t>(), counts.as<uint32_t>(),
-                                          (int64_t)part_off[P], s));
-  uint32_t* st_nnz = d_stats;
-  uint32_t* st_max = d_stats + T;
-  uint32_t* st_ne = d_stats + 2 * T;
-  BBTC_TRY(launch_layout(ctx, k_localize_stats, grid, 256, s, bt.d_rp, counts.as<uint32_t>(), d_cuts, P, d_part_off,
-                         part_off[P], st_max, st_ne));
-  BBTC_TRY(launch_layout(ctx, k_tile_offsets, 1, 32, s, bt.d_rp, d_rp_off, d_cuts, P, st_nnz, d_coloff));
   {
-    uint32_t maxH = 1;
-    for (uint32_t x = 0; x < P; x++) maxH = std::max(maxH, cuts[x + 1] - cuts[x]);
-    const uint32_t gx = std::min<uint32_t>(64, (maxH + 255) / 256);
-    BBTC_TRY(launch_layout(ctx, k_row_index, dim3(gx, T), 256, s, bt.d_rp, d_rp_off, d_cuts, P, d_coloff,
-                           bt.d_erow));
+    size_t tmp_bytes = 0;
+    BBTC_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, counts.as<uint32_t>(), counts.as<uint32_t>(),
+                                            (int64_t)slots, s));
+    DevBuf tmp;
+    BBTC_TRY(dalloc(tmp, tmp_bytes, s));
+    BBTC_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, tmp_bytes, counts.as<uint32_t>(), counts.as<uint32_t>(),
+                                            (int64_t)slots, s));
   }
-  if (m > 0) {
-    BBTC_TRY(launch_layout(ctx, k_entry_scatter, grid, 256, s, runs.as<uint32_t>(), d_indices, d_rows, m, d_cuts, P,
-                           d_rp_off, d_coloff, bt.d_rp, bt.d_col));
-  }
+  uint32_t maxH = 1;
+  for (uint32_t x = 0; x < P; x++) maxH = std::max(maxH, cuts[x + 1] - cuts[x]);
+  const uint32_t blocks = std::min<uint32_t>(std::max(64u, 4096 / T), maxH / 1024 + 1);  // 4 slots a thread, or more
+  BBTC_TRY(launch_layout(ctx, k_localize_stats, dim3(blocks, T), 256, s, bt.d_rp, counts.as<uint32_t>(), d_cuts, P,
+                         d_rp_off, st_max, st_ne));
+  BBTC_TRY(launch_layout(ctx, k_tile_offsets, 1, 32, s, bt.d_rp, d_rp_off, d_cuts, P, st_nnz, d_coloff));
+  if (m > 0)
+    BBTC_TRY(launch_layout(ctx, k_entry_scatter, grid, 256, s, d_indices, d_rows, m, d_cuts, P, d_rp_off,
+                           d_coloff, bt.d_rp, bt.d_col, bt.d_erow));
+  BBTC_CUDA(cudaMemcpyAsync(ctx->h_stage + kStageStats[which], d_stats, 20ull * T, cudaMemcpyDeviceToHost, s));
   return BBTC_OK;
 }
 
-// Read back a block CSR's tile statistics (synchronises the stream).
-int fetch_stats(bbtc_ctx* ctx, BlockTiles& bt, const uint32_t* d_stats, const uint64_t* d_coloff, cudaStream_t s) {
+// A built block CSR's statistics, from the staging (after the stream has run).
+void read_stats(const bbtc_ctx* ctx, BlockTiles& bt, int which) {
   const uint32_t T = bt.P * bt.P;
-  uint64_t* hc = reinterpret_cast<uint64_t*>(ctx->h_stage + kStageStats);  // pinned staging: column offsets, statistics
-  uint32_t* hs = reinterpret_cast<uint32_t*>(hc + T);
-  BBTC_CUDA(cudaMemcpyAsync(hc, d_coloff, T * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  BBTC_CUDA(cudaMemcpyAsync(hs, d_stats, 3 * T * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  BBTC_CUDA(cudaStreamSynchronize(s));
+  const uint64_t* hc = reinterpret_cast<const uint64_t*>(ctx->h_stage + kStageStats[which]);
+  const uint32_t* hs = reinterpret_cast<const uint32_t*>(hc + T);
   bt.col_off.assign(hc, hc + T);
   bt.nnz.assign(hs, hs + T);
   bt.maxdeg.assign(hs + T, hs + 2 * T);
   bt.nerows.assign(hs + 2 * T, hs + 3 * T);
-  return BBTC_OK;
 }
 
 // Layout kernels are grid-stride loops: no more blocks than the largest array
@@ -1246,37 +1314,43 @@ int build_layout(bbtc_graph* g, const uint32_t* in_indptr, const uint32_t* in_in
 
 namespace {
 
-// One block CSR of the per-task kernels, from the resident CSR (which passed
-// the contract check when it was uploaded): the forward one, or the reversed
-// one from the edges sorted by column (stable, so in-lists stay in source
-// order).
-int build_tiles(bbtc_graph* g, bool reversed) {
-  Range range(reversed ? "bbtc reversed tiles" : "bbtc forward tiles");
+// Block CSRs of the per-task kernels, from the resident CSR (which passed the
+// contract check when it was uploaded): the forward one, the reversed one from
+// the edges sorted by column (stable, so in-lists stay in source order), or
+// both, which share the row ids and one wait.  The first per-task count of a
+// graph pays for them (R-MAT s12 / s18 / s20, cuts into 8 equal parts, half the
+// list, us: 188 / 378 / 1,011, the next count 34 / 19 / 18; built apart, each
+// with its own row ids and wait, 249 / 528 / 1,434).
+int build_tiles(bbtc_graph* g, bool forward, bool reversed) {
+  Range range("bbtc block CSRs");
   bbtc_ctx* ctx = g->ctx;
   cudaStream_t s = ctx->stream;
   BBTC_CUDA(cudaSetDevice(ctx->device));
+  ScratchScope scratch(ctx, s);
   const uint32_t n = g->n, P = g->P, T = P * P;
   const uint64_t m = g->m, mm = std::max<uint64_t>(m, 1);
   const int grid = layout_grid(ctx, n, m, P);
-  BlockTiles& bt = reversed ? g->rev : g->fwd;
-  DevBuf d_cuts, rows, stats, coloff, keys, sources, rev_indptr;
+  DevBuf d_cuts, rows, stats[2], keys, sources;
   BBTC_TRY(dalloc(d_cuts, g->cuts.size() * sizeof(uint32_t), s));
   BBTC_TRY(dalloc(rows, mm * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(stats, 4 * T * sizeof(uint32_t), s));
-  BBTC_TRY(dalloc(coloff, T * sizeof(uint64_t), s));
   {
     uint32_t* h = reinterpret_cast<uint32_t*>(ctx->h_stage + kStageCuts);
     std::memcpy(h, g->cuts.data(), g->cuts.size() * sizeof(uint32_t));
     BBTC_CUDA(cudaMemcpyAsync(d_cuts.p, h, g->cuts.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   }
-  if (n > 0) BBTC_TRY(launch_layout(ctx, k_row_ids, grid, 256, s, g->d_indptr, n, rows.as<uint32_t>()));
-  const uint32_t* t_indptr = g->d_indptr;
-  const uint32_t* t_indices = g->d_indices;
-  const uint32_t* t_rows = rows.as<uint32_t>();
+  if (m > 0) {  // an even share of the edges per warp, but few where they are few
+    const uint64_t share = (m + 8ull * grid - 1) / (8ull * grid);
+    const uint32_t run = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((share + 31) & ~31ull, 64), 4096);
+    BBTC_TRY(launch_layout(ctx, k_row_ids, grid, 256, s, g->d_indptr, n, m, run, rows.as<uint32_t>()));
+  }
+  if (forward) {
+    BBTC_TRY(dalloc(stats[0], 20ull * T, s));
+    BBTC_TRY(build_block(ctx, g->fwd, g->d_indices, rows.as<uint32_t>(), m, g->cuts,
+                         d_cuts.as<uint32_t>(), stats[0].as<uint64_t>(), 0, grid));
+  }
   if (reversed) {
     BBTC_TRY(dalloc(keys, mm * sizeof(uint32_t), s));
     BBTC_TRY(dalloc(sources, mm * sizeof(uint32_t), s));
-    BBTC_TRY(dalloc(rev_indptr, ((size_t)n + 1) * sizeof(uint32_t), s));
     if (m > 0) {
       size_t tb = 0;
       BBTC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, g->d_indices, keys.as<uint32_t>(), rows.as<uint32_t>(),
@@ -1286,40 +1360,46 @@ int build_tiles(bbtc_graph* g, bool reversed) {
       BBTC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, g->d_indices, keys.as<uint32_t>(), rows.as<uint32_t>(),
                                                 sources.as<uint32_t>(), (int64_t)m, 0, key_bits(n), s));
     }
-    BBTC_TRY(launch_layout(ctx, k_rev_indptr, grid, 256, s, keys.as<uint32_t>(), m, n, rev_indptr.as<uint32_t>()));
-    t_indptr = rev_indptr.as<uint32_t>();
-    t_indices = sources.as<uint32_t>();
-    t_rows = keys.as<uint32_t>();
+    BBTC_TRY(dalloc(stats[1], 20ull * T, s));
+    BBTC_TRY(build_block(ctx, g->rev, sources.as<uint32_t>(), keys.as<uint32_t>(), m, g->cuts,
+                         d_cuts.as<uint32_t>(), stats[1].as<uint64_t>(), 1, grid));
   }
-  BBTC_TRY(build_block(ctx, bt, t_indptr, t_indices, t_rows, n, m, g->cuts, d_cuts.as<uint32_t>(),
-                       stats.as<uint32_t>(), coloff.as<uint64_t>(), grid));
-  BBTC_TRY(fetch_stats(ctx, bt, stats.as<uint32_t>(), coloff.as<uint64_t>(), s));
-  (reversed ? g->rev_built : g->fwd_built) = true;
-  g->device_bytes += block_bytes(bt);
+  BBTC_CUDA(cudaStreamSynchronize(s));
+  if (forward) {
+    read_stats(ctx, g->fwd, 0);
+    g->fwd_built = true;
+    g->device_bytes += block_bytes(g->fwd);
+  }
+  if (reversed) {
+    read_stats(ctx, g->rev, 1);
+    g->rev_built = true;
+    g->device_bytes += block_bytes(g->rev);
+  }
   return BBTC_OK;
 }
 
-int ensure(bbtc_graph* g, bool reversed) {
-  if (reversed ? g->rev_built : g->fwd_built) return BBTC_OK;
-  const int rc = build_tiles(g, reversed);
+int ensure(bbtc_graph* g, bool forward, bool reversed) {
+  forward = forward && !g->fwd_built;
+  reversed = reversed && !g->rev_built;
+  if (!forward && !reversed) return BBTC_OK;
+  const int rc = build_tiles(g, forward, reversed);
   if (rc != BBTC_OK) {
     // a failed build (say, out of memory half way) leaves nothing behind: the
     // frees are stream-ordered after whatever of it was enqueued
-    BlockTiles& bt = reversed ? g->rev : g->fwd;
-    bt.release(g->ctx->stream);
-    bt = BlockTiles();
+    for (BlockTiles* bt : {forward ? &g->fwd : nullptr, reversed ? &g->rev : nullptr})
+      if (bt) {
+        bt->release(g->ctx->stream);
+        *bt = BlockTiles();
+      }
   }
   return rc;
 }
 
 }  // namespace
 
-int ensure_fwd(bbtc_graph* g) { return ensure(g, false); }
+int ensure_fwd(bbtc_graph* g) { return ensure(g, true, false); }
 
-int ensure_tiles(bbtc_graph* g) {
-  BBTC_TRY(ensure(g, false));
-  return ensure(g, true);
-}
+int ensure_tiles(bbtc_graph* g) { return ensure(g, true, true); }
 
 }  // namespace bbtc
 
