@@ -4,9 +4,10 @@
 // kernel, copy the counts back, wait.  With this it is the kernel and the
 // wait, 4 to 5 us less (R-MAT s12: 37 -> 33 us a call).  Not inlined: its
 // pointers would be live, in local memory, across the whole count (R-MAT s22
-// 4.99 ms inlined, 4.92 as a call, 4.97 without it; with it ptxas also lays
-// out the fused count so that small graphs' last units end sooner: s16
-// 100 -> 77 us, s18 230 -> 196).
+// 4.99 ms inlined, 4.92 as a call, 4.97 without it).  Adding the call made the
+// fused kernel itself faster on small graphs (the same kernel without delivering
+// through it: s16 82.6 us against 100 before, s18 200.6 against 230); why is not
+// known, so a change of its code may take that back.
 #pragma once
 #include <cstdint>
 

@@ -10,9 +10,9 @@
 // shared memory and streams those pairs against it.
 //
 // What bounds it: instruction issue and the L1 / shared-memory pipe (R-MAT s20:
-// issue 65 %, that pipe 64 %, DRAM 10 %): every streamed pair is one 8-byte
-// global load and one random shared-memory read.  So the work around the pairs
-// is what the design keeps small:
+// issue 72 %, that pipe 76 %, DRAM at 14 % of the copy rate): every streamed
+// pair is one 8-byte global load and one random shared-memory read.  So the
+// work around the pairs is what the design keeps small:
 //   * no tiles: a pivot's in-edges lie together whatever the cut vector, and
 //     only vertices that are pivots are listed, so no warp walks empty row
 //     pointers (that had left the SMs idle for 30 % of the s20 count);
@@ -26,7 +26,10 @@
 //     queue ends;
 //   * the state between the probe loops lives in shared memory, and what is one
 //     call's is inlined: the loops fit 48 registers (5 blocks of 8 warps on an
-//     SM) without spilling, and few registers are saved around them.
+//     SM) and few registers are saved around them.  Where the loops are
+//     functions, the bitmap's, hash's and search's spill nothing, the rank's and
+//     the run's 16 bytes a call, and the kernel around them 136; inlined, 28 in
+//     all.
 // Per count, against the tiled task rows that this replaced (B200, ms): R-MAT
 // s22 7.09 -> 4.85, s20 1.86 -> 0.78, s16 0.160 -> 0.074, s12 0.095 -> 0.032,
 // Chung-Lu 2^23 17.5 -> 3.68, geometric 2^18 0.432 -> 0.105 (result included).

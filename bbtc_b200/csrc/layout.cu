@@ -145,7 +145,9 @@ __global__ void k_row_heads(const uint32_t* __restrict__ indptr, const uint32_t*
 // Tiles are small (8 warps of 8 chunks of 32) while few of them would leave
 // SMs idle, and large (16 warps of 16 chunks) where the sum over earlier tiles
 // would bound the pass.  Small and large, us: k_pairs R-MAT s12 7.2 / 12.4,
-// s18 45 / 32, s22 570 / 420; k_pivots 8.8 / 16.9, 36 / 42, 371 / 276.
+// s18 45 / 32, s22 570 / 420; k_pivots 8.8 / 16.9, 36 / 42, 371 / 276.  The large
+// forms run at 40 registers (3 blocks of 16 warps an SM) and spill 40 and 148
+// bytes a thread.
 constexpr uint32_t kSmallWarps = 8, kSmallChunks = 8, kLargeWarps = 16, kLargeChunks = 16;
 constexpr uint64_t kLargePairs = 1ull << 20, kLargePivots = 4ull << 20;  // edges from which tiles are large
 inline uint64_t tile_size(bool large) {

@@ -11,8 +11,6 @@
 //   * the word-compressed rows: wptr[0] = 0, non-decreasing; within a row the
 //     32-id words strictly increase, masks are non-zero, and the pairs expand
 //     to exactly the row's ids;
-//   * the pivot descriptors: per vertex its row start, pair start, first and
-//     last id;
 //   * each block CSR (forward: rows of part x, columns of part y; reversed:
 //     the same with the transposed graph): row-pointer segments start on
 //     16-byte boundaries, stay inside the pool and do not overlap; a tile's
@@ -23,11 +21,15 @@
 //     column part (so every edge sits in exactly one tile); the tile's longest
 //     row and non-empty row count are right; the row index of every 32nd entry
 //     names the row holding that entry;
-//   * the reversed tiles' records: entry (v, u) of row part x holds the end of
-//     row u's pairs and its first pair: the one that contains v, or -- when
-//     the first id L of v's row at or above cuts[x] lies in a lower 32-id
-//     word than v -- the first pair of row u whose word is >= L / 32.
 //   * the pivot lists of the fused count (Pivots below).
+//
+// Two further checks are of layouts that a caller builds by hand; the device
+// holds neither array: pivot descriptors per vertex (descs: row start, pair
+// start, first and last id) and, where Tiles::rec is set, the reversed tiles'
+// records (entry (v, u) of row part x holds the end of row u's pairs and its
+// first pair: the one that contains v, or -- when the first id L of v's row at
+// or above cuts[x] lies in a lower 32-id word than v -- the first pair of row u
+// whose word is >= L / 32).
 // Each check returns "" or a message naming the first broken rule.
 #pragma once
 

@@ -47,9 +47,12 @@ UNIT = "edges/s"
 FALLBACK_HBM_GBS = 6650.0
 # serving throughput peak on one B200: requests/s served when the offered
 # rate exceeds what the server sustains, with the server's default
-# configuration (1,800 req/s offered for 30 s: 1,450 and 1,454 served,
-# 4.44e9-4.45e9 edges/s, two runs); the default line serves at 80 % of it
-SERVE_PEAK_RPS = 1450.0
+# configuration (2,800 and 3,300 req/s offered for 10 s: 2,487 and 2,394 served,
+# 7.5e9 edges/s).  The default line's rate is 80 % of the 1,450 req/s that the
+# server sustained before the count ran over pivot lists, so that its records
+# compare.
+SERVE_PEAK_RPS = 2400.0
+SERVE_RATE_RPS = 1160.0
 
 
 def parse():
@@ -114,7 +117,7 @@ def parse():
     p.add_argument("--sub-batch-max-scale", type=int, default=14,
                    help="default line: largest R-MAT scale of the batched-launch sub-record")
     p.add_argument("--sub-serve-rate", type=float, default=0.0,
-                   help="default line: serving rate (0: 80 %% of SERVE_PEAK_RPS)")
+                   help="default line: serving rate (0: SERVE_RATE_RPS)")
     p.add_argument("--sub-serve-duration", type=float, default=10.0)
     return p.parse_args()
 
@@ -836,7 +839,7 @@ def main():
         batch_rec = child_line(["--config", "batch", "--batch-max-scale", str(args.sub_batch_max_scale),
                                 "--steps", "5", "--warmup", "2", "--batch-plain-steps", "0"])
     if rank == 0 and world == 1 and not args.no_serve:
-        rate = args.sub_serve_rate or (0.8 * SERVE_PEAK_RPS)
+        rate = args.sub_serve_rate or SERVE_RATE_RPS
         serve_rec = child_line(["--config", "serve", "--rate", f"{rate:g}", "--duration",
                                 f"{args.sub_serve_duration:g}", "--serve-max-scale", "22"])
         if serve_rec is not None:

@@ -105,8 +105,9 @@ int bbtc_ctx_set_zero_copy(bbtc_ctx* ctx, uint64_t max_bytes);
  *     the reference's task sum for any CSR that meets this contract.)
  *   - cuts[P+1]: cuts[0] = 0, non-decreasing, cuts[P] >= n (rows >= n are
  *     empty, like the phantom row the reference adds, utils.hpp:288); 1 <= P <= 64.
- * The library builds every tile's CSR and CSC on the device; segments start
- * 16-byte aligned.  The caller keeps its buffers. */
+ * The library builds the fused count's pivot lists on the device, and every
+ * tile's CSR and CSC when a per-task count or a tile statistic first asks for
+ * them; segments start 16-byte aligned.  The caller keeps its buffers. */
 int bbtc_graph_upload(bbtc_ctx* ctx, uint32_t n, const uint32_t* indptr, const uint32_t* indices,
                       uint64_t m, const uint32_t* cuts, uint32_t P, bbtc_graph** out);
 /* Same, with indptr / indices already in device memory of the context's
@@ -133,8 +134,10 @@ int bbtc_graph_info_get(const bbtc_graph* g, bbtc_graph_info* info);
  * at 0, never decrease and end at its nnz; segments start on 16-byte
  * boundaries, stay inside their pools and do not overlap; tile rows are
  * strictly increasing, columns < the tile width, and together hold every
- * edge exactly once; tile statistics, the row index of every 32nd entry and
- * the reversed tiles' forward-edge records are right.  BBTC_ERR_LAYOUT with
+ * edge exactly once; tile statistics and the row index of every 32nd entry
+ * are right; the pivot lists name every vertex's in-edges, the pairs of its
+ * row and the pairs that each in-edge's row can meet.  The tiles are checked
+ * when they have been built.  BBTC_ERR_LAYOUT with
  * the first broken rule in the message.  Costs about the graph's device
  * bytes in host memory; synchronises the context's stream. */
 int bbtc_graph_validate(const bbtc_graph* g);
@@ -184,12 +187,14 @@ typedef struct bbtc_opts {
   int kernel;                /* bbtc_kernel */
   uint32_t bitmap_words;     /* shared bitmap / list words per warp: 0 = default (1024) */
   uint32_t warps_per_block;  /* 0 = default (8) */
-  uint32_t unit_work;        /* target probes per work unit, 0 = default (by position in a fused count, 8192 per task) */
+  uint32_t unit_work;        /* target probes per work unit, 0 = default (fused: by position in the queue; per task:
+                                1024, fewer where the list is too small for eight units a warp) */
   uint32_t blocks_per_sm;    /* persistent grid = SMs x this, 0 = occupancy limit */
   int use_cuda_graph;        /* replay the launch sequence through a captured CUDA graph */
   int sort_tasks;            /* when tasks == NULL: 1 = cost-sorted descending (default) */
   uint32_t occupancy;        /* persistent form: register budget for 4, 5, 6 or 8 blocks per SM (5: fused counts only; 0: 5 for
-                                fused counts with a buffer of at most 1024 words, else 4) */
+                                fused counts with a buffer of at most 1024 words, else 4).  Fused counts of long
+                                in-lists keep four rows in flight at 5, two at the others */
 } bbtc_opts;
 
 void bbtc_opts_default(bbtc_opts* o);
