@@ -31,7 +31,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <sstream>
 
@@ -484,19 +483,23 @@ int kernel_smem_optin(bbtc_ctx* ctx, const bbtc_opts& o) {
   if (sm > ctx->smem_optin)
     return fail(BBTC_ERR_ARG, "bitmap_words x warps_per_block needs " + std::to_string(sm) +
                                   " bytes of shared memory; the device allows " + std::to_string(ctx->smem_optin));
+  if (sm <= ctx->smem_set) return BBTC_OK;
   // A kernel has one limit per device, whichever context launches it: it is
-  // only ever raised.
+  // only ever raised, so what a context found once holds.  The kernels' own
+  // attribute is asked, which a reset of the device takes back; it is raised
+  // for k_count_task last.
   static std::mutex mu;
-  static std::map<int, size_t> limit;
   std::lock_guard<std::mutex> lk(mu);
-  size_t& set = limit[ctx->device];
-  if (sm <= set) return BBTC_OK;
-  BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_CUDA(cudaFuncSetAttribute(k_count_task, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  BBTC_TRY(pivots_smem_optin(sm));
-  set = sm;
+  cudaFuncAttributes now;
+  BBTC_CUDA(cudaFuncGetAttributes(&now, k_count_task));
+  if ((size_t)now.maxDynamicSharedSizeBytes < sm) {
+    BBTC_TRY(pivots_smem_optin(sm));
+    BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    BBTC_CUDA(cudaFuncSetAttribute(k_count_queue<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    BBTC_CUDA(cudaFuncSetAttribute(k_count_task, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  }
+  ctx->smem_set = sm;
   return BBTC_OK;
 }
 

@@ -162,6 +162,7 @@ struct bbtc_ctx {
   cudaStream_t stream = nullptr;
   int sms = 0;
   size_t smem_optin = 0;
+  size_t smem_set = 0;                 // dynamic shared memory that the count kernels take, as far as asked
   bool open_carveout = false;          // layout kernels ask for the largest shared-memory carveout (launch_layout)
   uint32_t layout_blocks_per_sm = 8;   // grid cap of the layout kernels (256 threads a block)
   uint32_t upload_window = 0;          // host uploads: pieces in flight at most (0 = all at once)
